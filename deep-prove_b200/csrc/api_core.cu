@@ -740,25 +740,30 @@ int dpb_linear_combination(dpb_ctx* ctx, dpb_mle* const* mles, const void* coeff
         if (m->len > max_len) max_len = m->len;
     }
     const size_t es = gl ? 16 : 32;
-    void *d_src = nullptr, *d_coef = nullptr;
+    void *d_src = nullptr, *d_coef = nullptr, *d_rows = nullptr;
     DPB_TRY(device_alloc(ctx, n * sizeof(LinCombSrc), &d_src));
     int rc = device_alloc(ctx, n * es, &d_coef);
+    if (rc == DPB_OK && !gl) rc = device_alloc(ctx, (size_t)n * kLinRows * 32, &d_rows);
     if (rc == DPB_OK) rc = upload_small(ctx, d_src, src.data(), n * sizeof(LinCombSrc));
     if (rc == DPB_OK) rc = upload_small(ctx, d_coef, coeffs, n * es);
     dpb_mle* res = nullptr;
     if (rc == DPB_OK) rc = new_mle(ctx, gl ? DPB_GL_EXT : DPB_FR, max_len, &res);
     if (rc == DPB_OK) {
         if (gl)
-            linear_combination_kernel<GlFam><<<grid_for(ctx, max_len), kThreads, 0, ctx->stream>>>(
+            linear_combination_gl<<<grid_for(ctx, max_len), kThreads, 0, ctx->stream>>>(
                 (const LinCombSrc*)d_src, (const Gl2*)d_coef, n, max_len, (Gl2*)res->ptr);
-        else
-            linear_combination_kernel<FrFam><<<grid_for(ctx, max_len), kThreads, 0, ctx->stream>>>(
-                (const LinCombSrc*)d_src, (const Fr*)d_coef, n, max_len, (Fr*)res->ptr);
+        else {
+            lincomb_rows_kernel<<<(n * kLinRows + kThreads - 1) / kThreads, kThreads, 0, ctx->stream>>>(
+                (const LinCombSrc*)d_src, (const Fr*)d_coef, n, (uint32_t*)d_rows);
+            linear_combination_fr<<<grid_for(ctx, max_len), kThreads, 0, ctx->stream>>>(
+                (const LinCombSrc*)d_src, (const uint32_t*)d_rows, n, max_len, (Fr*)res->ptr);
+        }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) rc = fail(DPB_ECUDA, "linear combination: %s", cudaGetErrorString(e));
     }
     device_free(ctx, d_src);
     device_free(ctx, d_coef);
+    device_free(ctx, d_rows);
     if (rc != DPB_OK) {
         if (res) dpb_mle_free(res);
         return rc;
@@ -930,7 +935,6 @@ int dpb_mle_evaluate_many(dpb_ctx* ctx, dpb_mle* const* mles, uint32_t n, const 
         src[t].eq = eq[mv]->ptr;
         src[t].len = m->len;
         src[t].dtype = m->dtype;
-        src[t].pad = 0;
         if (gl) {
             Gl2 sc = GlFam::one();
             for (uint32_t j = mv; j < num_vars; j++) sc = GlFam::mul(sc, GlFam::sub(GlFam::one(), ((const Gl2*)point)[j]));
@@ -941,37 +945,36 @@ int dpb_mle_evaluate_many(dpb_ctx* ctx, dpb_mle* const* mles, uint32_t n, const 
             memcpy(scale.data() + (size_t)t * es, &sc, es);
         }
     }
-    uint64_t longest = 0;
-    for (const auto& t : src) longest = std::max(longest, t.len);
-    // enough blocks to fill the GPU a few times over, at most one slice per 256 entries of the longest table
-    uint32_t slices = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((longest + kThreads - 1) / kThreads,
-                                                                         ((uint64_t)ctx->sm_count * 8 + n - 1) / n));
+    // pieces of the tables, one block each: enough to fill the GPU a few times over, none below four entries a thread
+    uint64_t entries = 0;
+    for (const auto& t : src) entries += t.len;
+    uint64_t piece = entries / ((uint64_t)ctx->sm_count * 16) + 1;
+    if (piece < 4 * kThreads) piece = 4 * kThreads;
+    uint64_t pieces = 0;
+    for (auto& t : src) {
+        t.first = (uint32_t)pieces;
+        pieces += (t.len + piece - 1) / piece;
+    }
     void *d_src = nullptr, *d_scale = nullptr, *d_partial = nullptr, *d_out = nullptr;
     int rc = device_alloc(ctx, (size_t)n * sizeof(EvalManySrc), &d_src);
     if (rc == DPB_OK) rc = device_alloc(ctx, (size_t)n * es, &d_scale);
-    if (rc == DPB_OK) rc = device_alloc(ctx, (size_t)n * slices * es, &d_partial);
+    if (rc == DPB_OK) rc = device_alloc(ctx, pieces * es, &d_partial);
     if (rc == DPB_OK) rc = device_alloc(ctx, (size_t)n * es, &d_out);
     if (rc == DPB_OK) rc = upload_small(ctx, d_src, src.data(), (size_t)n * sizeof(EvalManySrc));
     if (rc == DPB_OK) rc = upload_small(ctx, d_scale, scale.data(), (size_t)n * es);
     if (rc == DPB_OK) {
-        // the grid's second dimension holds at most 65535 blocks
-        for (uint32_t first = 0; first < n; first += 65535) {
-            const uint32_t cnt = std::min<uint32_t>(65535, n - first);
-            const dim3 grid(slices, cnt);
-            if (gl)
-                evaluate_many_kernel<GlFam><<<grid, kThreads, 0, ctx->stream>>>((const EvalManySrc*)d_src + first, slices,
-                                                                                 (Gl2*)d_partial + (size_t)first * slices);
-            else
-                evaluate_many_kernel<FrFam><<<grid, kThreads, 0, ctx->stream>>>((const EvalManySrc*)d_src + first, slices,
-                                                                                 (Fr*)d_partial + (size_t)first * slices);
+        const uint32_t blocks = (uint32_t)(((uint64_t)n * 32 + kThreads - 1) / kThreads);
+        if (gl) {
+            evaluate_many_kernel<GlFam><<<(uint32_t)pieces, kThreads, 0, ctx->stream>>>((const EvalManySrc*)d_src, n, piece,
+                                                                                        (Gl2*)d_partial);
+            evaluate_many_finish<GlFam><<<blocks, kThreads, 0, ctx->stream>>>((const Gl2*)d_partial, (const EvalManySrc*)d_src, piece,
+                                                                              (const Gl2*)d_scale, n, (Gl2*)d_out);
+        } else {
+            evaluate_many_kernel<FrFam><<<(uint32_t)pieces, kThreads, 0, ctx->stream>>>((const EvalManySrc*)d_src, n, piece,
+                                                                                        (Fr*)d_partial);
+            evaluate_many_finish<FrFam><<<blocks, kThreads, 0, ctx->stream>>>((const Fr*)d_partial, (const EvalManySrc*)d_src, piece,
+                                                                              (const Fr*)d_scale, n, (Fr*)d_out);
         }
-        const uint32_t blocks = (n + kThreads - 1) / kThreads;
-        if (gl)
-            evaluate_many_finish<GlFam><<<blocks, kThreads, 0, ctx->stream>>>((const Gl2*)d_partial, slices, (const Gl2*)d_scale, n,
-                                                                                (Gl2*)d_out);
-        else
-            evaluate_many_finish<FrFam><<<blocks, kThreads, 0, ctx->stream>>>((const Fr*)d_partial, slices, (const Fr*)d_scale, n,
-                                                                                (Fr*)d_out);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, (size_t)n * es, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);

@@ -62,6 +62,15 @@ DPB_HD Fr fr_rr() {
     r.l[3] = DPB_FR_RR3;
     return r;
 }
+// 2^31 in Montgomery form
+DPB_HD Fr fr_two31() {
+    Fr r;
+    r.l[0] = 0x49f3c4328adc5cedULL;
+    r.l[1] = 0x8b6f9213582f50aaULL;
+    r.l[2] = 0x0938dba198155c1cULL;
+    r.l[3] = 0x035e01bf76361137ULL;
+    return r;
+}
 DPB_HD bool fr_eq(const Fr& a, const Fr& b) {
     return a.l[0] == b.l[0] && a.l[1] == b.l[1] && a.l[2] == b.l[2] && a.l[3] == b.l[3];
 }
@@ -224,6 +233,16 @@ __device__ __forceinline__ Fr fr_intacc_finish(const FrIntAcc& acc) {
     return fr_add(a, b);
 }
 
+// Sum of full products, reduced once: see frw::Wide.
+__device__ __forceinline__ Fr fr_wide_finish(const frw::Wide& s) {
+    frw::F8 lo, mid, top, one;
+    frw::wide_split(s, lo, mid, top);
+#pragma unroll
+    for (int i = 0; i < 8; i++) one.w[i] = i ? 0 : 1;
+    const frw::F8 a = frw::mul(lo, one), b = frw::mul(mid, frw::from_fr(fr_one())), c = frw::mul(top, frw::from_fr(fr_rr()));
+    return frw::to_fr(frw::add(frw::add(a, b), c));
+}
+
 // Integer -> Montgomery form without a full product: |x| = lo + 2^32 hi, and x R = lo * (+-R) + hi * (+-2^32 R)
 // mod r; the rows below hold those four constants times 2^64 (what frw::lin2_rows divides out again).
 static __device__ __constant__ const uint32_t kIntRowOnePos[8] = {0x7c5fb586u, 0xb4c6edf9u, 0xbfeb93beu, 0x708c8d50u,
@@ -241,7 +260,7 @@ __device__ __forceinline__ Fr fr_from_int_rows(int64_t x) {
                                      neg ? kIntRowHiNeg : kIntRowHiPos));
 }
 
-// 2^(32 i + 64) mod r as a plain integer, i = 0..7
+// 2^(32 i + 64) mod r as a plain integer, i = 0..9
 DPB_HD Fr fr_fixed_power(int i) {
     Fr x;
     x.l[0] = x.l[1] = x.l[2] = x.l[3] = 0;
@@ -250,16 +269,27 @@ DPB_HD Fr fr_fixed_power(int i) {
         x.l[e / 64] = 1ull << (e % 64);
     } else if (e == 256) {
         x = fr_one();  // 2^256 mod r
-    } else {  // 2^288 mod r
+    } else if (e == 288) {
         x.l[0] = 0x93e7886515b8b9daULL;
         x.l[1] = 0x16df2426b05ea154ULL;
         x.l[2] = 0x1271b743302ab839ULL;
         x.l[3] = 0x06bc037eec6c226eULL;
+    } else if (e == 320) {
+        x.l[0] = 0xb4c6edf97c5fb586ULL;
+        x.l[1] = 0x708c8d50bfeb93beULL;
+        x.l[2] = 0x9ffd1de404f7e0efULL;
+        x.l[3] = 0x215b02ac9a392866ULL;
+    } else {  // 352
+        x.l[0] = 0x54c81065af8b5a7aULL;
+        x.l[1] = 0x2b82a1ef97aa45f6ULL;
+        x.l[2] = 0xbe492693330a5a6dULL;
+        x.l[3] = 0x1847e4868229aff4ULL;
     }
     return x;
 }
 // Constants of frw::mul_fixed for the multiplicand c (Montgomery form): row i is
-// c * 2^(32 i + 64) / 2^256 mod r (a Montgomery product of c with the plain power).
+// c * 2^(32 i + 64) / 2^256 mod r (a Montgomery product of c with the plain power).  Rows 0..7 multiply the words of
+// a Montgomery form; rows 8 and 9 (8 rows times 2^256) the low and the high word of a plain integer.
 DPB_HD void fr_fixed_row(const Fr& c, int i, uint32_t* row) {
     const Fr ci = fr_mul(c, fr_fixed_power(i));
     for (int w = 0; w < 4; w++) {

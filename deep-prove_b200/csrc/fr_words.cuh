@@ -155,6 +155,25 @@ __device__ __forceinline__ F8 mul(const F8& a, const F8& b) {
     return reduce_once(s);
 }
 
+// (E + O) / 2^64 mod r for a sum of rows below 2^297 held as aligned pairs at even (E) and odd (O) positions: a
+// reduction word for position 0 (only E holds it), then one for position 1 (O's pair and E's left-over word).
+__device__ __forceinline__ F8 reduce_rows(uint32_t* E, uint32_t* O) {
+    const uint32_t m0 = E[0] * DPB_FRW_INV;
+    chain_mod_even(E, E[8], m0);
+    chain_mod_odd<false>(O + 1, O[9], m0, 0);
+    const uint32_t m1 = (O[1] + E[1]) * DPB_FRW_INV;
+    chain_mod_even(O + 1, O[9], m1);
+    chain_mod_odd<true>(E + 2, E[10], m1, E[1]);
+    F8 s;
+    asm("add.cc.u32 %0, %8, %16; addc.cc.u32 %1, %9, %17; addc.cc.u32 %2, %10, %18; addc.cc.u32 %3, %11, %19;\n\t"
+        "addc.cc.u32 %4, %12, %20; addc.cc.u32 %5, %13, %21; addc.cc.u32 %6, %14, %22; addc.u32 %7, %15, %23;"
+        : "=&r"(s.w[0]), "=&r"(s.w[1]), "=&r"(s.w[2]), "=&r"(s.w[3]), "=&r"(s.w[4]), "=&r"(s.w[5]), "=&r"(s.w[6]),
+          "=&r"(s.w[7])
+        : "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]), "r"(E[8]), "r"(E[9]), "r"(O[2]),
+          "r"(O[3]), "r"(O[4]), "r"(O[5]), "r"(O[6]), "r"(O[7]), "r"(O[8]), "r"(O[9]));
+    return reduce_once(s);
+}
+
 // Product by a multiplicand that is fixed for a whole launch (the challenge of a fold).
 // With a = sum_i a_i 2^(32 i), a * c / 2^256 = sum_i a_i * C_i for the eight constants
 // C_i = c * 2^(32 i) / 2^256 mod r, which the host computes once per round.  The sum of
@@ -174,21 +193,7 @@ __device__ __forceinline__ F8 mul_fixed(const F8& a, const FixedMul& k) {
         chain_mul(E, E[8], k.c[i][0], k.c[i][2], k.c[i][4], k.c[i][6], a.w[i]);
         chain_mul(O + 1, O[9], k.c[i][1], k.c[i][3], k.c[i][5], k.c[i][7], a.w[i]);
     }
-    // reduction word for position 0 (only E holds it), then for position 1 (O's pair and E's left-over word)
-    const uint32_t m0 = E[0] * DPB_FRW_INV;
-    chain_mod_even(E, E[8], m0);
-    chain_mod_odd<false>(O + 1, O[9], m0, 0);
-    const uint32_t m1 = (O[1] + E[1]) * DPB_FRW_INV;
-    chain_mod_even(O + 1, O[9], m1);
-    chain_mod_odd<true>(E + 2, E[10], m1, E[1]);
-    F8 s;
-    asm("add.cc.u32 %0, %8, %16; addc.cc.u32 %1, %9, %17; addc.cc.u32 %2, %10, %18; addc.cc.u32 %3, %11, %19;\n\t"
-        "addc.cc.u32 %4, %12, %20; addc.cc.u32 %5, %13, %21; addc.cc.u32 %6, %14, %22; addc.u32 %7, %15, %23;"
-        : "=&r"(s.w[0]), "=&r"(s.w[1]), "=&r"(s.w[2]), "=&r"(s.w[3]), "=&r"(s.w[4]), "=&r"(s.w[5]), "=&r"(s.w[6]),
-          "=&r"(s.w[7])
-        : "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]), "r"(E[8]), "r"(E[9]), "r"(O[2]),
-          "r"(O[3]), "r"(O[4]), "r"(O[5]), "r"(O[6]), "r"(O[7]), "r"(O[8]), "r"(O[9]));
-    return reduce_once(s);
+    return reduce_rows(E, O);
 }
 
 // Two small integers times two rows, the reduction of mul_fixed: what turns an integer, or the fold of two
@@ -202,22 +207,25 @@ __device__ __forceinline__ F8 lin2_rows(uint32_t ma, const uint32_t* ra, uint32_
     chain_mul(O + 1, O[9], ra[1], ra[3], ra[5], ra[7], ma);
     chain_mul(E, E[8], rd[0], rd[2], rd[4], rd[6], md);
     chain_mul(O + 1, O[9], rd[1], rd[3], rd[5], rd[7], md);
-    const uint32_t m0 = E[0] * DPB_FRW_INV;
-    chain_mod_even(E, E[8], m0);
-    chain_mod_odd<false>(O + 1, O[9], m0, 0);
-    const uint32_t m1 = (O[1] + E[1]) * DPB_FRW_INV;
-    chain_mod_even(O + 1, O[9], m1);
-    chain_mod_odd<true>(E + 2, E[10], m1, E[1]);
-    F8 s;
-    asm("add.cc.u32 %0, %8, %16; addc.cc.u32 %1, %9, %17; addc.cc.u32 %2, %10, %18; addc.cc.u32 %3, %11, %19;\n\t"
-        "addc.cc.u32 %4, %12, %20; addc.cc.u32 %5, %13, %21; addc.cc.u32 %6, %14, %22; addc.u32 %7, %15, %23;"
-        : "=&r"(s.w[0]), "=&r"(s.w[1]), "=&r"(s.w[2]), "=&r"(s.w[3]), "=&r"(s.w[4]), "=&r"(s.w[5]), "=&r"(s.w[6]),
-          "=&r"(s.w[7])
-        : "r"(E[2]), "r"(E[3]), "r"(E[4]), "r"(E[5]), "r"(E[6]), "r"(E[7]), "r"(E[8]), "r"(E[9]), "r"(O[2]),
-          "r"(O[3]), "r"(O[4]), "r"(O[5]), "r"(O[6]), "r"(O[7]), "r"(O[8]), "r"(O[9]));
-    return reduce_once(s);
+    return reduce_rows(E, O);
 }
 
+// Sum of (32-bit integer) * row products, rows made with a factor 2^64 as for mul_fixed: 8 multiply-adds and two
+// carry words per term, and the two-word reduction of mul_fixed once per sum.  Up to 2^10 terms: the sum stays below
+// 2^296, so that the reduced value is below 2r.
+struct RowAcc {
+    uint32_t E[12], O[12];
+};
+__device__ __forceinline__ RowAcc rowacc_zero() {
+    RowAcc a;
+#pragma unroll
+    for (int i = 0; i < 12; i++) a.E[i] = a.O[i] = 0;
+    return a;
+}
+__device__ __forceinline__ void rowacc_mac(RowAcc& a, const uint32_t* row, uint32_t x) {
+    chain_mul(a.E, a.E[8], row[0], row[2], row[4], row[6], x);
+    chain_mul(a.O + 1, a.O[9], row[1], row[3], row[5], row[7], x);
+}
 // Sum of (64-bit integer) * (field element) products kept as one unreduced integer: what the contraction of an
 // integer tensor against eq weights is made of.  A term is 16 wide multiply-adds and no reduction; the sum of up to
 // 2^24 terms stays below 2^352 and is reduced once (two Montgomery products).  Layout as in mul: E holds word pairs
@@ -242,23 +250,29 @@ __device__ __forceinline__ void chain_mul_long(uint32_t* c, uint32_t x0, uint32_
           "+r"(c[9]), "+r"(c[10])
         : "r"(y), "r"(x0), "r"(x1), "r"(x2), "r"(x3));
 }
-// acc += mag * w, mag a 64-bit magnitude, w any 256-bit value
-__device__ __forceinline__ void intacc_mac(IntAcc& a, const F8& w, uint64_t mag) {
-    const uint32_t m0 = (uint32_t)mag, m1 = (uint32_t)(mag >> 32);
+// acc += m0 * w
+__device__ __forceinline__ void intacc_mac_lo(IntAcc& a, const F8& w, uint32_t m0) {
     chain_mul_long(a.E, w.w[0], w.w[2], w.w[4], w.w[6], m0);      // positions (0,1) .. (6,7)
     chain_mul_long(a.O + 1, w.w[1], w.w[3], w.w[5], w.w[7], m0);  // positions (1,2) .. (7,8)
-    if (m1) {  // quantised values seldom need the upper word
-        chain_mul_long(a.O + 1, w.w[0], w.w[2], w.w[4], w.w[6], m1);  // one word up: (1,2) .. (7,8)
-        // two words up: (2,3) .. (8,9); the carry has one word of room left (the sum stays below 2^352)
-        asm("mad.lo.cc.u32 %0, %10, %9, %0; madc.hi.cc.u32 %1, %10, %9, %1;\n\t"
-            "madc.lo.cc.u32 %2, %11, %9, %2; madc.hi.cc.u32 %3, %11, %9, %3;\n\t"
-            "madc.lo.cc.u32 %4, %12, %9, %4; madc.hi.cc.u32 %5, %12, %9, %5;\n\t"
-            "madc.lo.cc.u32 %6, %13, %9, %6; madc.hi.cc.u32 %7, %13, %9, %7;\n\t"
-            "addc.cc.u32 %8, %8, 0;"
-            : "+r"(a.E[2]), "+r"(a.E[3]), "+r"(a.E[4]), "+r"(a.E[5]), "+r"(a.E[6]), "+r"(a.E[7]), "+r"(a.E[8]),
-              "+r"(a.E[9]), "+r"(a.E[10])
-            : "r"(m1), "r"(w.w[1]), "r"(w.w[3]), "r"(w.w[5]), "r"(w.w[7]));
-    }
+}
+// acc += 2^32 * m1 * w
+__device__ __forceinline__ void intacc_mac_hi(IntAcc& a, const F8& w, uint32_t m1) {
+    chain_mul_long(a.O + 1, w.w[0], w.w[2], w.w[4], w.w[6], m1);  // one word up: (1,2) .. (7,8)
+    // two words up: (2,3) .. (8,9); the carry has one word of room left (the sum stays below 2^352)
+    asm("mad.lo.cc.u32 %0, %10, %9, %0; madc.hi.cc.u32 %1, %10, %9, %1;\n\t"
+        "madc.lo.cc.u32 %2, %11, %9, %2; madc.hi.cc.u32 %3, %11, %9, %3;\n\t"
+        "madc.lo.cc.u32 %4, %12, %9, %4; madc.hi.cc.u32 %5, %12, %9, %5;\n\t"
+        "madc.lo.cc.u32 %6, %13, %9, %6; madc.hi.cc.u32 %7, %13, %9, %7;\n\t"
+        "addc.cc.u32 %8, %8, 0;"
+        : "+r"(a.E[2]), "+r"(a.E[3]), "+r"(a.E[4]), "+r"(a.E[5]), "+r"(a.E[6]), "+r"(a.E[7]), "+r"(a.E[8]),
+          "+r"(a.E[9]), "+r"(a.E[10])
+        : "r"(m1), "r"(w.w[1]), "r"(w.w[3]), "r"(w.w[5]), "r"(w.w[7]));
+}
+// acc += mag * w, mag a 64-bit magnitude, w any 256-bit value
+__device__ __forceinline__ void intacc_mac(IntAcc& a, const F8& w, uint64_t mag) {
+    const uint32_t m1 = (uint32_t)(mag >> 32);
+    intacc_mac_lo(a, w, (uint32_t)mag);
+    if (m1) intacc_mac_hi(a, w, m1);  // quantised values seldom need the upper word
 }
 // the sum as words 0..10 (E + O), low 8 words and the words above them
 __device__ __forceinline__ void intacc_split(const IntAcc& a, F8& lo, F8& hi) {
@@ -277,6 +291,62 @@ __device__ __forceinline__ void intacc_split(const IntAcc& a, F8& lo, F8& hi) {
     for (int i = 0; i < 4; i++) hi.w[i] = s[8 + i];
 #pragma unroll
     for (int i = 4; i < 8; i++) hi.w[i] = 0;
+}
+
+// Sum of full products kept unreduced: 64 multiply-adds per product instead of 128, the Montgomery reduction once per
+// sum.  A product is below 2^508, so 17 words hold the sum of up to 2^36 of them.
+struct Wide {
+    uint32_t w[17];
+};
+__device__ __forceinline__ Wide wide_zero() {
+    Wide a;
+#pragma unroll
+    for (int i = 0; i < 17; i++) a.w[i] = 0;
+    return a;
+}
+// one word of b: as mont_step without the reduction
+template <int I>
+__device__ __forceinline__ void wide_step(uint32_t* P, uint32_t* Q, const uint32_t* a, uint32_t bi) {
+    chain_mul(P + I, P[I + 8], a[0], a[2], a[4], a[6], bi);
+    chain_mul(Q + I + 1, Q[I + 9], a[1], a[3], a[5], a[7], bi);
+}
+__device__ __forceinline__ void wide_mac(Wide& s, const F8& a, const F8& b) {
+    uint32_t E[18], O[18];
+#pragma unroll
+    for (int i = 0; i < 18; i++) E[i] = O[i] = 0;
+    wide_step<0>(E, O, a.w, b.w[0]);
+    wide_step<1>(O, E, a.w, b.w[1]);
+    wide_step<2>(E, O, a.w, b.w[2]);
+    wide_step<3>(O, E, a.w, b.w[3]);
+    wide_step<4>(E, O, a.w, b.w[4]);
+    wide_step<5>(O, E, a.w, b.w[5]);
+    wide_step<6>(E, O, a.w, b.w[6]);
+    wide_step<7>(O, E, a.w, b.w[7]);
+    // the two halves are added one after the other: neither overflows into word 17 (see above)
+    auto add16 = [&](const uint32_t* x) {
+        asm("add.cc.u32 %0, %0, %17; addc.cc.u32 %1, %1, %18; addc.cc.u32 %2, %2, %19; addc.cc.u32 %3, %3, %20;\n\t"
+            "addc.cc.u32 %4, %4, %21; addc.cc.u32 %5, %5, %22; addc.cc.u32 %6, %6, %23; addc.cc.u32 %7, %7, %24;\n\t"
+            "addc.cc.u32 %8, %8, %25; addc.cc.u32 %9, %9, %26; addc.cc.u32 %10, %10, %27; addc.cc.u32 %11, %11, %28;\n\t"
+            "addc.cc.u32 %12, %12, %29; addc.cc.u32 %13, %13, %30; addc.cc.u32 %14, %14, %31; addc.cc.u32 %15, %15, %32;\n\t"
+            "addc.u32 %16, %16, 0;"
+            : "+r"(s.w[0]), "+r"(s.w[1]), "+r"(s.w[2]), "+r"(s.w[3]), "+r"(s.w[4]), "+r"(s.w[5]), "+r"(s.w[6]),
+              "+r"(s.w[7]), "+r"(s.w[8]), "+r"(s.w[9]), "+r"(s.w[10]), "+r"(s.w[11]), "+r"(s.w[12]), "+r"(s.w[13]),
+              "+r"(s.w[14]), "+r"(s.w[15]), "+r"(s.w[16])
+            : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(x[8]),
+              "r"(x[9]), "r"(x[10]), "r"(x[11]), "r"(x[12]), "r"(x[13]), "r"(x[14]), "r"(x[15]));
+    };
+    add16(E);
+    add16(O);
+}
+// the sum divided by 2^256 mod r (the Montgomery form of the sum of the products of Montgomery forms): with
+// lo + 2^256 mid + 2^512 top the three parts are the Montgomery products of lo with 1, mid with 2^256 and top with 2^512
+__device__ __forceinline__ void wide_split(const Wide& s, F8& lo, F8& mid, F8& top) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        lo.w[i] = s.w[i];
+        mid.w[i] = s.w[8 + i];
+        top.w[i] = i ? 0 : s.w[16];
+    }
 }
 
 __device__ __forceinline__ F8 add(const F8& a, const F8& b) {

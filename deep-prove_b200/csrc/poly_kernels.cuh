@@ -2,6 +2,7 @@
 // tables, partial evaluation of the top / bottom variables.
 #pragma once
 #include "family.cuh"
+#include "lazy_sum.cuh"
 
 namespace dpb {
 
@@ -133,37 +134,62 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // Many tables evaluated at one point: table t (2^m_t entries, any layout of its family) against the eq table of the
-// point's first m_t coordinates: partial[t * slices + s] = sum over slice s of table_t[x] * eq_{m_t}[x].
+// point's first m_t coordinates.  Every block sums one piece of `piece` entries of one table (pieces of all tables are
+// laid end to end, `first[t]` the first piece of table t), so a long table among many short ones still fills the GPU.
+// The sums stay unreduced (EntrySum).  128 BN254 int32 tables, 16 of them of 2^20 entries: 918 us with a reduction per
+// product and the same number of blocks for every table, 116 us since.
 struct EvalManySrc {
     const void* ptr;
     const void* eq;  // eq table over this table's variables (challenge elements)
     uint64_t len;
     int32_t dtype;
-    int32_t pad;
+    uint32_t first;
 };
-template <class F>
-__global__ void __launch_bounds__(kThreads)
-    evaluate_many_kernel(const EvalManySrc* __restrict__ src, uint32_t slices, typename F::E* __restrict__ partial) {
-    typedef typename F::E E;
-    const EvalManySrc t = src[blockIdx.y];
-    E acc[1] = {F::zero()};
-    const uint64_t stride = (uint64_t)slices * blockDim.x;
-    for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < t.len; x += stride)
-        acc[0] = F::add(acc[0], F::mul(F::load(t.ptr, t.dtype, x), ((const E*)t.eq)[x]));
-    block_sum<F, 1>(acc);
-    if (threadIdx.x == 0) partial[(size_t)blockIdx.y * slices + blockIdx.x] = acc[0];
+template <class F, bool INT>
+__device__ __forceinline__ typename F::E evaluate_piece(const EvalManySrc& t, uint64_t begin, uint64_t end) {
+    EntrySum<F, INT> acc;
+    acc.zero();
+    for (uint64_t x = begin + threadIdx.x; x < end; x += blockDim.x)
+        acc.mac(F::load(t.eq, F::kChalDtype, x), t.ptr, t.dtype, x);
+    return acc.finish();
 }
-// out[t] = scale[t] * sum_s partial[t * slices + s]
 template <class F>
 __global__ void __launch_bounds__(kThreads)
-    evaluate_many_finish(const typename F::E* __restrict__ partial, uint32_t slices, const typename F::E* __restrict__ scale,
-                         uint32_t n, typename F::E* __restrict__ out) {
+    evaluate_many_kernel(const EvalManySrc* __restrict__ src, uint32_t n, uint64_t piece, typename F::E* __restrict__ partial) {
     typedef typename F::E E;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t lo = 0, hi = n;  // the table with first <= this block's piece < the next table's first
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (src[mid].first <= blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    const EvalManySrc t = src[lo];
+    const uint64_t begin = (uint64_t)(blockIdx.x - t.first) * piece;
+    const uint64_t end = begin + piece < t.len ? begin + piece : t.len;
+    const bool ints = t.dtype >= DPB_GL_I64;
+    E acc[1] = {ints ? evaluate_piece<F, true>(t, begin, end) : evaluate_piece<F, false>(t, begin, end)};
+    block_sum<F, 1>(acc);
+    if (threadIdx.x == 0) partial[blockIdx.x] = acc[0];
+}
+// out[t] = scale[t] * (sum of the table's pieces, less 2^31 where EntrySum added it: a whole eq table sums to one);
+// one warp per table
+template <class F>
+__global__ void __launch_bounds__(kThreads)
+    evaluate_many_finish(const typename F::E* __restrict__ partial, const EvalManySrc* __restrict__ src, uint64_t piece,
+                         const typename F::E* __restrict__ scale, uint32_t n, typename F::E* __restrict__ out) {
+    typedef typename F::E E;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= n) return;
+    const EvalManySrc d = src[t];
+    const uint32_t pieces = (uint32_t)((d.len + piece - 1) / piece);
     E acc = F::zero();
-    for (uint32_t s = 0; s < slices; s++) acc = F::add(acc, partial[(size_t)t * slices + s]);
-    out[t] = F::mul(acc, scale[t]);
+    for (uint32_t s = lane; s < pieces; s += 32) acc = F::add(acc, partial[d.first + s]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc = F::add(acc, F::shfl_down(acc, off));
+    if (lane == 0) {
+        if (EntrySum<F, true>::kPlus31 && d.dtype >= DPB_GL_I64) acc = F::sub(acc, F::from_u64(0x80000000ull));
+        out[t] = F::mul(acc, scale[t]);
+    }
 }
 
 // One source table of a linear combination.
@@ -200,20 +226,79 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // out[i] = sum_j coeff[j] * table_j[i], tables shorter than the output read as zero beyond their length.
-// Consecutive threads read consecutive entries of each table in turn.
-template <class F>
+// Consecutive threads read consecutive entries of each table in turn.  BN254: the coefficients are laid out as rows
+// first (lincomb_rows_kernel), so that a term is 8 multiply-adds for an int32 entry (the row of the coefficient or of
+// its negative), 16 for a 64-bit one that needs its upper word and 64 for a field entry, and the sum is reduced once
+// (twice every kRowTerms terms).  119 int32 tables, 15 of 2^20 entries: 641 us with a field product per
+// term, 208 us since.
+constexpr uint32_t kLinRows = 8;        // rows per table: a field table's eight, or an integer table's c, -c, 2^32 c, -2^32 c
+constexpr uint32_t kRowTerms = 1024;    // row products a RowAcc may hold
 __global__ void __launch_bounds__(kThreads)
-    linear_combination_kernel(const LinCombSrc* __restrict__ src, const typename F::E* __restrict__ coeff, uint32_t n,
-                              uint64_t len, typename F::E* __restrict__ out) {
-    typedef typename F::E E;
+    lincomb_rows_kernel(const LinCombSrc* __restrict__ src, const Fr* __restrict__ coeff, uint32_t n, uint32_t* __restrict__ rows) {
+    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x, j = w / kLinRows, q = w % kLinRows;
+    if (j >= n) return;
+    uint32_t row[8];
+    if (src[j].dtype == DPB_FR) {
+        fr_fixed_row(coeff[j], (int)q, row);
+    } else {
+        if (q >= 4) return;
+        fr_fixed_row((q & 1) ? fr_neg(coeff[j]) : coeff[j], 8 + (int)(q >> 1), row);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) rows[(size_t)w * 8 + i] = row[i];
+}
+__device__ __forceinline__ void lincomb_row_mac(frw::RowAcc& acc, const uint32_t* __restrict__ row, uint32_t x) {
+    const uint4 a = ((const uint4*)row)[0], b = ((const uint4*)row)[1];
+    const uint32_t r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    frw::rowacc_mac(acc, r, x);
+}
+__global__ void __launch_bounds__(kThreads)
+    linear_combination_fr(const LinCombSrc* __restrict__ src, const uint32_t* __restrict__ rows, uint32_t n, uint64_t len,
+                          Fr* __restrict__ out) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += stride) {
-        E acc = F::zero();
+        Fr total = fr_zero();
+        frw::RowAcc acc = frw::rowacc_zero();
+        uint32_t terms = 0;
         for (uint32_t j = 0; j < n; j++) {
             const LinCombSrc s = src[j];
-            if (i < s.len) acc = F::add(acc, F::mul(coeff[j], F::load(s.ptr, s.dtype, i)));
+            if (i >= s.len) continue;
+            if (terms + 8 > kRowTerms) {
+                total = fr_add(total, frw::to_fr(frw::reduce_rows(acc.E, acc.O)));
+                acc = frw::rowacc_zero();
+                terms = 0;
+            }
+            const uint32_t* row = rows + (size_t)j * kLinRows * 8;
+            if (s.dtype == DPB_FR) {
+                const frw::F8 v = frw::from_fr(FrFam::load(s.ptr, DPB_FR, i));
+#pragma unroll
+                for (int w = 0; w < 8; w++) lincomb_row_mac(acc, row + 8 * w, v.w[w]);
+                terms += 8;
+            } else {
+                const int64_t x = s.dtype == DPB_FR_I32 ? (int64_t)((const int32_t*)s.ptr)[i] : ((const int64_t*)s.ptr)[i];
+                const uint64_t mag = x < 0 ? (uint64_t)0 - (uint64_t)x : (uint64_t)x;
+                if (x < 0) row += 8;
+                lincomb_row_mac(acc, row, (uint32_t)mag);
+                if (mag >> 32) lincomb_row_mac(acc, row + 16, (uint32_t)(mag >> 32));
+                terms += 2;
+            }
         }
-        F::store(out, i, acc);
+        FrFam::store(out, i, fr_add(total, frw::to_fr(frw::reduce_rows(acc.E, acc.O))));
+    }
+}
+// Goldilocks: the products are added up unreduced
+__global__ void __launch_bounds__(kThreads)
+    linear_combination_gl(const LinCombSrc* __restrict__ src, const Gl2* __restrict__ coeff, uint32_t n, uint64_t len,
+                          Gl2* __restrict__ out) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += stride) {
+        EntrySum<GlFam, false> acc;
+        acc.zero();
+        for (uint32_t j = 0; j < n; j++) {
+            const LinCombSrc s = src[j];
+            if (i < s.len) acc.mac(coeff[j], s.ptr, s.dtype, i);
+        }
+        GlFam::store(out, i, acc.finish());
     }
 }
 
