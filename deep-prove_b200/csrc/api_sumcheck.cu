@@ -17,6 +17,8 @@
 #include "fused_int.cuh"
 #include "generic_round.cuh"
 #include "comm.cuh"
+#include "eq_pairs.cuh"
+#include "eq_pairs.hpp"
 
 namespace dpb {
 
@@ -53,6 +55,7 @@ struct dpb_sc {
     // one-pass generic rounds (generic_round.cuh); off when the tables' slots do not fit in shared memory
     // zero-padded tables: each term is evaluated over the pairs where all its padded factors hold data
     bool ranged = false;
+    EqPairPlan eqp;  // zero-padded sumchecks over  sum_t c_t * table_t * eq_t: rounds of eq_pairs.cuh
     uint64_t* d_tile_prefix = nullptr;  // [n][n_terms + 1]
     uint64_t* d_term_pairs = nullptr;   // [n][n_terms]
     std::vector<uint64_t> total_tiles;  // per round
@@ -152,6 +155,54 @@ static void build_terms(const dpb_sc* sc, const dpb_term* terms, std::vector<uin
 
 // entries a zero-padded table holds in round i (it keeps one entry once all its own variables are bound)
 static uint64_t padded_entries(const MleTrack& t, uint32_t i) { return t.nv > i ? 1ull << (t.nv - i) : 1ull; }
+
+// A zero-padded sumcheck whose terms are all  c * table * eq table,  the two of one size, every table of the list in
+// exactly one term and every eq table tagged with its point (dpb_eq_table / dpb_eq_tables), runs the rounds of
+// eq_pairs.cuh.  Everything else stays with the general kernels: a table shared by terms would have to be bound once
+// for several tiles, and an untagged table need not be an eq table.
+static void plan_eq_pairs(dpb_sc* sc, dpb_mle* const* mles, const dpb_term* terms) {
+    if (!sc->ranged || sc->d != 2 || (uint64_t)sc->k != 2 * (uint64_t)sc->n_terms) return;
+    const size_t es = sc->gl ? 16 : 32;
+    std::vector<bool> used(sc->k, false);
+    std::vector<EqPairPlan::Term> list(sc->n_terms);
+    for (uint32_t t = 0; t < sc->n_terms; t++) {
+        if (terms[t].n_factors != 2) return;
+        uint32_t a = terms[t].idx[0], b = terms[t].idx[1];
+        if (used[a] || used[b] || a == b || sc->tr[a].nv != sc->tr[b].nv) return;
+        // a table below the sumcheck's variables that is not padded is a function of the last variables: not this form
+        if (sc->tr[a].nv < sc->n && (!sc->tr[a].padded || !sc->tr[b].padded)) return;
+        used[a] = used[b] = true;
+        const size_t point = (size_t)sc->tr[a].nv * es;
+        if (mles[b]->eq_point.size() != point || sc->tr[b].dtype != (sc->gl ? DPB_GL_EXT : DPB_FR)) std::swap(a, b);
+        if (mles[b]->eq_point.size() != point || sc->tr[b].dtype != (sc->gl ? DPB_GL_EXT : DPB_FR)) return;
+        list[t].f = a;
+        list[t].eq = b;
+    }
+    sc->eqp.terms = std::move(list);
+}
+
+// Per-round tiles of eq_pairs_round: [rounds][n_terms + 1] first tiles.  A thread takes up to kEqPairsPerThread pairs of
+// a tile, fewer while that would leave fewer than four tiles per SM.
+static void plan_eq_pair_tiles(dpb_sc* sc, std::vector<uint32_t>& prefix) {
+    const uint32_t T = (uint32_t)sc->eqp.terms.size();
+    prefix.resize((size_t)sc->n * (T + 1));
+    for (uint32_t i = 0; i < sc->n; i++) {
+        uint64_t pairs = 0;
+        for (const auto& t : sc->eqp.terms) pairs += sc->tr[t.f].nv > i ? 1ull << (sc->tr[t.f].nv - i - 1) : 1;
+        uint32_t per = 1;
+        while (per < kEqPairsPerThread && pairs >= (uint64_t)sc->ctx->sm_count * 4 * kThreads * 2 * per) per *= 2;
+        uint32_t run = 0;
+        for (uint32_t t = 0; t < T; t++) {
+            prefix[(size_t)i * (T + 1) + t] = run;
+            const uint32_t nv = sc->tr[sc->eqp.terms[t].f].nv;
+            const uint64_t items = nv > i ? 1ull << (nv - i - 1) : 1;
+            run += (uint32_t)((items + (uint64_t)kThreads * per - 1) / ((uint64_t)kThreads * per));
+        }
+        prefix[(size_t)i * (T + 1) + T] = run;
+        sc->eqp.per_thread.push_back(per);
+        sc->eqp.tiles.push_back(run);
+    }
+}
 
 template <class F, int D>
 static void launch_eval_ranged(dpb_sc* sc, uint32_t round) {
@@ -1027,6 +1078,9 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
     bool done = false;
     if (use_tail) {
         // the sums are already in raw
+    } else if (!sc->eqp.terms.empty()) {
+        eq_pairs_launch_round<F>(ctx, sc->eqp, i, r);
+        done = true;
     } else if (sc->fused_shape == kFusedProduct) {
         launch_fused(ctx, sc->h_desc.data() + (size_t)i * sc->k, i > 0 ? sc->h_fold.data() + (size_t)i * sc->k : nullptr,
                      sc->k, i, r, n_pairs);
@@ -1112,7 +1166,7 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
         E* coeffs = (E*)sc->prev_coeffs;
         E claim = F::zero();
         if (i > 0) claim = eval_coeffs<F>((int)sc->d, coeffs, r);
-        samples_to_evals<F>((int)sc->d, raw, i == 0, claim, (E*)out_evals, coeffs);
+        samples_to_evals<F>((int)sc->d, raw, i == 0 || !sc->eqp.terms.empty(), claim, (E*)out_evals, coeffs);
         memcpy(sc->prev_evals, out_evals, msg_bytes);
     } else {
         if (split) {
@@ -1137,7 +1191,15 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
         uint64_t bytes = 0;
         const char* name;
         const bool seg = sc->seg_ok && sc->d >= 2 && sc->d <= 4;
-        if (i == 0) {
+        if (!sc->eqp.terms.empty()) {
+            for (const auto& t : sc->eqp.terms) {
+                const uint32_t nv = sc->tr[t.f].nv, v = nv > i ? nv - i : 0;
+                bytes += (i == 0 ? dtype_size(sc->tr[t.f].dtype) << v
+                                 : (i == 1 ? 2 * dtype_size(sc->tr[t.f].dtype) : 2 * sizeof(E)) << v) +
+                         (i == 0 ? 0 : sizeof(E) << v) + (sizeof(E) << v) + (v ? sizeof(E) << (v - 1) : 0);
+            }
+            name = "eq_pairs_round";
+        } else if (i == 0) {
             for (uint32_t j = 0; j < sc->k; j++) bytes += dtype_size(sc->tr[j].dtype) << sc->tr[j].nv;
             name = done ? (sc->tr[0].dtype == DPB_GL_BASE ? "fused_eval0<base>"
                            : sc->tr[0].dtype == DPB_FR_I32 ? "fused_eval0<i32>" : "fused_eval0")
@@ -1183,8 +1245,11 @@ static int run_finish(dpb_sc* sc, const void* last_challenge, void* out) {
     dpb_ctx* ctx = sc->ctx;
     E r;
     memcpy(&r, last_challenge, sizeof(E));
-    sc_final_evals<F><<<(sc->k + 127) / 128, 128, 0, ctx->stream>>>(
-        sc->d_desc + (size_t)(sc->n - 1) * sc->k, sc->k, r, (E*)sc->d_final);
+    if (!sc->eqp.terms.empty())
+        eq_pairs_launch_finals<F>(ctx, sc->eqp, sc->n - 1, r, (E*)sc->d_final);
+    else
+        sc_final_evals<F><<<(sc->k + 127) / 128, 128, 0, ctx->stream>>>(
+            sc->d_desc + (size_t)(sc->n - 1) * sc->k, sc->k, r, (E*)sc->d_final);
     DPB_CUDA(cudaGetLastError());
     ctx->sumcheck_launches++;
     DPB_CUDA(cudaMemcpyAsync(out, sc->d_final, sc->k * sizeof(E), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1291,7 +1356,17 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
     // [fold buffers | table descriptors | fold descriptors | terms | final values | round tables | groups | program]
     std::vector<uint8_t> h_terms, h_groups, h_prog, h_segs, h_seg_prog;
     TracePhase t_plan("sumcheck.begin.plan");
-    if (gl) {
+    plan_eq_pairs(sc, mles, terms);
+    const bool eqp = !sc->eqp.terms.empty();
+    std::vector<uint32_t> h_eqp_prefix;
+    std::vector<uint8_t> h_eqp_points;
+    if (eqp) {
+        plan_eq_pair_tiles(sc, h_eqp_prefix);
+        for (const auto& t : sc->eqp.terms) h_eqp_points.insert(h_eqp_points.end(), mles[t.eq]->eq_point.begin(), mles[t.eq]->eq_point.end());
+    }
+    if (eqp) {
+        // no term list, no descriptors: the plan above says it all
+    } else if (gl) {
         build_terms<GlFam>(sc, terms, h_terms);
         if (!sc->ranged) plan_program<GlFam>(sc, terms, mles, h_groups, h_prog, h_segs, h_seg_prog);
     } else {
@@ -1300,7 +1375,7 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
     }
     // ranged evaluation: per round and term, the pairs to visit and the tiles that cover them
     std::vector<uint64_t> h_tile_prefix, h_term_pairs;
-    if (sc->ranged) {
+    if (sc->ranged && !eqp) {
         h_tile_prefix.resize((size_t)num_vars * (n_terms + 1));
         h_term_pairs.resize((size_t)num_vars * n_terms);
         sc->total_tiles.assign(num_vars, 0);
@@ -1328,13 +1403,15 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
         off = (off + bytes + 15) & ~(size_t)15;
         return o;
     };
-    const size_t nk = (size_t)num_vars * k;
+    const size_t nk = eqp ? 0 : (size_t)num_vars * k;
     const size_t o_desc = take(nk * sizeof(MleDesc)), o_fold = take(nk * sizeof(FoldDesc)), o_terms = take(h_terms.size()),
                  o_final = take(k * es), o_rtab = take(sc->has_prog ? nk * sizeof(RoundTab) : 0),
                  o_groups = take(h_groups.size()), o_prog = take(h_prog.size()),
                  o_tiles = take(h_tile_prefix.size() * 8), o_pairs = take(h_term_pairs.size() * 8),
                  o_rtab_eq = take(sc->spliteq ? nk * sizeof(RoundTab) : 0), o_segs = take(h_segs.size()),
-                 o_seg_prog = take(h_seg_prog.size());
+                 o_seg_prog = take(h_seg_prog.size()), o_eqp_terms = take(sc->eqp.terms.size() * sizeof(EqPairTerm)),
+                 o_eqp_points = take(h_eqp_points.size()), o_eqp_prefix = take(h_eqp_prefix.size() * 4),
+                 upload_end = off, o_eqp_s = take(2 * sc->eqp.terms.size() * es);
     t_plan.stop();
     TracePhase t_alloc("sumcheck.begin.alloc");
     // Sumchecks of one context run one after the other, each with one block of device memory for its fold buffers
@@ -1373,6 +1450,10 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
         sc->d_seg_prog = base + o_seg_prog;
         sc->d_tile_prefix = (uint64_t*)(base + o_tiles);
         sc->d_term_pairs = (uint64_t*)(base + o_pairs);
+        sc->eqp.d_terms = base + o_eqp_terms;
+        sc->eqp.d_points = base + o_eqp_points;
+        sc->eqp.d_prefix = (const uint32_t*)(base + o_eqp_prefix);
+        sc->eqp.d_s = base + o_eqp_s;
         // ping-pong fold buffers of every table, at the front of the block
         char* p = base;
         for (uint32_t j = 0; j < k; j++) {
@@ -1385,11 +1466,11 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
         }
     }
     // descriptors for every round
-    sc->h_desc.resize((size_t)num_vars * k);
-    sc->h_fold.resize((size_t)num_vars * k);
+    sc->h_desc.resize(nk);
+    sc->h_fold.resize(nk);
     sc->n_fold.assign(num_vars, 0);
     sc->max_fold_out.assign(num_vars, 0);
-    for (uint32_t i = 0; i < num_vars; i++) {
+    for (uint32_t i = 0; i < num_vars && !eqp; i++) {
         const uint32_t v = num_vars - i;
         for (uint32_t j = 0; j < k; j++) {
             const void* ptr;
@@ -1430,7 +1511,7 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
         return code;
     };
     {
-        std::vector<uint8_t> blob(off - o_desc, 0);
+        std::vector<uint8_t> blob(upload_end - o_desc, 0);
         auto put = [&](size_t o, const void* src, size_t bytes) {
             if (bytes) memcpy(blob.data() + (o - o_desc), src, bytes);
         };
@@ -1461,6 +1542,31 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
         put(o_seg_prog, h_seg_prog.data(), h_seg_prog.size());
         put(o_tiles, h_tile_prefix.data(), h_tile_prefix.size() * 8);
         put(o_pairs, h_term_pairs.data(), h_term_pairs.size() * 8);
+        if (eqp) {
+            std::vector<EqPairTerm> et(sc->eqp.terms.size());
+            uint32_t q = 0;
+            for (uint32_t t = 0; t < n_terms; t++) {
+                const uint32_t f = sc->eqp.terms[t].f, e = sc->eqp.terms[t].eq;
+                EqPairTerm& d = et[t];
+                memset(&d, 0, sizeof d);
+                d.f = sc->tr[f].orig;
+                d.eq = sc->tr[e].orig;
+                for (int b = 0; b < 2; b++) {
+                    d.fb[b] = sc->tr[f].buf[b];
+                    d.wb[b] = sc->tr[e].buf[b];
+                }
+                d.q_off = q;
+                d.nv = (uint16_t)sc->tr[f].nv;
+                d.dtype = (uint16_t)sc->tr[f].dtype;
+                d.f_id = f;
+                d.eq_id = e;
+                memcpy(d.coeff, terms[t].coeff, es);
+                q += sc->tr[f].nv;
+            }
+            put(o_eqp_terms, et.data(), et.size() * sizeof(EqPairTerm));
+            put(o_eqp_points, h_eqp_points.data(), h_eqp_points.size());
+            put(o_eqp_prefix, h_eqp_prefix.data(), h_eqp_prefix.size() * 4);
+        }
         rc = upload_small(ctx, (char*)sc->slab + o_desc, blob.data(), blob.size());
         if (rc != DPB_OK) return cleanup(rc);
     }

@@ -59,6 +59,7 @@ struct GlFam {
     DPB_HD static bool is_one(const E& a) { return a.c0 == 1 && a.c1 == 0; }
     DPB_HD static bool is_zero(const E& a) { return a.c0 == 0 && a.c1 == 0; }
     DPB_HD static E from_u64(uint64_t x) { return gl2_make(x % GL_P, 0); }
+    DPB_HD static E from_u64_pow64() { return gl2_make(GL_EPS, 0); }  // 2^64
     static E inv(const E& a) { return gl2_inv(a); }
     DPB_HD static size_t elem_size(int dtype) { return dtype == DPB_GL_BASE ? 8 : 16; }
 #if defined(__CUDACC__)
@@ -129,6 +130,7 @@ struct FrFam {
     DPB_HD static bool is_one(const E& a) { return fr_eq(a, fr_one()); }
     DPB_HD static bool is_zero(const E& a) { return fr_is_zero(a); }
     DPB_HD static E from_u64(uint64_t x) { return fr_from_u64(x); }
+    DPB_HD static E from_u64_pow64() { return fr_fixed_power(8); }  // 2^64: 2^320 mod r is its Montgomery form
     static E inv(const E& a) { return fr_inv(a); }
     DPB_HD static size_t elem_size(int) { return 32; }
 #if defined(__CUDACC__)

@@ -234,14 +234,7 @@ __device__ __forceinline__ Fr fr_intacc_finish(const FrIntAcc& acc) {
 }
 
 // Sum of full products, reduced once: see frw::Wide.
-__device__ __forceinline__ Fr fr_wide_finish(const frw::Wide& s) {
-    frw::F8 lo, mid, top, one;
-    frw::wide_split(s, lo, mid, top);
-#pragma unroll
-    for (int i = 0; i < 8; i++) one.w[i] = i ? 0 : 1;
-    const frw::F8 a = frw::mul(lo, one), b = frw::mul(mid, frw::from_fr(fr_one())), c = frw::mul(top, frw::from_fr(fr_rr()));
-    return frw::to_fr(frw::add(frw::add(a, b), c));
-}
+__device__ __forceinline__ Fr fr_wide_finish(const frw::Wide& s) { return frw::to_fr(frw::wide_reduce(s)); }
 
 // Integer -> Montgomery form without a full product: |x| = lo + 2^32 hi, and x R = lo * (+-R) + hi * (+-2^32 R)
 // mod r; the rows below hold those four constants times 2^64 (what frw::lin2_rows divides out again).

@@ -114,6 +114,15 @@ __device__ __forceinline__ void mont_step(uint32_t* P, uint32_t* Q, const uint32
     else chain_mod_odd<false>(Q + I + 1, Q[I + 9], m, 0);
 }
 
+// the reduction half of mont_step
+template <int I>
+__device__ __forceinline__ void redc_step(uint32_t* P, uint32_t* Q) {
+    const uint32_t m = (I ? P[I] + Q[I] : P[I]) * DPB_FRW_INV;
+    chain_mod_even(P + I, P[I + 8], m);
+    if (I) chain_mod_odd<true>(Q + I + 1, Q[I + 9], m, Q[I]);
+    else chain_mod_odd<false>(Q + I + 1, Q[I + 9], m, 0);
+}
+
 // a < 2r -> a mod r: subtract r; on a borrow add it back through a mask
 __device__ __forceinline__ F8 reduce_once(const F8& a) {
     F8 d;
@@ -338,15 +347,69 @@ __device__ __forceinline__ void wide_mac(Wide& s, const F8& a, const F8& b) {
     add16(E);
     add16(O);
 }
-// the sum divided by 2^256 mod r (the Montgomery form of the sum of the products of Montgomery forms): with
-// lo + 2^256 mid + 2^512 top the three parts are the Montgomery products of lo with 1, mid with 2^256 and top with 2^512
-__device__ __forceinline__ void wide_split(const Wide& s, F8& lo, F8& mid, F8& top) {
+// a - k if that does not borrow, else a
+__device__ __forceinline__ F8 sub_if_not_below(const F8& a, uint32_t k0, uint32_t k1, uint32_t k2, uint32_t k3, uint32_t k4,
+                                               uint32_t k5, uint32_t k6, uint32_t k7) {
+    F8 d;
+    uint32_t below;
+    asm("sub.cc.u32 %0, %9, %17; subc.cc.u32 %1, %10, %18; subc.cc.u32 %2, %11, %19; subc.cc.u32 %3, %12, %20;\n\t"
+        "subc.cc.u32 %4, %13, %21; subc.cc.u32 %5, %14, %22; subc.cc.u32 %6, %15, %23; subc.cc.u32 %7, %16, %24;\n\t"
+        "subc.u32 %8, 0, 0;"
+        : "=&r"(d.w[0]), "=&r"(d.w[1]), "=&r"(d.w[2]), "=&r"(d.w[3]), "=&r"(d.w[4]), "=&r"(d.w[5]), "=&r"(d.w[6]),
+          "=&r"(d.w[7]), "=&r"(below)
+        : "r"(a.w[0]), "r"(a.w[1]), "r"(a.w[2]), "r"(a.w[3]), "r"(a.w[4]), "r"(a.w[5]), "r"(a.w[6]), "r"(a.w[7]), "r"(k0),
+          "r"(k1), "r"(k2), "r"(k3), "r"(k4), "r"(k5), "r"(k6), "r"(k7));
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        lo.w[i] = s.w[i];
-        mid.w[i] = s.w[8 + i];
-        top.w[i] = i ? 0 : s.w[16];
+    for (int i = 0; i < 8; i++) d.w[i] = below ? a.w[i] : d.w[i];
+    return d;
+}
+// any 256-bit value mod r (it is below 6r): less 4r, 2r, r where that does not go below zero
+__device__ __forceinline__ F8 reduce_256(F8 a) {
+    a = sub_if_not_below(a, 0xc0000004u, 0x0f87d64fu, 0xe6e5c245u, 0xa0cfa121u, 0x06056174u, 0xe14116dau, 0x84c680a6u, 0xc19139cbu);
+    a = sub_if_not_below(a, 0xe0000002u, 0x87c3eb27u, 0xf372e122u, 0x5067d090u, 0x0302b0bau, 0x70a08b6du, 0xc2634053u, 0x60c89ce5u);
+    return reduce_once(a);
+}
+// The sum divided by 2^256 mod r (the Montgomery form of the sum of the products of Montgomery forms).  The low eight
+// words take a Montgomery reduction of their own (64 multiply-adds, result at most r); to it come the next eight and
+// the rest above 2^256, a count of overflows that is zero for up to 16 products: top * 2^512 / 2^256.
+__device__ __forceinline__ F8 mul(const F8& a, const F8& b);
+__device__ __forceinline__ F8 add(const F8& a, const F8& b);
+__device__ __forceinline__ F8 wide_reduce(const Wide& s) {
+    uint32_t E[18], O[18];
+#pragma unroll
+    for (int i = 0; i < 18; i++) {
+        E[i] = i < 8 ? s.w[i] : 0;
+        O[i] = 0;
     }
+    redc_step<0>(E, O);
+    redc_step<1>(O, E);
+    redc_step<2>(E, O);
+    redc_step<3>(O, E);
+    redc_step<4>(E, O);
+    redc_step<5>(O, E);
+    redc_step<6>(E, O);
+    redc_step<7>(O, E);
+    F8 v;
+    uint32_t top;
+    asm("add.cc.u32 %0, %9, %17; addc.cc.u32 %1, %10, %18; addc.cc.u32 %2, %11, %19; addc.cc.u32 %3, %12, %20;\n\t"
+        "addc.cc.u32 %4, %13, %21; addc.cc.u32 %5, %14, %22; addc.cc.u32 %6, %15, %23; addc.u32 %7, %16, %24;\n\t"
+        "add.cc.u32 %0, %0, %25; addc.cc.u32 %1, %1, %26; addc.cc.u32 %2, %2, %27; addc.cc.u32 %3, %3, %28;\n\t"
+        "addc.cc.u32 %4, %4, %29; addc.cc.u32 %5, %5, %30; addc.cc.u32 %6, %6, %31; addc.cc.u32 %7, %7, %32; addc.u32 %8, %33, 0;"
+        : "=&r"(v.w[0]), "=&r"(v.w[1]), "=&r"(v.w[2]), "=&r"(v.w[3]), "=&r"(v.w[4]), "=&r"(v.w[5]), "=&r"(v.w[6]),
+          "=&r"(v.w[7]), "=&r"(top)
+        : "r"(E[8]), "r"(E[9]), "r"(E[10]), "r"(E[11]), "r"(E[12]), "r"(E[13]), "r"(E[14]), "r"(E[15]), "r"(O[8]),
+          "r"(O[9]), "r"(O[10]), "r"(O[11]), "r"(O[12]), "r"(O[13]), "r"(O[14]), "r"(O[15]), "r"(s.w[8]), "r"(s.w[9]),
+          "r"(s.w[10]), "r"(s.w[11]), "r"(s.w[12]), "r"(s.w[13]), "r"(s.w[14]), "r"(s.w[15]), "r"(s.w[16]));
+    v = reduce_256(v);
+    if (top) {
+        F8 t, rr;
+#pragma unroll
+        for (int i = 0; i < 8; i++) t.w[i] = i ? 0 : top;
+        rr.w[0] = 0xae216da7u; rr.w[1] = 0x1bb8e645u; rr.w[2] = 0xe35c59e3u; rr.w[3] = 0x53fe3ab1u;
+        rr.w[4] = 0x53bb8085u; rr.w[5] = 0x8c49833du; rr.w[6] = 0x7f4e44a5u; rr.w[7] = 0x0216d0b1u;
+        v = add(v, mul(t, rr));
+    }
+    return v;
 }
 
 __device__ __forceinline__ F8 add(const F8& a, const F8& b) {
