@@ -468,7 +468,7 @@ static void plan_program(dpb_sc* sc, const dpb_term* terms, dpb_mle* const* mles
         memcpy(sc->lag_w, weights[sc->d], (sc->d + 1) * sizeof(E));
     }
     if (sc->k <= kTailMaxTables) {
-        // shared memory of the resident kernel: [program copy | round descriptors | slots or sum tree]
+        // shared memory of the resident kernel: [program copy | round descriptors | two sets of slots]
         const size_t prog_bytes = h_prog.size() + h_groups.size();
         sc->tail_prog_in_smem = prog_bytes <= (size_t)kTailProgBytes;
         size_t off = sc->tail_prog_in_smem ? prog_bytes : 0;
@@ -479,10 +479,11 @@ static void plan_program(dpb_sc* sc, const dpb_term* terms, dpb_mle* const* mles
         // pairs per round the kernel can take: two items per thread in the evaluation phase, and the slots must fit
         uint64_t max_pairs = 256;
         while (max_pairs * (sc->d + 1) > 2 * (uint64_t)kTailThreads) max_pairs >>= 1;
-        const size_t per_pair = std::max<size_t>((size_t)sc->k * 2, sc->d + 1) * sizeof(E);
-        while (max_pairs >= 1 && off + per_pair * max_pairs > (size_t)kOnePassMaxSmem) max_pairs >>= 1;
+        // the slots of its first round and, half as many, those of the next
+        const size_t per_pair = (size_t)sc->k * 2 * sizeof(E);
+        while (max_pairs >= 1 && off + per_pair * (max_pairs + (max_pairs + 1) / 2) > (size_t)kOnePassMaxSmem) max_pairs >>= 1;
         if (max_pairs >= 1) {
-            sc->tail_smem = off + per_pair * max_pairs;
+            sc->tail_smem = off + per_pair * (max_pairs + (max_pairs + 1) / 2);
             uint32_t i = 0;
             while (i < sc->n && (1ull << (sc->n - i - 1)) > max_pairs) i++;
             sc->tail_start = i;
