@@ -19,6 +19,7 @@
 #include "comm.cuh"
 #include "eq_pairs.cuh"
 #include "eq_pairs.hpp"
+#include "logup_tail.hpp"
 
 namespace dpb {
 
@@ -94,6 +95,13 @@ struct dpb_sc {
     void* d_logup = nullptr;     // [LogupConsts[n] | LogupInst[n]] (own allocation)
     uint32_t logup_n = 0, logup_eq = 0;
     alignas(16) uint8_t logup_lambda[32] = {0};
+    // the last rounds of a hinted logup layer (logup_tail.cuh)
+    LogupTailPlan lt;
+    bool lt_active = false;       // the running resident kernel is that one
+    uint32_t lt_first = 0;        // its first round and the challenges it got since, for playing them again
+    std::vector<uint8_t> lt_chal;
+    bool lt_have_h = false;       // the previous round's H and q are in lt_h: H(0), h1, h2, q
+    alignas(16) uint8_t lt_h[4 * 32] = {0};
     bool seg_ok = false;         // the program splits into segments over few tables each: sc_round_seg runs the large rounds
     void* d_segs = nullptr;
     void* d_seg_prog = nullptr;
@@ -349,33 +357,8 @@ static void plan_spliteq(dpb_sc* sc, dpb_mle* const* mles, const std::vector<Pro
         if (!have) return;  // nothing moves in some round: leave it to the direct kernels
         if (F::is_zero(rq[i]) || F::is_zero(F::sub(one, rq[i]))) return;
     }
-    // inverses: one field inversion for all of them (Montgomery's trick)
-    std::vector<E> vals;  // the values to invert: per round q, per lead the prefix products of (1 - q_k)
-    for (uint32_t i = 0; i < sc->n; i++) vals.push_back(rq[i]);
-    for (auto& l : leads) {
-        E zp = one;
-        vals.push_back(zp);
-        for (uint32_t k = 0; k < l.vars; k++) {
-            E q;
-            memcpy(&q, l.q.data() + (size_t)k * sizeof(E), sizeof(E));
-            zp = F::mul(zp, F::sub(one, q));
-            vals.push_back(zp);
-        }
-    }
-    std::vector<E> pre(vals.size() + 1, one);
-    for (size_t a = 0; a < vals.size(); a++) pre[a + 1] = F::mul(pre[a], vals[a]);
-    E inv_all = F::inv(pre[vals.size()]);
-    std::vector<E> inv(vals.size());
-    for (size_t a = vals.size(); a-- > 0;) {
-        inv[a] = F::mul(inv_all, pre[a]);
-        inv_all = F::mul(inv_all, vals[a]);
-    }
     sc->round_q.assign((const uint8_t*)rq.data(), (const uint8_t*)rq.data() + sc->n * sizeof(E));
-    sc->round_inv_q.assign((const uint8_t*)inv.data(), (const uint8_t*)inv.data() + sc->n * sizeof(E));
-    size_t at = sc->n;
     for (auto& l : leads) {
-        l.inv_zp.assign((const uint8_t*)(inv.data() + at), (const uint8_t*)(inv.data() + at) + (l.vars + 1) * sizeof(E));
-        at += l.vars + 1;
         memcpy(l.S, &one, sizeof(E));
         memcpy(l.S_prev, &one, sizeof(E));
     }
@@ -394,6 +377,41 @@ static void plan_spliteq(dpb_sc* sc, dpb_mle* const* mles, const std::vector<Pro
     sc->eq_leads = std::move(leads);
     sc->group_lead = std::move(group_lead);
     sc->spliteq = true;
+}
+
+// The inverses the split-eq rounds need, made when the first of them is needed: a sumcheck whose rounds all run in the
+// resident kernel makes them while that kernel computes.  One field inversion for all (Montgomery's trick).
+template <class F>
+static void spliteq_inverses(dpb_sc* sc) {
+    typedef typename F::E E;
+    if (!sc->round_inv_q.empty()) return;
+    const E one = F::one();
+    std::vector<E> vals(sc->n);  // the values to invert: per round q, per lead the prefix products of (1 - q_k)
+    memcpy(vals.data(), sc->round_q.data(), sc->n * sizeof(E));
+    for (auto& l : sc->eq_leads) {
+        E zp = one;
+        vals.push_back(zp);
+        for (uint32_t k = 0; k < l.vars; k++) {
+            E q;
+            memcpy(&q, l.q.data() + (size_t)k * sizeof(E), sizeof(E));
+            zp = F::mul(zp, F::sub(one, q));
+            vals.push_back(zp);
+        }
+    }
+    std::vector<E> pre(vals.size() + 1, one);
+    for (size_t a = 0; a < vals.size(); a++) pre[a + 1] = F::mul(pre[a], vals[a]);
+    E inv_all = F::inv(pre[vals.size()]);
+    std::vector<E> inv(vals.size());
+    for (size_t a = vals.size(); a-- > 0;) {
+        inv[a] = F::mul(inv_all, pre[a]);
+        inv_all = F::mul(inv_all, vals[a]);
+    }
+    sc->round_inv_q.assign((const uint8_t*)inv.data(), (const uint8_t*)inv.data() + sc->n * sizeof(E));
+    size_t at = sc->n;
+    for (auto& l : sc->eq_leads) {
+        l.inv_zp.assign((const uint8_t*)(inv.data() + at), (const uint8_t*)(inv.data() + at) + (l.vars + 1) * sizeof(E));
+        at += l.vars + 1;
+    }
 }
 
 // Host-side plan of the one-pass rounds and the resident kernel: the grouped term
@@ -489,9 +507,8 @@ static void plan_program(dpb_sc* sc, const dpb_term* terms, dpb_mle* const* mles
             sc->tail_start = i;
         }
     }
-    // split-eq form for the rounds before the resident kernel's; a sumcheck that is all "last rounds" skips the
-    // planning (it costs a field inversion on the host)
-    if (sc->tail_start > 0) plan_spliteq<F>(sc, mles, groups, prog);
+    // split-eq form for the rounds before the resident kernel's, and for a logup layer (degree 3) for all of them
+    if (sc->tail_start > 0 || sc->d == 3) plan_spliteq<F>(sc, mles, groups, prog);
 }
 
 // per-round descriptors of the one-pass kernels: which tables are bound inside the round's kernel
@@ -591,6 +608,7 @@ static int launch_spliteq(dpb_sc* sc, uint32_t round, uint64_t n_pairs, const ty
     dpb_ctx* ctx = sc->ctx;
     SplitEqArgs<F> eq;
     memset(&eq, 0, sizeof eq);
+    spliteq_inverses<F>(sc);
     for (size_t a = 0; a < sc->eq_leads.size(); a++) {
         const auto& l = sc->eq_leads[a];
         if (round < l.first_active) {
@@ -668,6 +686,7 @@ static int spliteq_materialize(dpb_sc* sc, uint32_t i) {
     typedef typename F::E E;
     dpb_ctx* ctx = sc->ctx;
     if (i == 0) return DPB_OK;
+    spliteq_inverses<F>(sc);
     for (const auto& l : sc->eq_leads) {
         if (i - 1 < l.first_active) continue;
         const uint32_t f = i - 1 - l.first_active;  // variables bound in the table of round i - 1
@@ -703,7 +722,12 @@ static int tail_wait_host(dpb_ctx* ctx, TailBox* box, Ready ready) {
     std::chrono::steady_clock::time_point t0;
     while (!ready()) {
         if (box->status == 3) return kTailNoHost;
-        if (box->status == 2) return kTailGaveUp;
+        if (box->status == 2) {
+            // the host may have been held up between the two looks: what it waits for can have come first
+            std::atomic_thread_fence(std::memory_order_acquire);
+            if (ready()) break;
+            return kTailGaveUp;
+        }
         if ((++spins & 0xFFF) == 0) {
             cudaError_t e = cudaStreamQuery(ctx->tail_stream);
             if (e != cudaSuccess && e != cudaErrorNotReady)
@@ -867,6 +891,172 @@ static int tail_finish(dpb_sc* sc, const void* last_challenge, void* out) {
     return rc;
 }
 
+// ---- resident last rounds of a logup layer: host side -------------------------------
+
+// (Re)starts the kernel at its first round; r is the challenge that ended the round before.
+template <class F>
+static int lt_start_kernel(dpb_sc* sc, const typename F::E& r) {
+    typedef typename F::E E;
+    dpb_ctx* ctx = sc->ctx;
+    TailBox* box = (TailBox*)ctx->tail_box_host;
+    memset(box, 0, sizeof(TailBox));
+    std::atomic_thread_fence(std::memory_order_seq_cst);
+    DPB_CUDA(cudaEventRecord(ctx->tail_ev[0], ctx->stream));
+    DPB_CUDA(cudaStreamWaitEvent(ctx->tail_stream, ctx->tail_ev[0], 0));
+    const auto& lead = sc->eq_leads[0];
+    E lam;
+    memcpy(&lam, sc->logup_lambda, sizeof(E));
+    DPB_TRY(logup_tail_launch<F>(ctx, sc->lt, sc->d_rtab_eq + (size_t)sc->lt_first * sc->k, sc->tr[lead.table].orig,
+                                 sc->lt_first + 1, lam, r, sc->lt_first, sc->n));
+    ((volatile TailChunk*)&box->hello)->seq = 1;
+    DPB_CUDA(cudaEventRecord(ctx->tail_ev[1], ctx->tail_stream));
+    ctx->sumcheck_launches++;
+    return DPB_OK;
+}
+
+// the samples of round j: H(0), H(1) (round 0 only) and H at infinity, without the eq table's scalar
+template <class F>
+static int lt_take(dpb_sc* sc, uint32_t j, typename F::E* raw) {
+    TailBox* box = (TailBox*)sc->ctx->tail_box_host;
+    uint32_t x = 0;
+    return tail_wait_host(sc->ctx, box, [&] {
+        while (x <= 2) {
+            if (j > 0 && x == 1) {
+                x++;
+                continue;
+            }
+            if (!tail_take<typename F::E>(box->evals, x, j + 1, &raw[x])) return false;
+            x++;
+        }
+        return true;
+    });
+}
+
+// The kernel gave up waiting (the host was held up): start it again and play the rounds before `upto` with the
+// challenges they had, and the challenge after them.
+template <class F>
+static int lt_replay(dpb_sc* sc, uint32_t upto) {
+    typedef typename F::E E;
+    dpb_ctx* ctx = sc->ctx;
+    DPB_CUDA(cudaStreamSynchronize(ctx->tail_stream));  // it has returned; make that certain
+    const E* ch = (const E*)sc->lt_chal.data();
+    DPB_TRY(lt_start_kernel<F>(sc, ch[0]));
+    for (uint32_t j = sc->lt_first; j < upto; j++) {
+        E raw[3];
+        const int rc = lt_take<F>(sc, j, raw);
+        if (rc != DPB_OK) return rc < 0 ? rc : fail(DPB_ETIMEOUT, "the resident round kernel gave up waiting for a challenge");
+        tail_post<E>((TailBox*)ctx->tail_box_host, &ch[j + 1 - sc->lt_first], j + 1);
+    }
+    return DPB_OK;
+}
+
+// Round i: posts the challenge (or starts the kernel), makes the claim while the kernel works, takes the samples and
+// turns them into the round message.  kTailNoHost: launches block the host, nothing has run.
+template <class F>
+static int lt_round(dpb_sc* sc, uint32_t i, const typename F::E& r, typename F::E* out) {
+    typedef typename F::E E;
+    dpb_ctx* ctx = sc->ctx;
+    const bool first = !sc->lt_active;
+    if (first) {
+        sc->lt_first = i;
+        sc->lt_chal.clear();
+        DPB_TRY(lt_start_kernel<F>(sc, r));
+        sc->lt_active = sc->tail_active = true;
+        ctx->tail_owner = sc;
+    } else {
+        tail_post<E>((TailBox*)ctx->tail_box_host, &r, i);
+    }
+    sc->lt_chal.insert(sc->lt_chal.end(), (const uint8_t*)&r, (const uint8_t*)&r + sizeof(E));
+    // s(0) + s(1) of this round = the previous round's polynomial at r
+    spliteq_inverses<F>(sc);
+    const E one = F::one();
+    E claim = F::zero(), q, inv_q, S, iz;
+    E* h = (E*)sc->lt_h;
+    if (i > 0) {
+        if (sc->lt_have_h) {
+            const E l = F::add(F::sub(one, h[3]), F::mul(F::sub(F::add(h[3], h[3]), one), r));
+            claim = F::mul(l, F::add(h[0], F::mul(r, F::add(h[1], F::mul(r, h[2])))));
+        } else {
+            claim = lagrange_eval<F>((int)sc->d, (const E*)sc->prev_evals, (const E*)sc->lag_w, r);
+        }
+    }
+    memcpy(&q, sc->round_q.data() + (size_t)i * sizeof(E), sizeof(E));
+    memcpy(&inv_q, sc->round_inv_q.data() + (size_t)i * sizeof(E), sizeof(E));
+    memcpy(&S, sc->eq_leads[0].S, sizeof(E));
+    memcpy(&iz, sc->eq_leads[0].inv_zp.data() + (size_t)(i + 1) * sizeof(E), sizeof(E));
+    const E kappa = F::mul(S, iz), q0 = F::sub(one, q);
+    E raw[3];
+    int rc = lt_take<F>(sc, i, raw);
+    if (rc == kTailNoHost) {
+        cudaStreamSynchronize(ctx->tail_stream);
+        ctx->tail_enabled = false;
+        sc->lt_active = sc->tail_active = false;
+        ctx->tail_owner = nullptr;
+        return rc;
+    }
+    if (rc == kTailGaveUp && !first) {
+        DPB_TRY(lt_replay<F>(sc, i));
+        rc = lt_take<F>(sc, i, raw);
+    }
+    if (rc == kTailGaveUp) return fail(DPB_ETIMEOUT, "the resident round kernel gave up waiting for a challenge");
+    if (rc != DPB_OK) return rc;
+    const E H0 = F::mul(kappa, raw[0]), Hi = F::mul(kappa, raw[2]);
+    // s(0) + s(1) = (1 - q) H(0) + q H(1)
+    const E H1 = i == 0 ? F::mul(kappa, raw[1]) : F::mul(F::sub(claim, F::mul(q0, H0)), inv_q);
+    const E h1 = F::sub(F::sub(H1, H0), Hi);
+    // H(x) = H0 + h1 x + Hi x^2 by differences; s(x) = ((1 - q) + (2 q - 1) x) H(x)
+    const E slope = F::sub(q, q0), step2 = F::add(Hi, Hi);
+    E H = H0, step = F::add(h1, Hi), l = q0;
+    for (uint32_t x = 0; x <= 3; x++) {
+        out[x] = F::mul(l, H);
+        H = F::add(H, step);
+        step = F::add(step, step2);
+        l = F::add(l, slope);
+    }
+    h[0] = H0;
+    h[1] = h1;
+    h[2] = Hi;
+    h[3] = q;
+    sc->lt_have_h = true;
+    return DPB_OK;
+}
+
+template <class F>
+static int lt_finish(dpb_sc* sc, const void* last_challenge, void* out) {
+    typedef typename F::E E;
+    dpb_ctx* ctx = sc->ctx;
+    TailBox* box = (TailBox*)ctx->tail_box_host;
+    tail_post<E>(box, last_challenge, sc->n);
+    E r;
+    memcpy(&r, last_challenge, sizeof(E));
+    sc->lt_chal.insert(sc->lt_chal.end(), (const uint8_t*)&r, (const uint8_t*)&r + sizeof(E));
+    uint32_t j = 0;
+    auto take = [&] {
+        while (j < sc->k) {
+            if (j != sc->lt.eq_table && !tail_take<E>(box->finals, j, sc->n + 1, (E*)out + j)) return false;
+            j++;
+        }
+        return true;
+    };
+    int rc = tail_wait_host(ctx, box, take);
+    if (rc == kTailGaveUp) {
+        rc = lt_replay<F>(sc, sc->n);
+        if (rc == DPB_OK) rc = tail_wait_host(ctx, box, take);
+        if (rc == kTailGaveUp) rc = fail(DPB_ETIMEOUT, "the resident round kernel gave up waiting for a challenge");
+    }
+    // later work of this context (frees, the next sumcheck) is ordered after the kernel's end
+    cudaStreamWaitEvent(ctx->stream, ctx->tail_ev[1], 0);
+    sc->lt_active = sc->tail_active = false;
+    ctx->tail_owner = nullptr;
+    if (rc != DPB_OK) return rc;
+    const auto& l = sc->eq_leads[0];
+    E q, S;
+    memcpy(&q, l.q.data() + (size_t)(sc->n - 1) * sizeof(E), sizeof(E));
+    memcpy(&S, l.S, sizeof(E));
+    ((E*)out)[l.table] = F::mul(S, eq_scalar<F>(q, r));
+    return DPB_OK;
+}
+
 // A sumcheck that is dropped before its last round: tell the kernel to leave and wait for it.
 static void tail_abort(dpb_sc* sc) {
     dpb_ctx* ctx = sc->ctx;
@@ -874,7 +1064,7 @@ static void tail_abort(dpb_sc* sc) {
     for (int i = 0; i < 4; i++) ((volatile TailChunk*)box->chal)[i].seq = kTailAbort;
     std::atomic_thread_fence(std::memory_order_seq_cst);
     cudaStreamSynchronize(ctx->tail_stream);  // bounded by the kernel's own wait limit
-    sc->tail_active = false;
+    sc->tail_active = sc->lt_active = false;
     ctx->tail_owner = nullptr;
 }
 
@@ -1052,7 +1242,22 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
         ctx->done_value = ctx->done_seq;
         ctx->chunk_out_dev = sharded ? nullptr : ctx->result_dev;
     }
+    if (i == 0 && sc->tail_start == 0 && !sc->lt.ok) sc->spliteq = false;  // every round is the generic resident kernel's
     if (sc->spliteq && i > 0) spliteq_advance<F>(sc, i, r);
+    // the last rounds of a hinted logup layer, under the same conditions as the generic resident kernel below
+    if (sc->lt_active || (sc->lt.ok && sc->spliteq && ctx->tail_enabled && !sharded && !ctx->profile && i >= sc->lt.start &&
+                          ctx->tail_owner == nullptr)) {
+        E msg[4];
+        const int rc = lt_round<F>(sc, i, r, msg);
+        if (rc != kTailNoHost) {
+            if (rc != DPB_OK) return rc;
+            sc->eq_unbound = true;
+            memcpy(out_evals, msg, msg_bytes);
+            memcpy(sc->prev_evals, msg, msg_bytes);
+            return DPB_OK;
+        }
+    }
+    sc->lt_have_h = false;
     // the last rounds go to the resident kernel (one per context at a time; not while profiling per launch)
     bool use_tail = sc->tail_active || (sc->has_prog && ctx->tail_enabled && !sharded && !ctx->profile && !sc->heavy &&
                                         i >= sc->tail_start && ctx->tail_owner == nullptr);
@@ -1625,13 +1830,31 @@ static void hint_logup_impl(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_in
         di[i].ncol = (uint16_t)inst[i].ncol;
         di[i].pad = 0;
     }
-    const size_t bytes = n_inst * (sizeof(LogupConsts<F>) + sizeof(LogupInst));
-    if (bytes > 96 * 1024) return;
+    const size_t round_bytes = n_inst * (sizeof(LogupConsts<F>) + sizeof(LogupInst));
+    if (round_bytes > 96 * 1024) return;
+    // the resident kernel's instances and constants (alpha, sep, constant), after the round kernel's
+    std::vector<LogupTailInst> ti(n_inst);
+    std::vector<E> tc(3 * (size_t)n_inst);
+    uint32_t n_tabs = 0;
+    for (uint32_t i = 0; i < n_inst; i++) {
+        ti[i].kind = (uint16_t)inst[i].kind;
+        ti[i].first = (uint16_t)inst[i].first;
+        ti[i].ncol = (uint16_t)inst[i].ncol;
+        ti[i].tab0 = (uint16_t)n_tabs;
+        n_tabs += (inst[i].kind == kLogupLookup ? 2 : 4) + (inst[i].kind != kLogupInner && inst[i].ncol == 2 ? 2 : 0);
+        memcpy(&tc[3 * i], inst[i].alpha, sizeof(E));
+        memcpy(&tc[3 * i + 1], inst[i].sep, sizeof(E));
+        memcpy(&tc[3 * i + 2], inst[i].constant, sizeof(E));
+    }
+    const size_t o_tc = (round_bytes + 15) & ~(size_t)15, o_ti = o_tc + tc.size() * sizeof(E);
+    const size_t bytes = o_ti + ti.size() * sizeof(LogupTailInst);
     void* d = nullptr;
     if (device_alloc(sc->ctx, bytes, &d) != DPB_OK) return;
-    std::vector<uint8_t> blob(bytes);
+    std::vector<uint8_t> blob(bytes, 0);
     memcpy(blob.data(), consts.data(), n_inst * sizeof(LogupConsts<F>));
     memcpy(blob.data() + n_inst * sizeof(LogupConsts<F>), di.data(), n_inst * sizeof(LogupInst));
+    memcpy(blob.data() + o_tc, tc.data(), tc.size() * sizeof(E));
+    memcpy(blob.data() + o_ti, ti.data(), ti.size() * sizeof(LogupTailInst));
     if (upload_small(sc->ctx, d, blob.data(), bytes) != DPB_OK) {
         device_free(sc->ctx, d);
         return;
@@ -1647,6 +1870,32 @@ static void hint_logup_impl(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_in
     sc->logup_eq = eq_table;
     memcpy(sc->logup_lambda, lambda, sizeof(E));
     sc->logup_ok = true;
+    // the resident kernel: the most pairs that fit, with as few of them as need be left to one block
+    if ((size_t)sc->k * (sizeof(E) / 8) > (size_t)kTailMaxTables * 4 || n_inst > kLogupTailMaxInst) return;  // the mailbox
+    LogupTailPlan& lt = sc->lt;
+    lt.n_inst = n_inst;
+    lt.n_tabs = n_tabs;
+    lt.eq_table = eq_table;
+    lt.d_consts = (char*)d + o_tc;
+    lt.d_inst = (char*)d + o_ti;
+    uint64_t best = 0;
+    for (uint32_t alone = 32; alone >= 4; alone /= 2) {
+        LogupTailPlan p = lt;
+        p.alone = alone;
+        for (uint64_t pairs = 256 * kLogupTailBlocks; pairs > best; pairs /= 2) {
+            size_t smem;
+            if (!logup_tail_blocks(p, pairs, sizeof(E), &smem)) continue;
+            // every later round fits as well: fewer pairs, or one block once `alone` pairs are left
+            if (!logup_tail_blocks(p, alone, sizeof(E), &smem)) continue;
+            best = pairs;
+            lt.alone = alone;
+        }
+    }
+    if (!best) return;
+    uint32_t i = 0;
+    while (i < sc->n && (1ull << (sc->n - i - 1)) > best) i++;
+    lt.start = i;
+    lt.ok = true;
 }
 
 void sumcheck_hint_logup(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_inst, const void* lambda, uint32_t eq_table) {
@@ -1716,6 +1965,8 @@ int dpb_sumcheck_finish(dpb_sc* sc, const void* last_challenge, void* out_final_
     if (sc->global_round != total) return fail(DPB_ESTATE, "only %u of %u rounds ran", sc->global_round, total);
     int rc;
     if (sc->log2_ranks > 0) rc = dpb_sumcheck_finish(sc->tail, last_challenge, out_final_evals);
+    else if (sc->lt_active) rc = sc->gl ? lt_finish<GlFam>(sc, last_challenge, out_final_evals)
+                                        : lt_finish<FrFam>(sc, last_challenge, out_final_evals);
     else if (sc->tail_active) rc = sc->gl ? tail_finish<GlFam>(sc, last_challenge, out_final_evals)
                                           : tail_finish<FrFam>(sc, last_challenge, out_final_evals);
     else rc = sc->gl ? run_finish<GlFam>(sc, last_challenge, out_final_evals)
