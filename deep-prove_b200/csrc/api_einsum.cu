@@ -130,12 +130,35 @@ static int einsum_impl(dpb_ctx* ctx, const int64_t* tensor, int tensor_on_device
     if (c_pad != C) cudaMemsetAsync(owner->ptr, 0, S * c_pad * sizeof(E), ctx->stream);
     const uint64_t n_outputs = S * C;
     const bool innermost_is_outer = rank > 0 && kind[rank - 1] == DPB_AXIS_OUTER;
-    if (innermost_is_outer)
-        einsum_contract_warp<F><<<grid_for(ctx, n_outputs * 32), kThreads, 0, ctx->stream>>>(
-            t_dev, kept, (const uint64_t*)d_off, (const E*)d_w, O, n_outputs, C, c_pad, (E*)owner->ptr);
-    else
-        einsum_contract_thread<F><<<grid_for(ctx, n_outputs), kThreads, 0, ctx->stream>>>(
-            t_dev, kept, (const uint64_t*)d_off, (const E*)d_w, O, n_outputs, C, c_pad, (E*)owner->ptr);
+    if (innermost_is_outer) {
+        // a block per output once its threads have two or more terms each, else a warp
+        const uint32_t group = O >= 2 * (uint64_t)kThreads ? (uint32_t)kThreads : 32u;
+        einsum_contract_strided<F><<<grid_for(ctx, n_outputs * group), kThreads, 0, ctx->stream>>>(
+            t_dev, kept, (const uint64_t*)d_off, (const E*)d_w, O, n_outputs, C, c_pad, group, (E*)owner->ptr);
+    } else {
+        // warps of a block share the outer index (at least four terms each); while that leaves SMs idle, slices of it do
+        uint32_t warps = 1;
+        while (warps < kEinsumLaneWarps && O >= 8 * (uint64_t)warps) warps *= 2;
+        const uint64_t tiles = (n_outputs + 31) / 32;
+        uint64_t slices = 1;
+        while (slices < 64 && tiles * slices * 2 <= (uint64_t)ctx->sm_count && O >= 8 * warps * slices) slices *= 2;
+        void* d_part = nullptr;
+        if (slices > 1) {
+            rc = device_alloc(ctx, slices * n_outputs * sizeof(E), &d_part);
+            if (rc != DPB_OK) {
+                free_eqs();
+                dpb_mle_free(owner);
+                return cleanup(rc);
+            }
+            to_free.push_back(d_part);
+        }
+        const dim3 grid((uint32_t)std::min<uint64_t>(tiles, (uint64_t)ctx->sm_count * 64), (uint32_t)slices);
+        einsum_contract_lanes<F><<<grid, 32 * warps, 0, ctx->stream>>>(
+            t_dev, kept, (const uint64_t*)d_off, (const E*)d_w, O, n_outputs, C, c_pad, (E*)owner->ptr, (E*)d_part);
+        if (slices > 1)
+            einsum_add_parts<F><<<grid_for(ctx, n_outputs), kThreads, 0, ctx->stream>>>((const E*)d_part, (uint32_t)slices, n_outputs,
+                                                                                         C, c_pad, (E*)owner->ptr);
+    }
     cudaError_t e = cudaGetLastError();
     // a host tensor is only read during the call: wait for its copy (device tensors need no wait)
     if (e == cudaSuccess && !tensor_on_device) e = cudaStreamSynchronize(ctx->stream);
