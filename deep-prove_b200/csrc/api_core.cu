@@ -248,7 +248,10 @@ int stage_to_device(dpb_ctx* ctx, const void* host, size_t bytes, size_t offset,
     return upload_small(ctx, *dev, host, bytes);
 }
 
-// eq(x, pt) table over m variables into freshly allocated device memory.
+static uint32_t eq_small_blocks(uint32_t m) { return m > 7 ? 1u << (m - 7) : 1u; }
+
+// eq(x, pt) table over m variables into freshly allocated device memory: directly up to kEqSmallBits variables, else the
+// product of the tables of the first ten coordinates and of the rest.
 template <class F>
 static int eq_table_dev(dpb_ctx* ctx, const typename F::E* pt_dev, uint32_t m,
                         typename F::E** out) {
@@ -256,21 +259,23 @@ static int eq_table_dev(dpb_ctx* ctx, const typename F::E* pt_dev, uint32_t m,
     const uint64_t n = 1ull << m;
     E* res = nullptr;
     DPB_TRY(device_alloc(ctx, n * sizeof(E), (void**)&res));
-    constexpr uint32_t kDirect = 10;
-    if (m <= kDirect) {
-        eq_direct<F><<<grid_for(ctx, n), kThreads, 0, ctx->stream>>>(pt_dev, m, res);
+    constexpr uint32_t kLow = 10;
+    if (m <= kEqSmallBits) {
+        eq_small<F><<<eq_small_blocks(m), kEqSmallThreads, 0, ctx->stream>>>(pt_dev, m, res, eq_small_blocks(m), nullptr, 0, nullptr);
     } else {
-        E* lo = nullptr;
-        E* hi = nullptr;
-        DPB_TRY(device_alloc(ctx, sizeof(E) << kDirect, (void**)&lo));
-        eq_direct<F><<<grid_for(ctx, 1ull << kDirect), kThreads, 0, ctx->stream>>>(pt_dev, kDirect, lo);
-        int rc = eq_table_dev<F>(ctx, pt_dev + kDirect, m - kDirect, &hi);
+        E *lo = nullptr, *hi = nullptr;
+        const uint32_t mh = m - kLow;
+        int rc = device_alloc(ctx, sizeof(E) << kLow, (void**)&lo);
+        if (rc == DPB_OK && mh > kEqSmallBits) rc = eq_table_dev<F>(ctx, pt_dev + kLow, mh, &hi);
+        else if (rc == DPB_OK) rc = device_alloc(ctx, sizeof(E) << mh, (void**)&hi);
         if (rc != DPB_OK) {
             device_free(ctx, lo);
             device_free(ctx, res);
             return rc;
         }
-        eq_combine<F><<<grid_for(ctx, n), kThreads, 0, ctx->stream>>>(lo, kDirect, hi, n, res);
+        const uint32_t b0 = eq_small_blocks(kLow), b1 = mh <= kEqSmallBits ? eq_small_blocks(mh) : 0;
+        eq_small<F><<<b0 + b1, kEqSmallThreads, 0, ctx->stream>>>(pt_dev, kLow, lo, b0, pt_dev + kLow, mh, hi);
+        eq_combine<F><<<grid_for(ctx, n), kThreads, 0, ctx->stream>>>(lo, kLow, hi, n, res);
         device_free(ctx, lo);
         device_free(ctx, hi);
     }
@@ -319,7 +324,7 @@ static int fix_vars_impl(dpb_ctx* ctx, const void* in, int dtype_in, uint64_t le
         // high: bind the top g of the variables still free, i.e. point[k-done-g .. k-done)
         // low : bind the bottom g, i.e. point[done .. done+g)
         const E* sub = high ? pt + (k - done - g) : pt + done;
-        eq_direct<F><<<1, 32, 0, ctx->stream>>>(sub, g, w);
+        eq_small<F><<<1, kEqSmallThreads, 0, ctx->stream>>>(sub, g, w, 1, nullptr, 0, nullptr);
         const uint64_t n_out = cur_len >> g;
         E* nxt = nullptr;
         int rc = device_alloc(ctx, n_out * sizeof(E), (void**)&nxt);
