@@ -1140,7 +1140,7 @@ static void launch_fused_fr(dpb_ctx* ctx, const MleDesc* desc, const FoldDesc* f
     V2Ptrs<K> ptrs;
     const ReduceScratch<FrFam> rs = reduce_scratch<FrFam>(ctx);
     Fr* out = (Fr*)ctx->round_out;
-    const uint32_t grid = grid_for(ctx, n_pairs, 4);
+    const uint32_t grid = grid_for(ctx, n_pairs, 2);  // the blocks that are resident
     for (int j = 0; j < K; j++) {
         ptrs.in[j] = round == 0 ? desc[j].ptr : folds[j].in;
         ptrs.out[j] = round == 0 ? nullptr : folds[j].out;
@@ -1148,7 +1148,7 @@ static void launch_fused_fr(dpb_ctx* ctx, const MleDesc* desc, const FoldDesc* f
     // integer tables (DPB_FR_I32, K <= 3): round 0 in integer arithmetic, round 1 folds integers (fused_int.cuh)
     if constexpr (K <= 3) {
         if (round == 0 && desc[0].dtype == DPB_FR_I32) {
-            v2_eval0_fr_i32<K><<<grid, kThreads, 0, ctx->stream>>>(ptrs, n_pairs, rs, out);
+            v2_eval0_fr_i32<K><<<grid_for(ctx, n_pairs, 4), kThreads, 0, ctx->stream>>>(ptrs, n_pairs, rs, out);
             return;
         }
         if (round > 0 && folds[0].dtype_in == DPB_FR_I32) {
@@ -1160,7 +1160,7 @@ static void launch_fused_fr(dpb_ctx* ctx, const MleDesc* desc, const FoldDesc* f
     }
     // two resident blocks per SM: these kernels wait on their multiply chains, more warps hide that
     if (round == 0) {
-        v2_eval0<OpsFr, K, 2><<<grid, kThreads, 0, ctx->stream>>>(ptrs, n_pairs, rs, out);
+        v2_eval0_fr<K, 2><<<grid, kThreads, 0, ctx->stream>>>(ptrs, n_pairs, rs, out);
     } else {
         frw::FixedMul rk;  // the fold multiplies everything by this round's challenge: precomputed rows
         fr_fixed_table(r, rk);

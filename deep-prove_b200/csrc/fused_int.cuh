@@ -84,27 +84,25 @@ __device__ __forceinline__ Fr fold_i32(const IntFoldKey& k, int32_t a0, int32_t 
 template <int K, int MINB = 1>
 __global__ void __launch_bounds__(kThreads, MINB)
     v2_fold_eval_fr_i32(V2Ptrs<K> ptrs, IntFoldKey key, uint64_t n_pairs, ReduceScratch<FrFam> rs, Fr* out) {
-    typedef OpsFr Ops;
+    typedef Sampler<OpsFr, K, false> S;
     __shared__ IntFoldKey k;
     if (threadIdx.x < 32) ((uint32_t*)&k)[threadIdx.x] = ((const uint32_t*)&key)[threadIdx.x];
     __syncthreads();
-    Fr acc[K + 1];
+    OpsFr::Acc acc[K + 1];
 #pragma unroll
-    for (int x = 0; x <= K; x++) acc[x] = fr_zero();
+    for (int x = 0; x <= K; x++) acc[x] = OpsFr::acc_zero();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_pairs; p += stride) {
-        Fr f[2][K];
-#pragma unroll
-        for (int j = 0; j < K; j++) {
+        S s;
+        absorb_all<S, K>(s, acc, [&](int j, Fr& f0, Fr& f1) {
             const int4 a = ((const int4*)ptrs.in[j])[p];  // entries 4p .. 4p+3
-            f[0][j] = fold_i32(k, a.x, a.y);
-            f[1][j] = fold_i32(k, a.z, a.w);
-            FrFam::store(ptrs.out[j], 2 * p, f[0][j]);
-            FrFam::store(ptrs.out[j], 2 * p + 1, f[1][j]);
-        }
-        sample_pair<Ops, K, false>(acc, f[0], f[1]);
+            f0 = fold_i32(k, a.x, a.y);
+            f1 = fold_i32(k, a.z, a.w);
+            FrFam::store(ptrs.out[j], 2 * p, f0);
+            FrFam::store(ptrs.out[j], 2 * p + 1, f1);
+        });
     }
-    publish<Ops, K>(acc, rs, out);
+    publish<OpsFr, K>(acc, rs, out);
 }
 
 // Host: the four rows for the challenge r (Montgomery form).  c * 2^64 as an integer mod p is the Montgomery

@@ -27,6 +27,7 @@ namespace dpb {
 // ---- per-layout arithmetic --------------------------------------------------
 // T: value held in registers; C: the challenge; Acc: accumulator of products.
 struct OpsGlBase {
+    static constexpr bool kDeriveM1 = false;
     typedef GlFam F;
     typedef uint64_t T;
     typedef glf::Acc160 Acc;
@@ -47,6 +48,7 @@ struct OpsGlBase {
 };
 
 struct OpsGlExt {
+    static constexpr bool kDeriveM1 = false;
     typedef GlFam F;
     typedef glf::L2 T;
     struct Acc {
@@ -117,16 +119,20 @@ struct OpsGlExt2 : OpsGlExt {
     }
 };
 
+// The last product of every sample stays unreduced (frw::Wide): 64 multiply-adds instead of 128.
 struct OpsFr {
     typedef FrFam F;
     typedef Fr T;
-    typedef Fr Acc;
+    typedef frw::Wide Acc;
+    static constexpr bool kDeriveM1 = true;
     __device__ __forceinline__ static T sub_c(const T& a, const T& c) { return fr_sub(a, c); }
     __device__ __forceinline__ static T add_c(const T& a, const T& c) { return fr_add(a, c); }
     __device__ __forceinline__ static T mul(const T& a, const T& b) { return fr_mul(a, b); }
-    __device__ __forceinline__ static Acc acc_zero() { return fr_zero(); }
-    __device__ __forceinline__ static void mac(Acc& acc, const T& a, const T& b) { acc = fr_add(acc, fr_mul(a, b)); }
-    __device__ __forceinline__ static Fr finish(const Acc& acc) { return acc; }
+    __device__ __forceinline__ static Acc acc_zero() { return frw::wide_zero(); }
+    __device__ __forceinline__ static void mac(Acc& acc, const T& a, const T& b) {
+        frw::wide_mac(acc, frw::from_fr(a), frw::from_fr(b));
+    }
+    __device__ __forceinline__ static Fr finish(const Acc& acc) { return fr_wide_finish(acc); }
     __device__ __forceinline__ static void load2(const void* p, uint64_t q, T (&a)[2]) {
         a[0] = FrFam::load(p, DPB_FR, 2 * q);
         a[1] = FrFam::load(p, DPB_FR, 2 * q + 1);
@@ -194,7 +200,13 @@ struct Sampler {
             p0 = Ops::mul(p0, f0);
             if (WITH_P1) p1 = Ops::mul(p1, f1);
             pinf = Ops::mul(pinf, e);
-            if (K >= 3) pm1 = Ops::mul(pm1, m);
+            if (Ops::kDeriveM1 && WITH_P1 && K == 3) {
+                // the product of two tables is quadratic: at -1 it is 2 q(0) + 2 q(infinity) - q(1)
+                const T s = Ops::add_c(p0, pinf);
+                pm1 = Ops::sub_c(Ops::add_c(s, s), p1);
+            } else if (K >= 3) {
+                pm1 = Ops::mul(pm1, m);
+            }
             if (K >= 4) p2 = Ops::mul(p2, g);
         } else {
             Ops::mac(acc[0], p0, f0);
@@ -205,6 +217,17 @@ struct Sampler {
         }
     }
 };
+
+// absorb<J>(load(J)) for J = 0 .. K-1
+template <class S, int K, class Acc, class Load, int J = 0>
+__device__ __forceinline__ void absorb_all(S& s, Acc& acc, const Load& load) {
+    if constexpr (J < K) {
+        typename S::T f0, f1;
+        load(J, f0, f1);
+        s.template absorb<J>(acc, f0, f1);
+        absorb_all<S, K, Acc, Load, J + 1>(s, acc, load);
+    }
+}
 
 template <int K>
 struct V2Ptrs {
@@ -299,30 +322,53 @@ __global__ void __launch_bounds__(kThreads, MINB)
     publish<Ops, K>(acc, rs, out);
 }
 
+// BN254: one table after the other into the running products (few live registers), the samples' sums unreduced.
+// What bounds these kernels is the multiplier: at 2^22 (K = 3) round 0 takes three products and four unreduced ones per
+// pair, 330 -> 224 us; a later round six folds (80 multiply-adds each), three products and three unreduced ones, 250 ->
+// 214 us (from a reduction per product, and four products of two tables in round 0).
+template <int K, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB)
+    v2_eval0_fr(V2Ptrs<K> ptrs, uint64_t n_pairs, ReduceScratch<FrFam> rs, Fr* out) {
+    typedef Sampler<OpsFr, K, true> S;
+    OpsFr::Acc acc[K + 1];
+#pragma unroll
+    for (int x = 0; x <= K; x++) acc[x] = OpsFr::acc_zero();
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_pairs; p += stride) {
+        S s;
+        absorb_all<S, K>(s, acc, [&](int j, Fr& f0, Fr& f1) {
+            f0 = FrFam::load(ptrs.in[j], DPB_FR, 2 * p);
+            f1 = FrFam::load(ptrs.in[j], DPB_FR, 2 * p + 1);
+        });
+    }
+    publish<OpsFr, K>(acc, rs, out);
+}
+
 // Rounds >= 1 over BN254.
 template <int K, int MINB = 1>
 __global__ void __launch_bounds__(kThreads, MINB)
     v2_fold_eval_fr(V2Ptrs<K> ptrs, frw::FixedMul rk, uint64_t n_pairs, ReduceScratch<FrFam> rs, Fr* out) {
-    typedef OpsFr Ops;
-    Fr acc[K + 1];
+    typedef Sampler<OpsFr, K, false> S;
+    OpsFr::Acc acc[K + 1];
 #pragma unroll
-    for (int x = 0; x <= K; x++) acc[x] = fr_zero();
+    for (int x = 0; x <= K; x++) acc[x] = OpsFr::acc_zero();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_pairs; p += stride) {
-        Fr f[2][K];
-#pragma unroll
-        for (int j = 0; j < K; j++) {
+        S s;
+        absorb_all<S, K>(s, acc, [&](int j, Fr& f0, Fr& f1) {
+            Fr f[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const Fr a0 = FrFam::load(ptrs.in[j], DPB_FR, 4 * p + 2 * h);
                 const Fr a1 = FrFam::load(ptrs.in[j], DPB_FR, 4 * p + 2 * h + 1);
-                f[h][j] = fr_add(a0, fr_mul_fixed(rk, fr_sub(a1, a0)));  // the challenge is fixed for the launch
-                FrFam::store(ptrs.out[j], 2 * p + h, f[h][j]);
+                f[h] = fr_add(a0, fr_mul_fixed(rk, fr_sub(a1, a0)));  // the challenge is fixed for the launch
+                FrFam::store(ptrs.out[j], 2 * p + h, f[h]);
             }
-        }
-        sample_pair<Ops, K, false>(acc, f[0], f[1]);
+            f0 = f[0];
+            f1 = f[1];
+        });
     }
-    publish<Ops, K>(acc, rs, out);
+    publish<OpsFr, K>(acc, rs, out);
 }
 
 // ---- host: samples -> evaluations at 0..=K -----------------------------------

@@ -8,6 +8,7 @@
 namespace dpb {
 
 struct OpsWBase {
+    static constexpr bool kDeriveM1 = false;
     typedef GlFam F;
     typedef glw::W T;
     typedef glw::A8 Acc;
@@ -22,6 +23,7 @@ struct OpsWBase {
 };
 
 struct OpsWExt {
+    static constexpr bool kDeriveM1 = false;
     typedef GlFam F;
     typedef glw::W2 T;
     struct Acc {
