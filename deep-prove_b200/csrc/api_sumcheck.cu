@@ -80,11 +80,11 @@ struct dpb_sc {
     bool heavy = false;          // a long term program: small rounds are spread over the terms instead
     bool has_prog = false;       // d_rtab / d_groups / d_prog are laid out (every shape that fits)
     uint32_t tail_start = ~0u;   // first round the resident last-rounds kernel may take over
+    uint32_t tail_alone = 0;     // pairs up to which it is one block
     bool tail_active = false;    // that kernel is running for this sumcheck
     uint32_t n_prog_terms = 0;
     bool tail_prog_in_smem = false;
     uint32_t tail_slots_offset = 0;
-    size_t tail_smem = 0;
     RoundTab* d_rtab = nullptr;  // [n][k]
     void* d_groups = nullptr;
     void* d_prog = nullptr;
@@ -121,6 +121,13 @@ struct dpb_sc {
     void* tail_dev = nullptr;
     std::vector<MleDesc> h_desc;
     std::vector<FoldDesc> h_fold;
+    // Tables that enter only through a linear combination with one cofactor (plan_merge): the sumcheck that runs is over
+    // the combination, this object forwards to it and evaluates the tables themselves at the end.
+    dpb_sc* merged = nullptr;
+    std::vector<dpb_mle*> merged_owned;     // the combinations
+    std::vector<int32_t> merged_slot;       // per table: its place in the inner sumcheck, or -1
+    std::vector<dpb_mle> merged_members;    // the tables without a place (borrowed memory), in the order of their ids
+    std::vector<uint8_t> merged_point;      // the challenges so far
 };
 
 namespace dpb {
@@ -494,14 +501,21 @@ static void plan_program(dpb_sc* sc, const dpb_term* terms, dpb_mle* const* mles
         off += 2 * (size_t)sc->k * sizeof(RoundTab);  // descriptors of the current and the next round
         off = (off + 15) & ~(size_t)15;
         sc->tail_slots_offset = (uint32_t)off;
-        // pairs per round the kernel can take: two items per thread in the evaluation phase, and the slots must fit
-        uint64_t max_pairs = 256;
-        while (max_pairs * (sc->d + 1) > 2 * (uint64_t)kTailThreads) max_pairs >>= 1;
-        // the slots of its first round and, half as many, those of the next
-        const size_t per_pair = (size_t)sc->k * 2 * sizeof(E);
-        while (max_pairs >= 1 && off + per_pair * (max_pairs + (max_pairs + 1) / 2) > (size_t)kOnePassMaxSmem) max_pairs >>= 1;
+        // pairs per round a block can take: two items per thread in the evaluation phase, and the slots of its first round
+        // and of the next must fit; a cluster takes kTailBlocks times as many
+        uint64_t nb = 256;
+        while (nb * (sc->d + 1) > 2 * (uint64_t)kTailThreads) nb >>= 1;
+        auto bytes = [&](uint64_t nb_, uint32_t blocks) {
+            return off + (tail_slot_pairs(nb_, blocks, sc->tail_alone, 0) + tail_slot_pairs(nb_, blocks, sc->tail_alone, 1)) * sc->k * 2 * sizeof(E);
+        };
+        sc->tail_alone = (uint32_t)std::min<uint64_t>(nb, sc->gl ? kTailAloneGl : kTailAloneFr);
+        while (sc->tail_alone >= 1 && bytes(sc->tail_alone, 1) > (size_t)kOnePassMaxSmem) sc->tail_alone >>= 1;
+        uint64_t max_pairs = sc->tail_alone;  // one block; with many tables that is all
+        if (sc->tail_alone >= kTailBlocks) {
+            while (nb >= 1 && bytes(nb, kTailBlocks) > (size_t)kOnePassMaxSmem) nb >>= 1;
+            max_pairs = std::max(max_pairs, nb * kTailBlocks);
+        }
         if (max_pairs >= 1) {
-            sc->tail_smem = off + per_pair * (max_pairs + (max_pairs + 1) / 2);
             uint32_t i = 0;
             while (i < sc->n && (1ull << (sc->n - i - 1)) > max_pairs) i++;
             sc->tail_start = i;
@@ -748,11 +762,26 @@ template <class F, int D>
 static int launch_tail(dpb_sc* sc, uint32_t round, const typename F::E& r) {
     dpb_ctx* ctx = sc->ctx;
     DPB_CUDA(cudaFuncSetAttribute(sc_tail_generic<F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOnePassMaxSmem));
-    sc_tail_generic<F, D><<<1, kTailThreads, sc->tail_smem, ctx->tail_stream>>>(
-        sc->d_rtab, sc->k, (const ProgGroup*)sc->d_groups, sc->n_groups, (const ProgTerm<F>*)sc->d_prog,
-        sc->n_prog_terms, r, round, sc->n, (TailBox*)ctx->tail_box_dev, ctx->tail_wait_ns, sc->tail_prog_in_smem ? 1u : 0u,
-        sc->tail_slots_offset);
-    DPB_CUDA(cudaGetLastError());
+    const uint64_t pairs = 1ull << (sc->n - round - 1);
+    const uint32_t blocks = pairs > sc->tail_alone ? kTailBlocks : 1;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = sc->tail_slots_offset + (tail_slot_pairs(pairs / blocks, blocks, sc->tail_alone, 0) +
+                                                    tail_slot_pairs(pairs / blocks, blocks, sc->tail_alone, 1)) *
+                                                       sc->k * 2 * sizeof(typename F::E);
+    cfg.stream = ctx->tail_stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    DPB_CUDA(cudaLaunchKernelEx(&cfg, sc_tail_generic<F, D>, (const RoundTab*)sc->d_rtab, sc->k, (const ProgGroup*)sc->d_groups,
+                                sc->n_groups, (const ProgTerm<F>*)sc->d_prog, sc->n_prog_terms, r, round, sc->n,
+                                (TailBox*)ctx->tail_box_dev, ctx->tail_wait_ns, sc->tail_prog_in_smem ? 1u : 0u,
+                                sc->tail_slots_offset, sc->tail_alone));
     return DPB_OK;
 }
 
@@ -1505,10 +1534,184 @@ static int start_tail(dpb_sc* sc, const void* prev_challenge) {
 
 }  // namespace dpb
 
-extern "C" {
+namespace dpb {
 
-int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k,
-                       const dpb_term* terms, uint32_t n_terms, dpb_sc** out) {
+// From which size merging pays.  The merged tables' values at the end cost one more pass and wait (about 60 us), unless
+// they are eq tables, whose values the host knows; what is saved grows with the tables left out and the rounds.
+// Measured, masked attention scores, before -> merged: BN254, 2^18, 12 heads 2584 -> 1336 us, 4 heads 1294 -> 1052, 2^10,
+// 12 heads 843 -> 694, 4 heads 486 -> 464, 2 heads 418 -> 427; Goldilocks, 2^18, 12 heads 1204 -> 859, 4 heads 692 ->
+// 658, 2^12, 4 heads 379 -> 386.  Claims on one tensor (eq tables): two claims, 2^10 221 -> 171, 2^20 965 -> 682.
+constexpr uint32_t kMergeMinVars = 10;
+static bool merge_pays(uint32_t num_vars, bool gl, size_t members, bool all_eq) {
+    return all_eq || (members - 1) * num_vars >= (gl ? 54u : 30u);
+}
+
+// Terms  c_j * M * t_j  that share their cofactor M, every t_j full-size and in no other term, are one term over the
+// linear combination  sum_j c_j t_j  (the masked attention scores of all heads, the claims merged on one tensor): the
+// same polynomial is summed, so the messages are the same, but rounds bind and multiply one table instead of many.
+// Returns the groups (term indices, at least two each); empty: nothing to merge.  position[t]: where in term t its t_j is.
+static std::vector<std::vector<uint32_t>> plan_merge(uint32_t num_vars, dpb_ctx* ctx, dpb_mle* const* mles, uint32_t k,
+                                                     const dpb_term* terms, uint32_t n_terms, std::vector<int>& position) {
+    std::vector<std::vector<uint32_t>> groups;
+    if (num_vars < kMergeMinVars || num_vars > 40 || n_terms < 2 || k < 2 || k > 65535) return groups;
+    // anything the general path refuses is left to it
+    const bool gl = mles[0] && is_gl(mles[0]->dtype);
+    for (uint32_t j = 0; j < k; j++)
+        if (!mles[j] || mles[j]->ctx != ctx || !valid_dtype(mles[j]->dtype) || is_gl(mles[j]->dtype) != gl) return groups;
+    std::vector<uint32_t> uses(k, 0);
+    for (uint32_t t = 0; t < n_terms; t++) {
+        if (terms[t].n_factors > 6) return groups;
+        for (uint32_t j = 0; j < terms[t].n_factors; j++) {
+            if (terms[t].idx[j] >= k) return groups;
+            uses[terms[t].idx[j]]++;
+        }
+    }
+    position.assign(n_terms, -1);
+    std::map<std::vector<uint16_t>, std::vector<uint32_t>> by_cofactor;
+    for (uint32_t t = 0; t < n_terms; t++) {
+        int at = -1;
+        bool two = false;
+        for (uint32_t j = 0; j < terms[t].n_factors; j++) {
+            const dpb_mle* m = mles[terms[t].idx[j]];
+            if (uses[terms[t].idx[j]] != 1 || m->len != (1ull << num_vars)) continue;
+            two = at >= 0;
+            at = (int)j;
+        }
+        if (at < 0 || two) continue;  // none, or a product of two private tables: no shared cofactor
+        std::vector<uint16_t> co;
+        for (uint32_t j = 0; j < terms[t].n_factors; j++)
+            if ((int)j != at) co.push_back(terms[t].idx[j]);
+        std::sort(co.begin(), co.end());
+        position[t] = at;
+        by_cofactor[co].push_back(t);
+    }
+    for (auto& kv : by_cofactor) {
+        bool all_eq = true;
+        for (uint32_t t : kv.second)
+            all_eq &= mles[terms[t].idx[position[t]]]->eq_point.size() == (size_t)num_vars * (gl ? 16 : 32);
+        if (kv.second.size() < 2 || !merge_pays(num_vars, gl, kv.second.size(), all_eq)) {
+            for (uint32_t t : kv.second) position[t] = -1;
+            continue;
+        }
+        groups.push_back(kv.second);
+    }
+    return groups;
+}
+
+static int begin_general(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k, const dpb_term* terms,
+                         uint32_t n_terms, dpb_sc** out);
+
+static int begin_merged(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k, const dpb_term* terms,
+                        uint32_t n_terms, const std::vector<std::vector<uint32_t>>& groups, const std::vector<int>& position,
+                        dpb_sc** out) {
+    const bool gl = is_gl(mles[0]->dtype);
+    const size_t es = gl ? 16 : 32;
+    dpb_sc* sc = new (std::nothrow) dpb_sc();
+    if (!sc) return fail(DPB_ENOMEM, "host allocation failed");
+    sc->ctx = ctx;
+    sc->gl = gl;
+    sc->n = num_vars;
+    sc->k = k;
+    std::vector<bool> member(k, false);
+    for (const auto& g : groups)
+        for (uint32_t t : g) member[terms[t].idx[position[t]]] = true;
+    std::vector<dpb_mle*> tabs;
+    sc->merged_slot.assign(k, -1);
+    for (uint32_t j = 0; j < k; j++) {
+        if (member[j]) {
+            sc->merged_members.push_back(*mles[j]);
+            continue;
+        }
+        sc->merged_slot[j] = (int32_t)tabs.size();
+        tabs.push_back(mles[j]);
+    }
+    std::vector<dpb_term> inner;
+    auto remapped = [&](const dpb_term& t, int skip) {
+        dpb_term r;
+        memset(&r, 0, sizeof r);
+        memcpy(r.coeff, t.coeff, sizeof r.coeff);
+        for (uint32_t j = 0; j < t.n_factors; j++)
+            if ((int)j != skip) r.idx[r.n_factors++] = (uint16_t)sc->merged_slot[t.idx[j]];
+        return r;
+    };
+    for (uint32_t t = 0; t < n_terms; t++)
+        if (position[t] < 0) inner.push_back(remapped(terms[t], -1));
+    for (const auto& g : groups) {
+        std::vector<dpb_mle*> list;
+        std::vector<uint8_t> coef(g.size() * es);
+        for (size_t q = 0; q < g.size(); q++) {
+            list.push_back(mles[terms[g[q]].idx[position[g[q]]]]);
+            memcpy(coef.data() + q * es, terms[g[q]].coeff, es);
+        }
+        dpb_mle* l = nullptr;
+        const int rc = dpb_linear_combination(ctx, list.data(), coef.data(), (uint32_t)list.size(), &l);
+        if (rc != DPB_OK) {
+            dpb_sumcheck_free(sc);
+            return rc;
+        }
+        sc->merged_owned.push_back(l);
+        dpb_term r = remapped(terms[g[0]], position[g[0]]);
+        memset(r.coeff, 0, sizeof r.coeff);
+        if (gl) {
+            const Gl2 one = GlFam::one();
+            memcpy(r.coeff, &one, sizeof one);
+        } else {
+            const Fr one = FrFam::one();
+            memcpy(r.coeff, &one, sizeof one);
+        }
+        r.idx[r.n_factors++] = (uint16_t)tabs.size();
+        tabs.push_back(l);
+        inner.push_back(r);
+    }
+    const int rc = begin_general(ctx, num_vars, tabs.data(), (uint32_t)tabs.size(), inner.data(), (uint32_t)inner.size(), &sc->merged);
+    if (rc != DPB_OK) {
+        dpb_sumcheck_free(sc);
+        return rc;
+    }
+    sc->d = sc->merged->d;
+    *out = sc;
+    return DPB_OK;
+}
+
+// The last challenge of a merged sumcheck: the inner one's evaluations, and the merged tables' at the point (eq tables
+// from their coordinates, the others in one pass over all of them).
+template <class F>
+static int merged_finish(dpb_sc* sc, const void* last_challenge, void* out) {
+    typedef typename F::E E;
+    std::vector<E> inner(sc->merged->k);
+    DPB_TRY(dpb_sumcheck_finish(sc->merged, last_challenge, inner.data()));
+    sc->merged_point.insert(sc->merged_point.end(), (const uint8_t*)last_challenge, (const uint8_t*)last_challenge + sizeof(E));
+    const E* point = (const E*)sc->merged_point.data();
+    std::vector<E> values(sc->merged_members.size());
+    std::vector<dpb_mle*> list;
+    std::vector<size_t> place;
+    for (size_t q = 0; q < sc->merged_members.size(); q++) {
+        dpb_mle& m = sc->merged_members[q];
+        if (m.eq_point.size() == (size_t)sc->n * sizeof(E)) {
+            E v = F::one();
+            for (uint32_t i = 0; i < sc->n; i++) {
+                E c;
+                memcpy(&c, m.eq_point.data() + (size_t)i * sizeof(E), sizeof(E));
+                v = F::mul(v, eq_scalar<F>(c, point[i]));
+            }
+            values[q] = v;
+        } else {
+            list.push_back(&m);
+            place.push_back(q);
+        }
+    }
+    if (!list.empty()) {
+        std::vector<E> got(list.size());
+        DPB_TRY(dpb_mle_evaluate_many(sc->ctx, list.data(), (uint32_t)list.size(), point, sc->n, got.data()));
+        for (size_t q = 0; q < list.size(); q++) values[place[q]] = got[q];
+    }
+    size_t next = 0;
+    for (uint32_t j = 0; j < sc->k; j++) ((E*)out)[j] = sc->merged_slot[j] >= 0 ? inner[sc->merged_slot[j]] : values[next++];
+    return DPB_OK;
+}
+
+static int begin_general(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k,
+                         const dpb_term* terms, uint32_t n_terms, dpb_sc** out) {
     if (!ctx || !mles || !terms || !out) return fail(DPB_EINVAL, "null argument");
     if (num_vars < 1 || num_vars > 40) return fail(DPB_EINVAL, "num_vars %u out of range", num_vars);
     if (k < 1 || k > 65535) return fail(DPB_EINVAL, "table count %u out of range", k);
@@ -1780,6 +1983,20 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
     return DPB_OK;
 }
 
+}  // namespace dpb
+
+extern "C" {
+
+int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k,
+                       const dpb_term* terms, uint32_t n_terms, dpb_sc** out) {
+    if (ctx && mles && terms && out) {
+        std::vector<int> position;
+        const auto groups = plan_merge(num_vars, ctx, mles, k, terms, n_terms, position);
+        if (!groups.empty()) return begin_merged(ctx, num_vars, mles, k, terms, n_terms, groups, position, out);
+    }
+    return begin_general(ctx, num_vars, mles, k, terms, n_terms, out);
+}
+
 uint32_t dpb_sumcheck_degree(const dpb_sc* sc) { return sc ? sc->d : 0; }
 
 int dpb_sumcheck_begin_sharded(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k,
@@ -1799,7 +2016,7 @@ int dpb_sumcheck_begin_sharded(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* 
     if ((size_t)k * ctx->nranks * 32 > ctx->result_bytes || (size_t)k * ctx->nranks * 32 > ctx->gather_bytes)
         return fail(DPB_EINVAL, "too many tables (%u) for the tail exchange", k);
     dpb_sc* sc = nullptr;
-    DPB_TRY(dpb_sumcheck_begin(ctx, n_loc, mles, k, terms, n_terms, &sc));
+    DPB_TRY(begin_general(ctx, n_loc, mles, k, terms, n_terms, &sc));
     sc->log2_ranks = c;
     sc->spliteq = false;  // the shards of an eq table are not eq tables
     sc->terms_copy.assign(terms, terms + n_terms);
@@ -1879,7 +2096,7 @@ static void hint_logup_impl(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_in
     lt.d_consts = (char*)d + o_tc;
     lt.d_inst = (char*)d + o_ti;
     uint64_t best = 0;
-    for (uint32_t alone = 32; alone >= 4; alone /= 2) {
+    for (uint32_t alone = sc->gl ? kTailAloneGl : kTailAloneFr; alone >= 4; alone /= 2) {
         LogupTailPlan p = lt;
         p.alone = alone;
         for (uint64_t pairs = 256 * kLogupTailBlocks; pairs > best; pairs /= 2) {
@@ -1899,7 +2116,7 @@ static void hint_logup_impl(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_in
 }
 
 void sumcheck_hint_logup(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_inst, const void* lambda, uint32_t eq_table) {
-    if (!sc || !inst || !lambda || n_inst == 0 || n_inst > kLogupMaxInst || sc->logup_ok || getenv("DPB_NO_LOGUP_KERNEL")) return;
+    if (!sc || sc->merged || !inst || !lambda || n_inst == 0 || n_inst > kLogupMaxInst || sc->logup_ok || getenv("DPB_NO_LOGUP_KERNEL")) return;
     // usable only by a degree-3 sumcheck in split-eq form whose one eq table is the hint's and whose other tables are
     // exactly the instances', in order
     if (!sc->spliteq || sc->d != 3 || sc->eq_leads.size() != 1 || sc->eq_leads[0].table != eq_table ||
@@ -1929,7 +2146,7 @@ int dpb_sumcheck_begin_partial(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* 
     if (ctx->nranks <= 1) return dpb_sumcheck_begin(ctx, num_vars, mles, k, terms, n_terms, out);
     if (!ctx->nccl_comm) return fail(DPB_ESTATE, "the context has no communicator (dpb_comm_init)");
     dpb_sc* sc = nullptr;
-    DPB_TRY(dpb_sumcheck_begin(ctx, num_vars, mles, k, terms, n_terms, &sc));
+    DPB_TRY(begin_general(ctx, num_vars, mles, k, terms, n_terms, &sc));
     sc->partial = true;
     *out = sc;
     return DPB_OK;
@@ -1937,6 +2154,13 @@ int dpb_sumcheck_begin_partial(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* 
 
 int dpb_sumcheck_round(dpb_sc* sc, const void* prev_challenge, void* out_evals, uint32_t* n_evals) {
     if (!sc || !out_evals) return fail(DPB_EINVAL, "null argument");
+    if (sc->merged) {
+        DPB_TRY(dpb_sumcheck_round(sc->merged, prev_challenge, out_evals, n_evals));
+        if (prev_challenge)
+            sc->merged_point.insert(sc->merged_point.end(), (const uint8_t*)prev_challenge,
+                                    (const uint8_t*)prev_challenge + (sc->gl ? 16 : 32));
+        return DPB_OK;
+    }
     const uint32_t total = sc->n + sc->log2_ranks;
     if (sc->finished || sc->global_round >= total) return fail(DPB_ESTATE, "all %u rounds already ran", total);
     if (sc->global_round == 0 && prev_challenge) return fail(DPB_ESTATE, "the first round takes no challenge");
@@ -1960,6 +2184,8 @@ int dpb_sumcheck_round(dpb_sc* sc, const void* prev_challenge, void* out_evals, 
 
 int dpb_sumcheck_finish(dpb_sc* sc, const void* last_challenge, void* out_final_evals) {
     if (!sc || !last_challenge || !out_final_evals) return fail(DPB_EINVAL, "null argument");
+    if (sc->merged)
+        return sc->gl ? merged_finish<GlFam>(sc, last_challenge, out_final_evals) : merged_finish<FrFam>(sc, last_challenge, out_final_evals);
     if (sc->finished) return fail(DPB_ESTATE, "already finished");
     const uint32_t total = sc->n + sc->log2_ranks;
     if (sc->global_round != total) return fail(DPB_ESTATE, "only %u of %u rounds ran", sc->global_round, total);
@@ -1978,6 +2204,8 @@ int dpb_sumcheck_finish(dpb_sc* sc, const void* last_challenge, void* out_final_
 
 void dpb_sumcheck_free(dpb_sc* sc) {
     if (!sc) return;
+    if (sc->merged) dpb_sumcheck_free(sc->merged);
+    for (auto* m : sc->merged_owned) dpb_mle_free(m);
     if (sc->tail_active) tail_abort(sc);
     if (sc->tail) dpb_sumcheck_free(sc->tail);
     for (auto* m : sc->tail_mles) dpb_mle_free(m);

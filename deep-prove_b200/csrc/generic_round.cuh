@@ -18,7 +18,10 @@
 //    multiplies the group's sum once per point instead of once per term.
 // Results are exact field sums, so they equal the two-pass kernels' bit for bit.
 #pragma once
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <vector>
 
 #include "sumcheck_kernels.cuh"
 
@@ -628,6 +631,17 @@ __device__ __forceinline__ int tail_wait(TailBox* box, uint32_t want, unsigned l
 }
 
 constexpr int kTailThreads = 512;
+constexpr uint32_t kTailBlocks = 8;   // blocks of the cluster that runs larger rounds (the portable size)
+// Pairs from which one block goes on alone (at most): the cluster divides a round's products by eight and adds two
+// cluster barriers, which pays for BN254 rounds of more than 32 pairs (n = 8: 105 -> 100 us a proof) and makes no
+// difference to Goldilocks rounds of up to 256 (n = 10: 102.4 us handed over at 32 pairs, 103.6 at 256).
+constexpr uint32_t kTailAloneFr = 32, kTailAloneGl = 256;
+// Pairs the slots of even and of odd rounds are laid out for, nb pairs of a block in the first round: a cluster's first
+// block needs room for all that is left when it goes on alone, in whichever set that falls.
+__host__ __device__ __forceinline__ size_t tail_slot_pairs(size_t nb, uint32_t blocks, uint32_t alone, int set) {
+    const size_t own = set ? (nb + 1) / 2 : nb, gathered = blocks > 1 ? (size_t)alone : 0;
+    return own > gathered ? own : gathered;
+}
 constexpr int kTailProgBytes = 8 * 1024;  // the term program is staged in shared memory when it fits
 
 // Shared-memory slots addressed by pair instead of by thread: slot s of pair p, n pairs in the round.
@@ -708,7 +722,10 @@ __device__ __forceinline__ typename F::E segment_sum(typename F::E v, uint32_t n
     return v;
 }
 
-// One block; round `round` has n_pairs = 2^(n_rounds - round - 1) <= max_pairs pairs.  Per round:
+// One block, or a cluster of kTailBlocks blocks while a round has more than `alone` pairs: every block then holds a
+// contiguous part of the pairs, partial sums and the challenge travel through distributed shared memory, and the first
+// block goes on alone.  (Blocks of a cluster are resident together, so their barriers end; the one wait for the host
+// is bounded, and its outcome is handed to all.)  Per round of 2^(n_rounds - round - 1) pairs:
 //   A. items (pair, table): bind the previous challenge and fill the pair's slots.  The values to bind are the slots of
 //      the round before (two sets of slots, used in turn); only the first round reads tables from memory.  The bound
 //      tables are stored all the same, so that the kernel can be started again at any round;
@@ -718,19 +735,26 @@ __device__ __forceinline__ typename F::E segment_sum(typename F::E v, uint32_t n
 // Latency is all that counts here: one thread's chain of products, barriers, and trips to memory and to the host.
 // Dynamic shared memory: [program copy | round descriptors | slots of even rounds | slots of odd rounds].
 // Product of three tables over BN254, n = 8: 14.1 us a round with the tables read back from memory, a tree of
-// barriers for the sums and a challenge read chunk by chunk, 11.2 us since (Goldilocks 9.5, 7.1).
+// barriers for the sums and a challenge read chunk by chunk, 11.2 us since (Goldilocks 9.5, 7.1); with the cluster
+// three more rounds are resident: n = 12 201 -> 153 us a proof (Goldilocks 148 -> 129), n = 20 631 -> 555 us.
 template <class F, int D>
 __global__ void __launch_bounds__(kTailThreads)
     sc_tail_generic(const RoundTab* __restrict__ tabs_all, uint32_t k, const ProgGroup* __restrict__ groups_g,
                     uint32_t n_groups, const ProgTerm<F>* __restrict__ terms_g, uint32_t n_prog_terms,
                     typename F::E r, uint32_t first_round, uint32_t n_rounds, TailBox* box,
-                    unsigned long long wait_ns, uint32_t prog_in_smem, uint32_t slots_offset) {
+                    unsigned long long wait_ns, uint32_t prog_in_smem, uint32_t slots_offset, uint32_t alone) {
     typedef typename F::E E;
+    namespace cg = cooperative_groups;
+    constexpr int W8 = sizeof(E) / 8;
+    cg::cluster_group cluster = cg::this_cluster();
+    uint32_t blocks = cluster.num_blocks();
+    const uint32_t rank = cluster.block_rank();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) E sh_r;
     __shared__ int sh_stop;
     __shared__ typename F::FoldKey sh_key;  // the current challenge in the form the folds multiply by
     __shared__ E sh_sum[2 * kTailThreads / 32];
+    __shared__ __align__(16) E sh_part[D + 1][kTailBlocks];
     const ProgGroup* groups = groups_g;
     const ProgTerm<F>* terms = terms_g;
     unsigned char* cursor = smem_raw;
@@ -748,95 +772,142 @@ __global__ void __launch_bounds__(kTailThreads)
                              (RoundTab*)(smem_raw + slots_offset - (size_t)k * sizeof(RoundTab))};
     for (uint32_t j = threadIdx.x; j < k; j += blockDim.x) tabs_buf[0][j] = tabs_all[(size_t)first_round * k + j];
     const RoundTab* tabs = tabs_buf[0];
-    const uint32_t first_pairs = 1u << (n_rounds - first_round - 1);
+    uint32_t nb = (1u << (n_rounds - first_round - 1)) / blocks;  // pairs of this block
+    const size_t set_words = (size_t)2 * k * PairSlots<F>::W * tail_slot_pairs(nb, blocks, alone, 0);
     PairSlots<F> sl, old;
     sl.base = old.base = (uint4*)(smem_raw + slots_offset);
-    sl.n = old.n = 0;
+    sl.n = old.n = nb;
+    if (blocks > 1) cluster.sync();  // every block has started: its shared memory may be written
     if (threadIdx.x == 0) {
-        sh_stop = tail_hello(box, kTailHelloNs) ? 0 : 1;
+        if (rank == 0) {
+            const int stop = tail_hello(box, kTailHelloNs) ? 0 : 1;
+            for (uint32_t b = 0; b < blocks; b++) *cluster.map_shared_rank(&sh_stop, b) = stop;
+        }
         sh_r = r;
     }
     F::fold_key_block(r, &sh_key);
-    __syncthreads();
+    if (blocks > 1) cluster.sync();
+    else __syncthreads();
     if (sh_stop) return;
     for (uint32_t round = first_round; round < n_rounds; round++) {
-        const uint32_t n_pairs = 1u << (n_rounds - round - 1);
-        old = sl;
-        sl.n = n_pairs;
-        sl.base = (uint4*)(smem_raw + slots_offset) + (((round - first_round) & 1) ? (size_t)2 * k * PairSlots<F>::W * first_pairs : 0);
+        const bool gather = round > first_round && blocks > 1 && nb * blocks <= 2 * alone;
+        if (round > first_round) {
+            old = sl;
+            nb = gather ? nb * blocks / 2 : nb / 2;
+            sl.n = nb;
+            sl.base = (uint4*)(smem_raw + slots_offset) + (((round - first_round) & 1) ? set_words : 0);
+        }
         tabs = tabs_buf[(round - first_round) & 1];
         if (round + 1 < n_rounds) {
             RoundTab* nxt = tabs_buf[(round + 1 - first_round) & 1];
             for (uint32_t j = threadIdx.x; j < k; j += blockDim.x) nxt[j] = tabs_all[(size_t)(round + 1) * k + j];
         }
         // A
-        for (uint32_t w = threadIdx.x; w < n_pairs * k; w += blockDim.x) {
-            const uint32_t j = w / n_pairs, p = w % n_pairs;
-            const RoundTab t = tabs[j];
-            E f0, f1;
-            if (t.out) {
-                E a0, b0, da, db;
-                if (round > first_round) {
-                    a0 = old.get(2 * j, 2 * p);
-                    da = old.get(2 * j + 1, 2 * p);
-                    b0 = old.get(2 * j, 2 * p + 1);
-                    db = old.get(2 * j + 1, 2 * p + 1);
+        const uint64_t p0 = gather ? 0 : (uint64_t)rank * nb;  // first pair of this block
+        if (!gather || rank == 0) {
+            for (uint32_t w = threadIdx.x; w < nb * k; w += blockDim.x) {
+                const uint32_t j = w / nb, p = w % nb;
+                const RoundTab t = tabs[j];
+                E f0, f1;
+                if (t.out) {
+                    E a0, b0, da, db;
+                    if (round > first_round) {
+                        PairSlots<F> src = old;
+                        uint32_t q = 2 * p;
+                        if (gather) {  // a block held 2 * alone / kTailBlocks pairs, an even number
+                            src.base = cluster.map_shared_rank(old.base, q / old.n);
+                            q %= old.n;
+                        }
+                        a0 = src.get(2 * j, q);
+                        da = src.get(2 * j + 1, q);
+                        b0 = src.get(2 * j, q + 1);
+                        db = src.get(2 * j + 1, q + 1);
+                    } else {
+                        E a1, b1;
+                        F::load_pair(t.in, t.dtype_in, 2 * (p0 + p), a0, a1);
+                        F::load_pair(t.in, t.dtype_in, 2 * (p0 + p) + 1, b0, b1);
+                        da = F::sub(a1, a0);
+                        db = F::sub(b1, b0);
+                    }
+                    f0 = F::add(a0, F::mul_key(sh_key, da));
+                    f1 = F::add(b0, F::mul_key(sh_key, db));
+                    F::store(t.out, 2 * (p0 + p), f0);
+                    F::store(t.out, 2 * (p0 + p) + 1, f1);
+                } else if (t.shift < 0) {
+                    F::load_pair(t.in, t.dtype_in, p0 + p, f0, f1);
                 } else {
-                    E a1, b1;
-                    F::load_pair(t.in, t.dtype_in, 2 * (uint64_t)p, a0, a1);
-                    F::load_pair(t.in, t.dtype_in, 2 * (uint64_t)p + 1, b0, b1);
-                    da = F::sub(a1, a0);
-                    db = F::sub(b1, b0);
+                    f0 = F::load(t.in, t.dtype_in, (p0 + p) >> t.shift);
+                    f1 = f0;
                 }
-                f0 = F::add(a0, F::mul_key(sh_key, da));
-                f1 = F::add(b0, F::mul_key(sh_key, db));
-                F::store(t.out, 2 * (uint64_t)p, f0);
-                F::store(t.out, 2 * (uint64_t)p + 1, f1);
-            } else if (t.shift < 0) {
-                F::load_pair(t.in, t.dtype_in, p, f0, f1);
-            } else {
-                f0 = F::load(t.in, t.dtype_in, p >> t.shift);
-                f1 = f0;
+                sl.put(2 * j, p, f0);
+                sl.put(2 * j + 1, p, F::sub(f1, f0));
             }
-            sl.put(2 * j, p, f0);
-            sl.put(2 * j + 1, p, F::sub(f1, f0));
+        }
+        if (gather) {
+            cluster.sync();  // the other blocks' slots have been read
+            if (rank != 0) return;
+            blocks = 1;
         }
         __syncthreads();
         // B: the points are 0, 1, .., D in round 0 and 0, 2, .., D later (index 1 is left out); at most two items per
-        // thread (n_pairs * n_points <= 2 * blockDim)
+        // thread (nb * n_points <= 2 * blockDim)
         const uint32_t n_points = round > 0 ? D : D + 1;
-        const uint32_t n_items = n_pairs * n_points;
-        uint32_t parts = n_pairs > 32 ? n_pairs / 32 : 1;  // partial sums per point
+        const uint32_t n_items = nb * n_points;
+        const uint32_t parts = nb > 32 ? nb / 32 : 1;  // partial sums per point
         for (uint32_t w0 = 0; w0 < n_items; w0 += blockDim.x) {
             const uint32_t w = w0 + threadIdx.x;
             if ((w & ~31u) >= n_items) continue;  // whole warps: the sums below shuffle
             E v = F::zero();
-            const uint32_t xi = w / n_pairs, p = w % n_pairs;
+            const uint32_t xi = w / nb, p = w % nb;
             if (w < n_items) {
                 const uint32_t x = (round > 0 && xi >= 1) ? xi + 1 : xi;
                 v = eval_program_at<F>(sl, p, x, groups, n_groups, terms);
             }
-            v = segment_sum<F>(v, n_pairs);
+            v = segment_sum<F>(v, nb);
             if (w < n_items && (p & 31) == 0) sh_sum[xi * parts + p / 32] = v;
         }
         __syncthreads();
         // C
         if (threadIdx.x < 32) {
-            constexpr int W8 = sizeof(E) / 8;
             const uint32_t lane = threadIdx.x;
             // n_points segments of `parts` partial sums (at most 32 sums in all: n_items <= 2 * kTailThreads)
             E v = lane < n_points * parts ? sh_sum[lane] : F::zero();
             v = segment_sum<F>(v, parts);
             if (lane < n_points * parts && lane % parts == 0) {
-                const uint32_t xi = lane / parts, x = (round > 0 && xi >= 1) ? xi + 1 : xi;
-                chunks_store<E>(&box->evals[x * W8], v, round + 1);
+                const uint32_t xi = lane / parts;
+                if (blocks > 1) {
+                    cluster.map_shared_rank(&sh_part[0][0], 0)[xi * kTailBlocks + rank] = v;
+                } else {
+                    const uint32_t x = (round > 0 && xi >= 1) ? xi + 1 : xi;
+                    chunks_store<E>(&box->evals[x * W8], v, round + 1);
+                }
+            }
+            __syncwarp();
+        }
+        if (blocks > 1) cluster.sync();
+        if (rank == 0 && threadIdx.x < 32) {
+            const uint32_t lane = threadIdx.x;
+            if (blocks > 1) {
+                for (uint32_t x0 = 0; x0 < n_points; x0 += 32 / kTailBlocks) {  // four points at a time
+                    const uint32_t xi = x0 + lane / kTailBlocks;
+                    E v = xi < n_points ? sh_part[xi][lane % kTailBlocks] : F::zero();
+                    v = segment_sum<F>(v, kTailBlocks);
+                    if (xi < n_points && lane % kTailBlocks == 0) {
+                        const uint32_t x = (round > 0 && xi >= 1) ? xi + 1 : xi;
+                        chunks_store<E>(&box->evals[x * W8], v, round + 1);
+                    }
+                }
             }
             uint64_t word = 0;
             const int stop = tail_wait<E>(box, round + 1, wait_ns, word);
-            if (lane < W8) ((uint64_t*)&sh_r)[lane] = word;
-            if (lane == 0) sh_stop = stop;
+            for (uint32_t q = 0; q < blocks; q++) {
+                if (lane < W8) ((uint64_t*)cluster.map_shared_rank(&sh_r, q))[lane] = word;
+                if (lane == 0) *cluster.map_shared_rank(&sh_stop, q) = stop;
+            }
+            __syncwarp();
         }
-        __syncthreads();
+        if (blocks > 1) cluster.sync();
+        else __syncthreads();
         if (sh_stop) return;
         r = sh_r;
         F::fold_key_block(r, &sh_key);

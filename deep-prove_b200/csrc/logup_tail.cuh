@@ -13,7 +13,7 @@
 //    its alpha once per round;
 //  * a cluster of eight blocks runs the rounds that are too large for one: every block holds a contiguous eighth of the
 //    pairs, partial sums and the challenge travel through distributed shared memory, and one block goes on alone once
-//    32 pairs (fewer with many tables) are left.  Blocks of a cluster are resident together, so their barriers end; the one wait for the host
+//    32 pairs (BN254; 256 Goldilocks, fewer with many tables) are left.  Blocks of a cluster are resident together, so their barriers end; the one wait for the host
 //    is bounded and its outcome is handed to all.
 // Measured, BN254, three instances of 2^21 rows: 144 rounds of up to 256 pairs took 3460 us in sc_tail_generic and 32
 // rounds of up to 2048 pairs 1100 us as fold + evaluation launches and the gaps between them; 176 rounds take 2730 us
@@ -215,17 +215,18 @@ __global__ void __launch_bounds__(kTailThreads)
                 }
             }
             if (gather) {
-                // the weights come along; then the other blocks are done
+                // the weights come along (through the sums' space); then the other blocks are done
+                static_assert(kTailAloneGl <= 3 * kLogupTailMaxInst, "the weights pass through sh_sum");
                 if (rank == 0) {
                     const uint32_t stride = first_pairs * blocks / nb;  // in the first round's weights
                     for (uint32_t p = threadIdx.x; p < nb; p += blockDim.x) {
                         const uint32_t at = p * stride;
-                        sh_sum[0][p] = cluster.map_shared_rank(weights, at / first_pairs)[at % first_pairs];
+                        (&sh_sum[0][0])[p] = cluster.map_shared_rank(weights, at / first_pairs)[at % first_pairs];
                     }
                 }
                 cluster.sync();
                 if (rank != 0) return;
-                for (uint32_t p = threadIdx.x; p < nb; p += blockDim.x) weights[p] = sh_sum[0][p];
+                for (uint32_t p = threadIdx.x; p < nb; p += blockDim.x) weights[p] = (&sh_sum[0][0])[p];
                 blocks = 1;
             }
             __syncthreads();
