@@ -1,6 +1,8 @@
 // C ABI: logup-GKR fraction tree of one instance, every level resident on the
 // device (the batched prover walks the levels top-down and needs all of them,
 // zkml/src/lookup/logup_gkr/prover.rs:144-147).
+#include <algorithm>
+
 #include "common.cuh"
 #include "logup_kernels.cuh"
 
@@ -16,60 +18,131 @@ struct dpb_logup {
 
 namespace dpb {
 
-constexpr uint64_t kSmallLevel = 1024;  // levels of at most this many fractions are finished by one block
+static int check_spec(dpb_ctx* ctx, const LogupSpec& p) {
+    if (!p.columns || !p.constant || !p.sep) return fail(DPB_EINVAL, "null argument");
+    if (p.kind != DPB_LOGUP_LOOKUP && p.kind != DPB_LOGUP_TABLE) return fail(DPB_EINVAL, "unknown kind %d", p.kind);
+    if (p.n_cols < 1 || p.n_cols > (uint32_t)kMaxLogupCols)
+        return fail(DPB_EINVAL, "No column evals were provided or too many (%u, max %d)", p.n_cols, kMaxLogupCols);
+    if ((p.kind == DPB_LOGUP_TABLE) != (p.mult != nullptr))
+        return fail(DPB_EINVAL, "multiplicities are required for tables and only for tables");
+    for (uint32_t j = 0; j < p.n_cols; j++)
+        if (!p.columns[j] || p.columns[j]->ctx != ctx) return fail(DPB_EINVAL, "column %u is null or foreign", j);
+    const uint64_t len = p.columns[0]->len;
+    const bool gl = is_gl(p.columns[0]->dtype);
+    for (uint32_t j = 1; j < p.n_cols; j++) {
+        if (p.columns[j]->len != len) return fail(DPB_EINVAL, "All sets of evaluations should be the same length");
+        if (is_gl(p.columns[j]->dtype) != gl) return fail(DPB_EINVAL, "columns mix fields");
+    }
+    if (p.mult && (p.mult->len != len || is_gl(p.mult->dtype) != gl))
+        return fail(DPB_EINVAL, "Multiplicities length was not equal to column evaluations length, multiplicities: %llu, columns: %llu",
+                    (unsigned long long)p.mult->len, (unsigned long long)len);
+    if (len < 4) return fail(DPB_EINVAL, "columns need at least 4 entries, got %llu", (unsigned long long)len);
+    return DPB_OK;
+}
 
+static void int_rows(LogupTree<FrFam>& t, uint32_t j) {
+    for (int half = 0; half < 2; half++) fr_fixed_row(t.sep_pow[j], 8 + half, t.rows[j][half]);
+}
+static void int_rows(LogupTree<GlFam>&, uint32_t) {}
+
+// The trees' levels, and their outputs (4 elements each) to the host when asked for.
 template <class F>
-static int build_tree(dpb_logup* lu, int kind, dpb_mle* const* columns, uint32_t n_cols,
-                      const dpb_mle* mult, const void* constant_chal, const void* sep_chal) {
+static int build_trees(dpb_ctx* ctx, const LogupSpec* specs, uint32_t n, dpb_logup** out, void* host_outputs) {
     typedef typename F::E E;
-    dpb_ctx* ctx = lu->ctx;
-    const uint32_t m = lu->m;
-    const uint32_t levels = m - 1;
-    // level l has 2 * 2^(m-l) entries; total < 2 * 2^m
-    size_t total = 0;
-    for (uint32_t l = 1; l <= levels; l++) total += 2ull << (m - l);
-    DPB_TRY(device_alloc(ctx, total * sizeof(E), &lu->slab));
-    {
-        E* p = (E*)lu->slab;
-        for (uint32_t l = 1; l <= levels; l++) {
-            lu->num.push_back(p);
-            p += 1ull << (m - l);
-            lu->den.push_back(p);
-            p += 1ull << (m - l);
+    std::vector<LogupTree<F>> trees(n);
+    uint32_t max_m = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        const LogupSpec& p = specs[i];
+        dpb_logup* lu = out[i];
+        LogupTree<F>& t = trees[i];
+        memset((void*)&t, 0, sizeof t);
+        const uint32_t m = lu->m;
+        max_m = std::max(max_m, m);
+        DPB_TRY(device_alloc(ctx, logup_level_offset(m, m) * sizeof(E), &lu->slab));
+        for (uint32_t l = 1; l < m; l++) {
+            lu->num.push_back((E*)lu->slab + logup_level_offset(m, l));
+            lu->den.push_back((E*)lu->slab + logup_level_offset(m, l) + (1ull << (m - l)));
         }
+        t.slab = (E*)lu->slab;
+        t.m = m;
+        t.n_cols = p.n_cols;
+        t.is_table = p.kind == DPB_LOGUP_TABLE;
+        if (p.mult) {
+            t.mult = p.mult->ptr;
+            t.mult_dtype = p.mult->dtype;
+        }
+        memcpy(&t.constant, p.constant, sizeof(E));
+        E sep, pw = F::one();
+        memcpy(&sep, p.sep, sizeof(E));
+        t.int_cols = 1;
+        E sum = F::zero();
+        for (uint32_t j = 0; j < p.n_cols; j++) {
+            t.col[j] = p.columns[j]->ptr;
+            t.dtype[j] = p.columns[j]->dtype;
+            if (!is_int_dtype(t.dtype[j])) t.int_cols = 0;
+            t.sep_pow[j] = pw;
+            sum = F::add(sum, pw);
+            pw = F::mul(pw, sep);
+        }
+        t.int_constant = F::sub(t.constant, F::mul(F::from_u64(0x80000000ull), sum));
+        for (uint32_t j = 0; t.int_cols && j < p.n_cols; j++) int_rows(t, j);
     }
-    LogupCols<F> c;
-    memset(&c, 0, sizeof c);
-    c.n_cols = n_cols;
-    memcpy(&c.constant, constant_chal, sizeof(E));
-    E sep;
-    memcpy(&sep, sep_chal, sizeof(E));
-    E pw = F::one();
-    for (uint32_t j = 0; j < n_cols; j++) {
-        c.col[j] = columns[j]->ptr;
-        c.dtype[j] = columns[j]->dtype;
-        c.sep_pow[j] = pw;
-        pw = F::mul(pw, sep);
+    char* d = nullptr;  // [trees | outputs]
+    const size_t o_out = (n * sizeof(LogupTree<F>) + 31) & ~(size_t)31;
+    DPB_TRY(device_alloc(ctx, o_out + (size_t)n * 4 * sizeof(E), (void**)&d));
+    const LogupTree<F>* dt = (const LogupTree<F>*)d;
+    int rc = upload_small(ctx, d, trees.data(), n * sizeof(LogupTree<F>));
+    if (rc == DPB_OK) {
+        auto blocks = [&](uint64_t items) {  // per tree; all trees together fill the GPU
+            const uint64_t want = (items + kThreads - 1) / kThreads, cap = ((uint64_t)ctx->sm_count * 8 + n - 1) / n;
+            return (uint32_t)std::max<uint64_t>(1, std::min(want, cap));
+        };
+        for (uint32_t first = 0; first < n; first += 65535) {  // the grid's second dimension
+            const uint32_t cnt = std::min<uint32_t>(65535, n - first);
+            logup_leaf_levels<F><<<dim3(blocks(1ull << (max_m - 2)), cnt), kThreads, 0, ctx->stream>>>(dt + first);
+            for (uint32_t l = 2; l + 2 <= max_m && (1ull << (max_m - l)) > kLogupSmall; l += 2)
+                logup_two_levels<F><<<dim3(blocks(1ull << (max_m - l - 2)), cnt), kThreads, 0, ctx->stream>>>(dt + first, l);
+            logup_small_levels<F><<<cnt, kThreads, 0, ctx->stream>>>(dt + first, (E*)(d + o_out) + 4 * (size_t)first);
+        }
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess && host_outputs) {
+            TracePhase t_out("logup.outputs");
+            e = cudaMemcpyAsync(host_outputs, d + o_out, (size_t)n * 4 * sizeof(E), cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        }
+        if (e != cudaSuccess) rc = fail(DPB_ECUDA, "logup trees: %s", cudaGetErrorString(e));
     }
-    uint64_t half = 1ull << (m - 1);
-    if (kind == DPB_LOGUP_LOOKUP)
-        logup_initial_lookup<F><<<grid_for(ctx, half), kThreads, 0, ctx->stream>>>(c, half, (E*)lu->num[0], (E*)lu->den[0]);
-    else
-        logup_initial_table<F><<<grid_for(ctx, half), kThreads, 0, ctx->stream>>>(c, mult->ptr, mult->dtype, half,
-                                                                                   (E*)lu->num[0], (E*)lu->den[0]);
-    for (uint32_t l = 2; l <= levels; l++) {
-        half = 1ull << (m - l);
-        if (half <= kSmallLevel) {
-            // levels l..levels in one launch (they lie one behind the other in the slab)
-            logup_small_levels<F><<<1, kThreads, 0, ctx->stream>>>((const E*)lu->num[l - 2], (const E*)lu->den[l - 2], half,
-                                                                   (E*)lu->num[l - 1]);
+    device_free(ctx, d);
+    return rc;
+}
+
+int logup_build_batch(dpb_ctx* ctx, const LogupSpec* specs, uint32_t n, dpb_logup** out, void* host_outputs) {
+    if (!ctx || !specs || !out || n == 0) return fail(DPB_EINVAL, "null argument");
+    for (uint32_t i = 0; i < n; i++) {
+        out[i] = nullptr;
+        DPB_TRY(check_spec(ctx, specs[i]));
+        if (is_gl(specs[i].columns[0]->dtype) != is_gl(specs[0].columns[0]->dtype))
+            return fail(DPB_EINVAL, "instance %u is of another field", i);
+    }
+    const bool gl = is_gl(specs[0].columns[0]->dtype);
+    int rc = DPB_OK;
+    for (uint32_t i = 0; i < n && rc == DPB_OK; i++) {
+        out[i] = new (std::nothrow) dpb_logup();
+        if (!out[i]) {
+            rc = fail(DPB_ENOMEM, "host allocation failed");
             break;
         }
-        logup_next_level<F><<<grid_for(ctx, half), kThreads, 0, ctx->stream>>>(
-            (const E*)lu->num[l - 2], (const E*)lu->den[l - 2], half, (E*)lu->num[l - 1], (E*)lu->den[l - 1]);
+        out[i]->ctx = ctx;
+        out[i]->gl = gl;
+        out[i]->m = log2u(specs[i].columns[0]->len);
     }
-    DPB_CUDA(cudaGetLastError());
-    return DPB_OK;
+    if (rc == DPB_OK) rc = gl ? build_trees<GlFam>(ctx, specs, n, out, host_outputs) : build_trees<FrFam>(ctx, specs, n, out, host_outputs);
+    if (rc != DPB_OK)
+        for (uint32_t i = 0; i < n; i++) {
+            dpb_logup_free(out[i]);
+            out[i] = nullptr;
+        }
+    return rc;
 }
 
 }  // namespace dpb
@@ -80,34 +153,15 @@ int dpb_logup_build(dpb_ctx* ctx, int kind, dpb_mle* const* columns, uint32_t n_
                     const dpb_mle* mult, const void* constant_chal, const void* sep_chal,
                     dpb_logup** out) {
     if (!ctx || !columns || !constant_chal || !sep_chal || !out) return fail(DPB_EINVAL, "null argument");
-    if (kind != DPB_LOGUP_LOOKUP && kind != DPB_LOGUP_TABLE) return fail(DPB_EINVAL, "unknown kind %d", kind);
-    if (n_cols < 1 || n_cols > (uint32_t)kMaxLogupCols)
-        return fail(DPB_EINVAL, "No column evals were provided or too many (%u, max %d)", n_cols, kMaxLogupCols);
-    if ((kind == DPB_LOGUP_TABLE) != (mult != nullptr))
-        return fail(DPB_EINVAL, "multiplicities are required for tables and only for tables");
-    for (uint32_t j = 0; j < n_cols; j++)
-        if (!columns[j] || columns[j]->ctx != ctx) return fail(DPB_EINVAL, "column %u is null or foreign", j);
-    const uint64_t len = columns[0]->len;
-    const bool gl = is_gl(columns[0]->dtype);
-    for (uint32_t j = 1; j < n_cols; j++) {
-        if (columns[j]->len != len) return fail(DPB_EINVAL, "All sets of evaluations should be the same length");
-        if (is_gl(columns[j]->dtype) != gl) return fail(DPB_EINVAL, "columns mix fields");
-    }
-    if (mult && (mult->len != len || is_gl(mult->dtype) != gl))
-        return fail(DPB_EINVAL, "Multiplicities length was not equal to column evaluations length, multiplicities: %llu, columns: %llu",
-                    (unsigned long long)mult->len, (unsigned long long)len);
-    if (len < 4) return fail(DPB_EINVAL, "columns need at least 4 entries, got %llu", (unsigned long long)len);
-    dpb_logup* lu = new (std::nothrow) dpb_logup();
-    if (!lu) return fail(DPB_ENOMEM, "host allocation failed");
-    lu->ctx = ctx;
-    lu->gl = gl;
-    lu->m = log2u(len);
-    int rc = gl ? build_tree<GlFam>(lu, kind, columns, n_cols, mult, constant_chal, sep_chal)
-                : build_tree<FrFam>(lu, kind, columns, n_cols, mult, constant_chal, sep_chal);
-    if (rc != DPB_OK) {
-        dpb_logup_free(lu);
-        return rc;
-    }
+    LogupSpec p;
+    p.kind = kind;
+    p.columns = columns;
+    p.n_cols = n_cols;
+    p.mult = mult;
+    p.constant = constant_chal;
+    p.sep = sep_chal;
+    dpb_logup* lu = nullptr;
+    DPB_TRY(logup_build_batch(ctx, &p, 1, &lu, nullptr));
     *out = lu;
     return DPB_OK;
 }

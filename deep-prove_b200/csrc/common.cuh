@@ -217,6 +217,19 @@ int stage_to_device(dpb_ctx* ctx, const void* host, size_t bytes, size_t offset,
 // rank: a copy.  Bounded wait; DPB_EINVAL when nranks * bytes exceeds the context's exchange buffer.
 int comm_allgather_host(dpb_ctx* ctx, const void* in, size_t bytes, void* out);
 
+// One instance of a logup batch, as dpb_logup_build takes it.
+struct LogupSpec {
+    int kind;
+    dpb_mle* const* columns;
+    uint32_t n_cols;
+    const dpb_mle* mult;
+    const void* constant;  // challenge elements on the host
+    const void* sep;
+};
+// dpb_logup_build for n instances of one field in one go (api_logup.cu); host_outputs, when given, receives the trees'
+// outputs (dpb_logup_outputs, 4 elements each), and the call then waits for them.  out: n handles, all or none.
+int logup_build_batch(dpb_ctx* ctx, const LogupSpec* specs, uint32_t n, dpb_logup** out, void* host_outputs);
+
 // What the batched logup prover knows about a layer sumcheck it is about to run (host/logup.hpp): the instances in the
 // order of the sumcheck's tables, and the layer's constants.  sumcheck_hint_logup hands it to a sumcheck right after
 // dpb_sumcheck_begin; when the sumcheck runs in split-eq form with that single eq table, its large rounds then use

@@ -78,13 +78,29 @@ template <class F>
 class LogUpCircuit {
    public:
     typedef typename F::E E;
-    LogUpCircuit(dpb_ctx* ctx, ProofType kind, std::vector<dpb_mle*> cols, dpb_mle* mult, const E& constant,
-                 const E& sep)
+    LogUpCircuit(ProofType kind, std::vector<dpb_mle*> cols, dpb_mle* mult, const E& constant, const E& sep)
         : kind_(kind), cols_(std::move(cols)), mult_(mult), constant_(constant), sep_(sep) {
         m_ = 0;
         while ((1ull << m_) < dpb_mle_len(cols_[0])) m_++;
-        check(dpb_logup_build(ctx, kind == ProofType::Table ? DPB_LOGUP_TABLE : DPB_LOGUP_LOOKUP, cols_.data(),
-                              (uint32_t)cols_.size(), mult_, &constant_, &sep_, &tree_));
+    }
+    // the trees of all circuits of a batch at once; their outputs, 4 elements each
+    static std::vector<E> build(dpb_ctx* ctx, const std::vector<std::unique_ptr<LogUpCircuit>>& circuits) {
+        std::vector<dpb::LogupSpec> specs;
+        for (const auto& c : circuits) {
+            dpb::LogupSpec p;
+            p.kind = c->kind_ == ProofType::Table ? DPB_LOGUP_TABLE : DPB_LOGUP_LOOKUP;
+            p.columns = c->cols_.data();
+            p.n_cols = (uint32_t)c->cols_.size();
+            p.mult = c->mult_;
+            p.constant = &c->constant_;
+            p.sep = &c->sep_;
+            specs.push_back(p);
+        }
+        std::vector<dpb_logup*> trees(specs.size(), nullptr);
+        std::vector<E> outputs(4 * specs.size());
+        check(dpb::logup_build_batch(ctx, specs.data(), (uint32_t)specs.size(), trees.data(), outputs.data()));
+        for (size_t i = 0; i < trees.size(); i++) circuits[i]->tree_ = trees[i];
+        return outputs;
     }
     LogUpCircuit(const LogUpCircuit&) = delete;
     LogUpCircuit& operator=(const LogUpCircuit&) = delete;
@@ -303,13 +319,13 @@ LogUpBatchProof<F> new_batch_multiple_sizes_prove(dpb_ctx* ctx, const std::vecto
     std::vector<std::unique_ptr<LogUpCircuit<F>>> circuits;
     for (const auto& in : input) {
         if (in.kind == ProofType::Table) {
-            circuits.emplace_back(new LogUpCircuit<F>(ctx, in.kind, in.column_evals, in.multiplicities,
+            circuits.emplace_back(new LogUpCircuit<F>(in.kind, in.column_evals, in.multiplicities,
                                                       in.constant_challenge, in.column_separation_challenge));
         } else {
             for (size_t i = 0; i < in.column_evals.size(); i += in.columns_per_instance) {
                 std::vector<dpb_mle*> cols(in.column_evals.begin() + i,
                                            in.column_evals.begin() + i + in.columns_per_instance);
-                circuits.emplace_back(new LogUpCircuit<F>(ctx, in.kind, cols, nullptr, in.constant_challenge,
+                circuits.emplace_back(new LogUpCircuit<F>(in.kind, cols, nullptr, in.constant_challenge,
                                                           in.column_separation_challenge));
             }
         }
@@ -325,14 +341,10 @@ LogUpBatchProof<F> new_batch_multiple_sizes_prove(dpb_ctx* ctx, const std::vecto
 
     LogUpBatchProof<F> proof;
     proof.proof_type = proof_type;
+    // every circuit's tree and outputs (LogUpCircuit::outputs, circuit.rs:558-560) with one wait for the device
+    const std::vector<E> flat = LogUpCircuit<F>::build(ctx, circuits);
     t_trees.stop();
     {
-        dpb::TracePhase t_out("logup.outputs");
-        // every circuit's outputs (LogUpCircuit::outputs, circuit.rs:558-560) with one wait for the device
-        std::vector<const dpb_logup*> trees;
-        for (const auto& c : circuits) trees.push_back(c->tree());
-        std::vector<E> flat(4 * trees.size());
-        check(dpb_logup_outputs_batch(trees.data(), (uint32_t)trees.size(), flat.data()));
         if (partial) {
             // every rank must hold the same shapes: compare a signature before anything depends on it
             std::vector<E> sig;
@@ -345,12 +357,12 @@ LogUpBatchProof<F> new_batch_multiple_sizes_prove(dpb_ctx* ctx, const std::vecto
                 if (memcmp(sigs.data() + q * sig.size(), sig.data(), sig.size() * sizeof(E)) != 0)
                     throw Error(DPB_EINVAL, "the ranks of a partial logup batch must hold instances of the same shapes");
             const std::vector<E> all = gather(flat);
-            for (size_t i = 0; i < trees.size(); i++)
+            for (size_t i = 0; i < circuits.size(); i++)
                 for (size_t q = 0; q < G; q++)
                     proof.circuit_outputs.emplace_back(all.begin() + q * flat.size() + 4 * i,
                                                        all.begin() + q * flat.size() + 4 * i + 4);
         } else {
-            for (size_t i = 0; i < trees.size(); i++)
+            for (size_t i = 0; i < circuits.size(); i++)
                 proof.circuit_outputs.emplace_back(flat.begin() + 4 * i, flat.begin() + 4 * i + 4);
         }
     }

@@ -62,4 +62,32 @@ struct EntrySum<GlFam, INT> {
     }
 };
 
+// c u + a d, reduced once
+template <class F>
+struct TwoProducts;
+template <>
+struct TwoProducts<FrFam> {
+    __device__ __forceinline__ static Fr sum(const Fr& c, const Fr& u, const Fr& a, const Fr& d) {
+        frw::Wide s = frw::wide_zero();
+        frw::wide_mac(s, frw::from_fr(c), frw::from_fr(u));
+        frw::wide_mac(s, frw::from_fr(a), frw::from_fr(d));
+        return fr_wide_finish(s);
+    }
+};
+template <>
+struct TwoProducts<GlFam> {
+    __device__ __forceinline__ static Gl2 sum(const Gl2& c, const Gl2& u, const Gl2& a, const Gl2& d) {
+        glw::A8 s0 = glw::acc_zero(), s1 = glw::acc_zero();
+        auto mac = [&](const glw::W2& x, const glw::W2& y) {
+            glw::acc_mac(s0, x.c0, y.c0);
+            glw::acc_mac(s0, glw::mul7(x.c1), y.c1);
+            glw::acc_mac(s1, x.c0, y.c1);
+            glw::acc_mac(s1, x.c1, y.c0);
+        };
+        mac(gl2_words(c), gl2_words(u));
+        mac(gl2_words(a), gl2_words(d));
+        return gl2_make(glw::to_u64(glw::canon(glw::acc_reduce(s0))), glw::to_u64(glw::canon(glw::acc_reduce(s1))));
+    }
+};
+
 }  // namespace dpb

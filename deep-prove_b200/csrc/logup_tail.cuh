@@ -23,6 +23,7 @@
 
 #include "logup_tail.hpp"
 #include "generic_round.cuh"
+#include "lazy_sum.cuh"
 
 namespace dpb {
 
@@ -59,34 +60,6 @@ __host__ __device__ __forceinline__ size_t logup_tail_set_entries(size_t nb, uin
 __host__ __device__ __forceinline__ size_t logup_tail_weights(size_t nb, uint32_t blocks, uint32_t alone) {
     return blocks > 1 && alone > nb ? alone : nb;
 }
-
-// c u + a d, reduced once
-template <class F>
-struct LogupSum;
-template <>
-struct LogupSum<FrFam> {
-    __device__ __forceinline__ static Fr two(const Fr& c, const Fr& u, const Fr& a, const Fr& d) {
-        frw::Wide s = frw::wide_zero();
-        frw::wide_mac(s, frw::from_fr(c), frw::from_fr(u));
-        frw::wide_mac(s, frw::from_fr(a), frw::from_fr(d));
-        return fr_wide_finish(s);
-    }
-};
-template <>
-struct LogupSum<GlFam> {
-    __device__ __forceinline__ static Gl2 two(const Gl2& c, const Gl2& u, const Gl2& a, const Gl2& d) {
-        glw::A8 s0 = glw::acc_zero(), s1 = glw::acc_zero();
-        auto mac = [&](const glw::W2& x, const glw::W2& y) {
-            glw::acc_mac(s0, x.c0, y.c0);
-            glw::acc_mac(s0, glw::mul7(x.c1), y.c1);
-            glw::acc_mac(s1, x.c0, y.c1);
-            glw::acc_mac(s1, x.c1, y.c0);
-        };
-        mac(gl2_words(c), gl2_words(u));
-        mac(gl2_words(a), gl2_words(d));
-        return gl2_make(glw::to_u64(glw::canon(glw::acc_reduce(s0))), glw::to_u64(glw::canon(glw::acc_reduce(s1))));
-    }
-};
 
 // entry e of an original table in the kernel's first round
 template <class F>
@@ -254,9 +227,9 @@ __global__ void __launch_bounds__(kTailThreads)
                 } else {
                     const E u0 = cur.get(in.tab0 + 2, 2 * p), a0 = cur.get(in.tab0 + 3, 2 * p);
                     const E u1 = cur.get(in.tab0 + 2, 2 * p + 1), a1 = cur.get(in.tab0 + 3, 2 * p + 1);
-                    g0 = LogupSum<F>::two(c0, u0, a0, d0);
-                    gi = LogupSum<F>::two(dc, F::sub(u1, u0), F::sub(a1, a0), dd);
-                    if (with_one) g1 = LogupSum<F>::two(c1, u1, a1, d1);
+                    g0 = TwoProducts<F>::sum(c0, u0, a0, d0);
+                    gi = TwoProducts<F>::sum(dc, F::sub(u1, u0), F::sub(a1, a0), dd);
+                    if (with_one) g1 = TwoProducts<F>::sum(c1, u1, a1, d1);
                 }
                 g0 = F::mul(g0, wt);
                 gi = F::mul(gi, wt);
