@@ -5,8 +5,6 @@
 // and evaluates (two launches on the fallback path for very many tables).  The
 // kernel's last block writes the round polynomial straight into mapped host
 // memory and raises a flag the host polls.
-#include <atomic>
-#include <chrono>
 #include <mutex>
 
 #include "common.cuh"
@@ -19,11 +17,10 @@
 #include "comm.cuh"
 #include "eq_pairs.cuh"
 #include "eq_pairs.hpp"
-#include "logup_tail.hpp"
+#include "tail_host.hpp"
 
 namespace dpb {
 
-constexpr size_t kSlabCacheMax = (size_t)4 << 30;  // larger blocks (claim batching over a whole model) are not kept
 constexpr int kOnePassMaxSmem = 200 * 1024;  // dynamic shared memory the one-pass generic rounds may use
 
 struct MleTrack {
@@ -91,17 +88,6 @@ struct dpb_sc {
     uint32_t n_groups = 0;
     uint32_t op_threads = 0;
     size_t op_smem = 0;
-    bool logup_ok = false;       // a usable hint of the logup prover: sc_round_logup runs the large rounds
-    void* d_logup = nullptr;     // [LogupConsts[n] | LogupInst[n]] (own allocation)
-    uint32_t logup_n = 0, logup_eq = 0;
-    alignas(16) uint8_t logup_lambda[32] = {0};
-    // the last rounds of a hinted logup layer (logup_tail.cuh)
-    LogupTailPlan lt;
-    bool lt_active = false;       // the running resident kernel is that one
-    uint32_t lt_first = 0;        // its first round and the challenges it got since, for playing them again
-    std::vector<uint8_t> lt_chal;
-    bool lt_have_h = false;       // the previous round's H and q are in lt_h: H(0), h1, h2, q
-    alignas(16) uint8_t lt_h[4 * 32] = {0};
     bool seg_ok = false;         // the program splits into segments over few tables each: sc_round_seg runs the large rounds
     void* d_segs = nullptr;
     void* d_seg_prog = nullptr;
@@ -521,8 +507,8 @@ static void plan_program(dpb_sc* sc, const dpb_term* terms, dpb_mle* const* mles
             sc->tail_start = i;
         }
     }
-    // split-eq form for the rounds before the resident kernel's, and for a logup layer (degree 3) for all of them
-    if (sc->tail_start > 0 || sc->d == 3) plan_spliteq<F>(sc, mles, groups, prog);
+    // split-eq form for the rounds before the resident kernel's
+    if (sc->tail_start > 0) plan_spliteq<F>(sc, mles, groups, prog);
 }
 
 // per-round descriptors of the one-pass kernels: which tables are bound inside the round's kernel
@@ -575,47 +561,6 @@ static void spliteq_advance(dpb_sc* sc, uint32_t i, const typename F::E& r) {
     }
 }
 
-// The large rounds of a logup layer from the layer's own formula (see sumcheck_hint_logup).
-template <class F>
-static int launch_logup(dpb_sc* sc, uint32_t round, uint64_t n_pairs, const typename F::E& r, const SplitEqArgs<F>& eq) {
-    typedef typename F::E E;
-    dpb_ctx* ctx = sc->ctx;
-    const uint64_t per_sm = sizeof(E) == 16 ? 4 : 3;  // resident blocks: 126 registers per thread (Goldilocks), 168 (BN254)
-    // blocks of 128 threads, of 64 when the pairs do not fill the GPU even then; and when they still do not, the
-    // instances are cut into slices that run as blocks of their own
-    uint32_t threads = 128;
-    if (n_pairs < (uint64_t)ctx->sm_count * threads) threads = 64;
-    uint64_t blocks_x = (n_pairs + threads - 1) / threads;
-    const uint64_t room = (uint64_t)ctx->sm_count * per_sm * (128 / threads);
-    if (blocks_x > room) blocks_x = room;
-    uint32_t slices = 1;
-    if (blocks_x < room) slices = (uint32_t)std::min<uint64_t>(sc->logup_n, room / blocks_x);
-    const uint32_t inst_per_slice = (sc->logup_n + slices - 1) / slices;
-    slices = (sc->logup_n + inst_per_slice - 1) / inst_per_slice;
-    uint64_t blocks = blocks_x * slices;
-    if (blocks > ctx->max_blocks) {
-        slices = 1;
-        blocks = blocks_x = std::min<uint64_t>(blocks_x, ctx->max_blocks);
-    }
-    const RoundTab* tabs = sc->d_rtab_eq + (size_t)round * sc->k;
-    const typename F::FoldKey rk = F::fold_key(r);
-    E lam;
-    memcpy(&lam, sc->logup_lambda, sizeof(E));
-    const typename F::FoldKey lamk = F::fold_key(lam);
-    const LogupConsts<F>* consts = (const LogupConsts<F>*)sc->d_logup;
-    const LogupInst* inst = (const LogupInst*)((const char*)sc->d_logup + (size_t)sc->logup_n * sizeof(LogupConsts<F>));
-    const size_t smem = (size_t)sc->logup_n * (sizeof(LogupConsts<F>) + sizeof(LogupInst));
-    if (round > 0)
-        sc_round_logup<F, true><<<(uint32_t)blocks, threads, smem, ctx->stream>>>(
-            tabs, inst, consts, sc->logup_n, rk, lamk, sc->logup_eq, eq.scale[0], eq.stride_log2[0], n_pairs,
-            (uint32_t)blocks_x, slices == 1 ? sc->logup_n : inst_per_slice, reduce_scratch<F>(ctx), (E*)ctx->round_out);
-    else
-        sc_round_logup<F, false><<<(uint32_t)blocks, threads, smem, ctx->stream>>>(
-            tabs, inst, consts, sc->logup_n, rk, lamk, sc->logup_eq, eq.scale[0], eq.stride_log2[0], n_pairs,
-            (uint32_t)blocks_x, slices == 1 ? sc->logup_n : inst_per_slice, reduce_scratch<F>(ctx), (E*)ctx->round_out);
-    return DPB_OK;
-}
-
 template <class F, int D>
 static int launch_spliteq(dpb_sc* sc, uint32_t round, uint64_t n_pairs, const typename F::E& r) {
     typedef typename F::E E;
@@ -638,10 +583,6 @@ static int launch_spliteq(dpb_sc* sc, uint32_t round, uint64_t n_pairs, const ty
         eq.stride_log2[eq.n_eq] = ip + 1;
         eq.scale[eq.n_eq] = F::mul(S, iz);
         eq.n_eq++;
-    }
-    if constexpr (D == 3) {
-        if (sc->logup_ok && eq.n_eq == 1 && eq.const_groups == 0 && eq.table[0] == sc->logup_eq)
-            return launch_logup<F>(sc, round, n_pairs, r, eq);
     }
     if constexpr (D >= 2 && D <= 4) {
         if (sc->seg_ok) return launch_seg<F, D, true>(sc, round, n_pairs, r, eq);
@@ -725,39 +666,6 @@ static int spliteq_materialize(dpb_sc* sc, uint32_t i) {
 // ---- resident last-rounds kernel: host side -------------------------------------
 
 
-// Polls the mailbox until `ready` holds; bounded, and the stream is queried now and then so that a
-// kernel that died or returned early surfaces as an error.
-constexpr int kTailNoHost = 1;  // internal: the kernel found that launches block the host; fall back to launches
-constexpr int kTailGaveUp = 2;  // internal: the kernel's wait for a challenge ran out and it returned
-
-template <class Ready>
-static int tail_wait_host(dpb_ctx* ctx, TailBox* box, Ready ready) {
-    uint64_t spins = 0;
-    std::chrono::steady_clock::time_point t0;
-    while (!ready()) {
-        if (box->status == 3) return kTailNoHost;
-        if (box->status == 2) {
-            // the host may have been held up between the two looks: what it waits for can have come first
-            std::atomic_thread_fence(std::memory_order_acquire);
-            if (ready()) break;
-            return kTailGaveUp;
-        }
-        if ((++spins & 0xFFF) == 0) {
-            cudaError_t e = cudaStreamQuery(ctx->tail_stream);
-            if (e != cudaSuccess && e != cudaErrorNotReady)
-                return fail(DPB_ECUDA, "resident round kernel: %s", cudaGetErrorString(e));
-            if (e == cudaSuccess && box->status != 2 && box->status != 3 && !ready())
-                return fail(DPB_ECUDA, "the resident round kernel returned without a result (%s)",
-                            cudaGetErrorString(cudaGetLastError()));
-            if (spins == 0x1000) t0 = std::chrono::steady_clock::now();
-            else if (std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > 120.0)
-                return fail(DPB_ETIMEOUT, "the resident round kernel did not answer within 120 s");
-        }
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    return DPB_OK;
-}
-
 template <class F, int D>
 static int launch_tail(dpb_sc* sc, uint32_t round, const typename F::E& r) {
     dpb_ctx* ctx = sc->ctx;
@@ -783,29 +691,6 @@ static int launch_tail(dpb_sc* sc, uint32_t round, const typename F::E& r) {
                                 (TailBox*)ctx->tail_box_dev, ctx->tail_wait_ns, sc->tail_prog_in_smem ? 1u : 0u,
                                 sc->tail_slots_offset, sc->tail_alone));
     return DPB_OK;
-}
-
-// the challenge as chunks: data first, then the sequence numbers
-template <class E>
-static void tail_post(TailBox* box, const void* chal, uint32_t seq) {
-    const uint64_t* w = (const uint64_t*)chal;
-    constexpr int W8 = sizeof(E) / 8;
-    for (int i = 0; i < W8; i++) ((volatile TailChunk*)box->chal)[i].data = w[i];
-    std::atomic_thread_fence(std::memory_order_release);
-    for (int i = 0; i < W8; i++) ((volatile TailChunk*)box->chal)[i].seq = seq;
-}
-// element `idx` of a chunk array, once every chunk of it carries `seq`
-template <class E>
-static bool tail_take(const TailChunk* base, uint32_t idx, uint32_t seq, E* out) {
-    constexpr int W8 = sizeof(E) / 8;
-    const volatile TailChunk* c = (const volatile TailChunk*)base + (size_t)idx * W8;
-    uint64_t* w = (uint64_t*)out;
-    for (int i = 0; i < W8; i++) {
-        if (c[i].seq != seq) return false;
-        std::atomic_thread_fence(std::memory_order_acquire);
-        w[i] = c[i].data;
-    }
-    return true;
 }
 
 // Round i through the resident kernel: start it (first use) or post the challenge
@@ -920,172 +805,6 @@ static int tail_finish(dpb_sc* sc, const void* last_challenge, void* out) {
     return rc;
 }
 
-// ---- resident last rounds of a logup layer: host side -------------------------------
-
-// (Re)starts the kernel at its first round; r is the challenge that ended the round before.
-template <class F>
-static int lt_start_kernel(dpb_sc* sc, const typename F::E& r) {
-    typedef typename F::E E;
-    dpb_ctx* ctx = sc->ctx;
-    TailBox* box = (TailBox*)ctx->tail_box_host;
-    memset(box, 0, sizeof(TailBox));
-    std::atomic_thread_fence(std::memory_order_seq_cst);
-    DPB_CUDA(cudaEventRecord(ctx->tail_ev[0], ctx->stream));
-    DPB_CUDA(cudaStreamWaitEvent(ctx->tail_stream, ctx->tail_ev[0], 0));
-    const auto& lead = sc->eq_leads[0];
-    E lam;
-    memcpy(&lam, sc->logup_lambda, sizeof(E));
-    DPB_TRY(logup_tail_launch<F>(ctx, sc->lt, sc->d_rtab_eq + (size_t)sc->lt_first * sc->k, sc->tr[lead.table].orig,
-                                 sc->lt_first + 1, lam, r, sc->lt_first, sc->n));
-    ((volatile TailChunk*)&box->hello)->seq = 1;
-    DPB_CUDA(cudaEventRecord(ctx->tail_ev[1], ctx->tail_stream));
-    ctx->sumcheck_launches++;
-    return DPB_OK;
-}
-
-// the samples of round j: H(0), H(1) (round 0 only) and H at infinity, without the eq table's scalar
-template <class F>
-static int lt_take(dpb_sc* sc, uint32_t j, typename F::E* raw) {
-    TailBox* box = (TailBox*)sc->ctx->tail_box_host;
-    uint32_t x = 0;
-    return tail_wait_host(sc->ctx, box, [&] {
-        while (x <= 2) {
-            if (j > 0 && x == 1) {
-                x++;
-                continue;
-            }
-            if (!tail_take<typename F::E>(box->evals, x, j + 1, &raw[x])) return false;
-            x++;
-        }
-        return true;
-    });
-}
-
-// The kernel gave up waiting (the host was held up): start it again and play the rounds before `upto` with the
-// challenges they had, and the challenge after them.
-template <class F>
-static int lt_replay(dpb_sc* sc, uint32_t upto) {
-    typedef typename F::E E;
-    dpb_ctx* ctx = sc->ctx;
-    DPB_CUDA(cudaStreamSynchronize(ctx->tail_stream));  // it has returned; make that certain
-    const E* ch = (const E*)sc->lt_chal.data();
-    DPB_TRY(lt_start_kernel<F>(sc, ch[0]));
-    for (uint32_t j = sc->lt_first; j < upto; j++) {
-        E raw[3];
-        const int rc = lt_take<F>(sc, j, raw);
-        if (rc != DPB_OK) return rc < 0 ? rc : fail(DPB_ETIMEOUT, "the resident round kernel gave up waiting for a challenge");
-        tail_post<E>((TailBox*)ctx->tail_box_host, &ch[j + 1 - sc->lt_first], j + 1);
-    }
-    return DPB_OK;
-}
-
-// Round i: posts the challenge (or starts the kernel), makes the claim while the kernel works, takes the samples and
-// turns them into the round message.  kTailNoHost: launches block the host, nothing has run.
-template <class F>
-static int lt_round(dpb_sc* sc, uint32_t i, const typename F::E& r, typename F::E* out) {
-    typedef typename F::E E;
-    dpb_ctx* ctx = sc->ctx;
-    const bool first = !sc->lt_active;
-    if (first) {
-        sc->lt_first = i;
-        sc->lt_chal.clear();
-        DPB_TRY(lt_start_kernel<F>(sc, r));
-        sc->lt_active = sc->tail_active = true;
-        ctx->tail_owner = sc;
-    } else {
-        tail_post<E>((TailBox*)ctx->tail_box_host, &r, i);
-    }
-    sc->lt_chal.insert(sc->lt_chal.end(), (const uint8_t*)&r, (const uint8_t*)&r + sizeof(E));
-    // s(0) + s(1) of this round = the previous round's polynomial at r
-    spliteq_inverses<F>(sc);
-    const E one = F::one();
-    E claim = F::zero(), q, inv_q, S, iz;
-    E* h = (E*)sc->lt_h;
-    if (i > 0) {
-        if (sc->lt_have_h) {
-            const E l = F::add(F::sub(one, h[3]), F::mul(F::sub(F::add(h[3], h[3]), one), r));
-            claim = F::mul(l, F::add(h[0], F::mul(r, F::add(h[1], F::mul(r, h[2])))));
-        } else {
-            claim = lagrange_eval<F>((int)sc->d, (const E*)sc->prev_evals, (const E*)sc->lag_w, r);
-        }
-    }
-    memcpy(&q, sc->round_q.data() + (size_t)i * sizeof(E), sizeof(E));
-    memcpy(&inv_q, sc->round_inv_q.data() + (size_t)i * sizeof(E), sizeof(E));
-    memcpy(&S, sc->eq_leads[0].S, sizeof(E));
-    memcpy(&iz, sc->eq_leads[0].inv_zp.data() + (size_t)(i + 1) * sizeof(E), sizeof(E));
-    const E kappa = F::mul(S, iz), q0 = F::sub(one, q);
-    E raw[3];
-    int rc = lt_take<F>(sc, i, raw);
-    if (rc == kTailNoHost) {
-        cudaStreamSynchronize(ctx->tail_stream);
-        ctx->tail_enabled = false;
-        sc->lt_active = sc->tail_active = false;
-        ctx->tail_owner = nullptr;
-        return rc;
-    }
-    if (rc == kTailGaveUp && !first) {
-        DPB_TRY(lt_replay<F>(sc, i));
-        rc = lt_take<F>(sc, i, raw);
-    }
-    if (rc == kTailGaveUp) return fail(DPB_ETIMEOUT, "the resident round kernel gave up waiting for a challenge");
-    if (rc != DPB_OK) return rc;
-    const E H0 = F::mul(kappa, raw[0]), Hi = F::mul(kappa, raw[2]);
-    // s(0) + s(1) = (1 - q) H(0) + q H(1)
-    const E H1 = i == 0 ? F::mul(kappa, raw[1]) : F::mul(F::sub(claim, F::mul(q0, H0)), inv_q);
-    const E h1 = F::sub(F::sub(H1, H0), Hi);
-    // H(x) = H0 + h1 x + Hi x^2 by differences; s(x) = ((1 - q) + (2 q - 1) x) H(x)
-    const E slope = F::sub(q, q0), step2 = F::add(Hi, Hi);
-    E H = H0, step = F::add(h1, Hi), l = q0;
-    for (uint32_t x = 0; x <= 3; x++) {
-        out[x] = F::mul(l, H);
-        H = F::add(H, step);
-        step = F::add(step, step2);
-        l = F::add(l, slope);
-    }
-    h[0] = H0;
-    h[1] = h1;
-    h[2] = Hi;
-    h[3] = q;
-    sc->lt_have_h = true;
-    return DPB_OK;
-}
-
-template <class F>
-static int lt_finish(dpb_sc* sc, const void* last_challenge, void* out) {
-    typedef typename F::E E;
-    dpb_ctx* ctx = sc->ctx;
-    TailBox* box = (TailBox*)ctx->tail_box_host;
-    tail_post<E>(box, last_challenge, sc->n);
-    E r;
-    memcpy(&r, last_challenge, sizeof(E));
-    sc->lt_chal.insert(sc->lt_chal.end(), (const uint8_t*)&r, (const uint8_t*)&r + sizeof(E));
-    uint32_t j = 0;
-    auto take = [&] {
-        while (j < sc->k) {
-            if (j != sc->lt.eq_table && !tail_take<E>(box->finals, j, sc->n + 1, (E*)out + j)) return false;
-            j++;
-        }
-        return true;
-    };
-    int rc = tail_wait_host(ctx, box, take);
-    if (rc == kTailGaveUp) {
-        rc = lt_replay<F>(sc, sc->n);
-        if (rc == DPB_OK) rc = tail_wait_host(ctx, box, take);
-        if (rc == kTailGaveUp) rc = fail(DPB_ETIMEOUT, "the resident round kernel gave up waiting for a challenge");
-    }
-    // later work of this context (frees, the next sumcheck) is ordered after the kernel's end
-    cudaStreamWaitEvent(ctx->stream, ctx->tail_ev[1], 0);
-    sc->lt_active = sc->tail_active = false;
-    ctx->tail_owner = nullptr;
-    if (rc != DPB_OK) return rc;
-    const auto& l = sc->eq_leads[0];
-    E q, S;
-    memcpy(&q, l.q.data() + (size_t)(sc->n - 1) * sizeof(E), sizeof(E));
-    memcpy(&S, l.S, sizeof(E));
-    ((E*)out)[l.table] = F::mul(S, eq_scalar<F>(q, r));
-    return DPB_OK;
-}
-
 // A sumcheck that is dropped before its last round: tell the kernel to leave and wait for it.
 static void tail_abort(dpb_sc* sc) {
     dpb_ctx* ctx = sc->ctx;
@@ -1093,7 +812,7 @@ static void tail_abort(dpb_sc* sc) {
     for (int i = 0; i < 4; i++) ((volatile TailChunk*)box->chal)[i].seq = kTailAbort;
     std::atomic_thread_fence(std::memory_order_seq_cst);
     cudaStreamSynchronize(ctx->tail_stream);  // bounded by the kernel's own wait limit
-    sc->tail_active = sc->lt_active = false;
+    sc->tail_active = false;
     ctx->tail_owner = nullptr;
 }
 
@@ -1210,39 +929,7 @@ static void launch_fused(dpb_ctx* ctx, const MleDesc* desc, const FoldDesc* fold
     else launch_fused_fr<4>(ctx, desc, folds, round, r, n_pairs);
 }
 
-// Collects the sums of the round just launched from the chunk area in mapped host memory: every chunk carries
-// the launch's sequence number once it has arrived.  The stream is queried now and then so that a failed launch
-// surfaces, and the wait is bounded.
-static int wait_round_chunks(dpb_ctx* ctx, size_t msg_bytes, void* out) {
-    const unsigned int want = ctx->done_value;
-    const volatile TailChunk* c = (const volatile TailChunk*)ctx->result_host;
-    uint64_t* dst = (uint64_t*)out;
-    uint64_t spins = 0;
-    std::chrono::steady_clock::time_point t0;
-    for (size_t w = 0; w < msg_bytes / 8; w++) {
-        while (c[w].seq != want) {
-            if ((++spins & 0xFFF) == 0) {
-                cudaError_t e = cudaStreamQuery(ctx->stream);
-                if (e != cudaSuccess && e != cudaErrorNotReady) return fail(DPB_ECUDA, "round kernel: %s", cudaGetErrorString(e));
-                if (e == cudaSuccess && c[w].seq != want) {
-                    // the stream drained without the result: the launch itself failed
-                    e = cudaGetLastError();
-                    if (c[w].seq == want) break;
-                    return fail(DPB_ECUDA, "round kernel did not deliver its result (%s)", cudaGetErrorString(e));
-                }
-                if (spins == 0x1000) t0 = std::chrono::steady_clock::now();
-                else if (std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > 120.0)
-                    return fail(DPB_ETIMEOUT, "round kernel did not finish within 120 s");
-            }
-        }
-        std::atomic_thread_fence(std::memory_order_acquire);
-        dst[w] = c[w].data;
-    }
-    return DPB_OK;
-}
-
 constexpr uint64_t kSpreadPairs = 4096;  // rounds up to this size of a heavy program are spread over its terms
-constexpr uint64_t kLogupMinPairs = 4096;  // rounds above this size of a hinted logup layer run sc_round_logup
 constexpr uint64_t kSpreadLightPairs = 16384;  // and of any other program (measured: 14-15 % off a logup batch)
 
 template <class F>
@@ -1271,22 +958,7 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
         ctx->done_value = ctx->done_seq;
         ctx->chunk_out_dev = sharded ? nullptr : ctx->result_dev;
     }
-    if (i == 0 && sc->tail_start == 0 && !sc->lt.ok) sc->spliteq = false;  // every round is the generic resident kernel's
     if (sc->spliteq && i > 0) spliteq_advance<F>(sc, i, r);
-    // the last rounds of a hinted logup layer, under the same conditions as the generic resident kernel below
-    if (sc->lt_active || (sc->lt.ok && sc->spliteq && ctx->tail_enabled && !sharded && !ctx->profile && i >= sc->lt.start &&
-                          ctx->tail_owner == nullptr)) {
-        E msg[4];
-        const int rc = lt_round<F>(sc, i, r, msg);
-        if (rc != kTailNoHost) {
-            if (rc != DPB_OK) return rc;
-            sc->eq_unbound = true;
-            memcpy(out_evals, msg, msg_bytes);
-            memcpy(sc->prev_evals, msg, msg_bytes);
-            return DPB_OK;
-        }
-    }
-    sc->lt_have_h = false;
     // the last rounds go to the resident kernel (one per context at a time; not while profiling per launch)
     bool use_tail = sc->tail_active || (sc->has_prog && ctx->tail_enabled && !sharded && !ctx->profile && !sc->heavy &&
                                         i >= sc->tail_start && ctx->tail_owner == nullptr);
@@ -1294,11 +966,7 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
     // (pair, slice of the term list) items: a thread's chain of dependent field products is what such a round
     // waits for, and the spread form makes it several times shorter.  Heavy programs: up to kSpreadPairs pairs;
     // every other program: between the resident kernel's rounds and kSpreadLightPairs.
-    // a logup layer with its own round kernel spreads over instances inside that kernel instead
-    // (down to kLogupMinPairs pairs; measured: a 36-instance batch of 2^18 rows 18.7 -> 17.0 ms, below that no gain)
-    const bool logup_round = sc->logup_ok && sc->spliteq && !use_tail && n_pairs > kLogupMinPairs;
-    const bool spread = !logup_round &&
-                        ((sc->heavy && n_pairs <= kSpreadPairs) ||
+    const bool spread = ((sc->heavy && n_pairs <= kSpreadPairs) ||
                          (!use_tail && !sc->ranged && sc->has_prog && n_pairs <= kSpreadLightPairs)) &&
                         sc->fused_shape != kFusedProduct;
     if (spread && sc->eq_unbound) DPB_TRY(spliteq_materialize<F>(sc, i));
@@ -1438,7 +1106,7 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
             for (uint32_t j = 0; j < sc->k; j++) bytes += dtype_size(sc->tr[j].dtype) << sc->tr[j].nv;
             name = done ? (sc->tr[0].dtype == DPB_GL_BASE ? "fused_eval0<base>"
                            : sc->tr[0].dtype == DPB_FR_I32 ? "fused_eval0<i32>" : "fused_eval0")
-                        : split ? (sc->logup_ok && sc->d == 3 ? "sc_round_logup" : seg ? "sc_round_seg<spliteq>" : "sc_round_spliteq")
+                        : split ? (seg ? "sc_round_seg<spliteq>" : "sc_round_spliteq")
                         : one_pass ? (seg ? "sc_round_seg" : "sc_round_generic") : "sc_eval_generic";
         } else {
             const FoldDesc* fd = sc->h_fold.data() + (size_t)i * sc->k;
@@ -1448,7 +1116,7 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
                 if (sc->h_desc[(size_t)i * sc->k + j].shift >= 0) bytes += dtype_size(sc->tr[j].dtype) << sc->tr[j].nv;
             name = done ? (fd[0].dtype_in == DPB_GL_BASE ? "fused_fold_eval<base>"
                            : fd[0].dtype_in == DPB_FR_I32 ? "fused_fold_eval<i32>" : "fused_fold_eval")
-                        : split ? (sc->logup_ok && sc->d == 3 ? "sc_round_logup" : seg ? "sc_round_seg<spliteq>" : "sc_round_spliteq")
+                        : split ? (seg ? "sc_round_seg<spliteq>" : "sc_round_spliteq")
                         : one_pass ? (seg ? "sc_round_seg" : "sc_round_generic") : "sc_fold_generic+sc_eval_generic";
         }
         bool found = false;
@@ -2026,118 +1694,6 @@ int dpb_sumcheck_begin_sharded(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* 
 
 }  // extern "C"
 
-namespace dpb {
-
-template <class F>
-static void hint_logup_impl(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_inst, const void* lambda, uint32_t eq_table) {
-    typedef typename F::E E;
-    std::vector<LogupConsts<F>> consts(n_inst);
-    std::vector<LogupInst> di(n_inst);
-    memset(consts.data(), 0, consts.size() * sizeof(LogupConsts<F>));
-    for (uint32_t i = 0; i < n_inst; i++) {
-        E a, s, c;
-        memcpy(&a, inst[i].alpha, sizeof(E));
-        memcpy(&s, inst[i].sep, sizeof(E));
-        memcpy(&c, inst[i].constant, sizeof(E));
-        consts[i].alpha = F::fold_key(a);
-        consts[i].sep = F::fold_key(s);
-        consts[i].c = c;
-        di[i].kind = (uint16_t)inst[i].kind;
-        di[i].first = (uint16_t)inst[i].first;
-        di[i].ncol = (uint16_t)inst[i].ncol;
-        di[i].pad = 0;
-    }
-    const size_t round_bytes = n_inst * (sizeof(LogupConsts<F>) + sizeof(LogupInst));
-    if (round_bytes > 96 * 1024) return;
-    // the resident kernel's instances and constants (alpha, sep, constant), after the round kernel's
-    std::vector<LogupTailInst> ti(n_inst);
-    std::vector<E> tc(3 * (size_t)n_inst);
-    uint32_t n_tabs = 0;
-    for (uint32_t i = 0; i < n_inst; i++) {
-        ti[i].kind = (uint16_t)inst[i].kind;
-        ti[i].first = (uint16_t)inst[i].first;
-        ti[i].ncol = (uint16_t)inst[i].ncol;
-        ti[i].tab0 = (uint16_t)n_tabs;
-        n_tabs += (inst[i].kind == kLogupLookup ? 2 : 4) + (inst[i].kind != kLogupInner && inst[i].ncol == 2 ? 2 : 0);
-        memcpy(&tc[3 * i], inst[i].alpha, sizeof(E));
-        memcpy(&tc[3 * i + 1], inst[i].sep, sizeof(E));
-        memcpy(&tc[3 * i + 2], inst[i].constant, sizeof(E));
-    }
-    const size_t o_tc = (round_bytes + 15) & ~(size_t)15, o_ti = o_tc + tc.size() * sizeof(E);
-    const size_t bytes = o_ti + ti.size() * sizeof(LogupTailInst);
-    void* d = nullptr;
-    if (device_alloc(sc->ctx, bytes, &d) != DPB_OK) return;
-    std::vector<uint8_t> blob(bytes, 0);
-    memcpy(blob.data(), consts.data(), n_inst * sizeof(LogupConsts<F>));
-    memcpy(blob.data() + n_inst * sizeof(LogupConsts<F>), di.data(), n_inst * sizeof(LogupInst));
-    memcpy(blob.data() + o_tc, tc.data(), tc.size() * sizeof(E));
-    memcpy(blob.data() + o_ti, ti.data(), ti.size() * sizeof(LogupTailInst));
-    if (upload_small(sc->ctx, d, blob.data(), bytes) != DPB_OK) {
-        device_free(sc->ctx, d);
-        return;
-    }
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(sc_round_logup<F, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        cudaFuncSetAttribute(sc_round_logup<F, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        attr_set = true;
-    }
-    sc->d_logup = d;
-    sc->logup_n = n_inst;
-    sc->logup_eq = eq_table;
-    memcpy(sc->logup_lambda, lambda, sizeof(E));
-    sc->logup_ok = true;
-    // the resident kernel: the most pairs that fit, with as few of them as need be left to one block
-    if ((size_t)sc->k * (sizeof(E) / 8) > (size_t)kTailMaxTables * 4 || n_inst > kLogupTailMaxInst) return;  // the mailbox
-    LogupTailPlan& lt = sc->lt;
-    lt.n_inst = n_inst;
-    lt.n_tabs = n_tabs;
-    lt.eq_table = eq_table;
-    lt.d_consts = (char*)d + o_tc;
-    lt.d_inst = (char*)d + o_ti;
-    uint64_t best = 0;
-    for (uint32_t alone = sc->gl ? kTailAloneGl : kTailAloneFr; alone >= 4; alone /= 2) {
-        LogupTailPlan p = lt;
-        p.alone = alone;
-        for (uint64_t pairs = 256 * kLogupTailBlocks; pairs > best; pairs /= 2) {
-            size_t smem;
-            if (!logup_tail_blocks(p, pairs, sizeof(E), &smem)) continue;
-            // every later round fits as well: fewer pairs, or one block once `alone` pairs are left
-            if (!logup_tail_blocks(p, alone, sizeof(E), &smem)) continue;
-            best = pairs;
-            lt.alone = alone;
-        }
-    }
-    if (!best) return;
-    uint32_t i = 0;
-    while (i < sc->n && (1ull << (sc->n - i - 1)) > best) i++;
-    lt.start = i;
-    lt.ok = true;
-}
-
-void sumcheck_hint_logup(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_inst, const void* lambda, uint32_t eq_table) {
-    if (!sc || sc->merged || !inst || !lambda || n_inst == 0 || n_inst > kLogupMaxInst || sc->logup_ok || getenv("DPB_NO_LOGUP_KERNEL")) return;
-    // usable only by a degree-3 sumcheck in split-eq form whose one eq table is the hint's and whose other tables are
-    // exactly the instances', in order
-    if (!sc->spliteq || sc->d != 3 || sc->eq_leads.size() != 1 || sc->eq_leads[0].table != eq_table ||
-        sc->eq_leads[0].first_active != 0 || sc->log2_ranks != 0)
-        return;
-    uint32_t next = 0;
-    for (uint32_t i = 0; i < n_inst; i++) {
-        const LogupHintInst& h = inst[i];
-        if (h.first != next) return;
-        if (h.kind == kLogupInner) next += 4;
-        else if ((h.kind == kLogupLookup || h.kind == kLogupTable) && (h.ncol == 1 || h.ncol == 2))
-            next += 2 * h.ncol + (h.kind == kLogupTable ? 2 : 0);
-        else return;
-    }
-    if (next != eq_table || next + 1 != sc->k) return;
-    if (sc->gl) hint_logup_impl<GlFam>(sc, inst, n_inst, lambda, eq_table);
-    else hint_logup_impl<FrFam>(sc, inst, n_inst, lambda, eq_table);
-}
-
-}  // namespace dpb
-
 extern "C" {
 
 int dpb_sumcheck_begin_partial(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k,
@@ -2191,8 +1747,6 @@ int dpb_sumcheck_finish(dpb_sc* sc, const void* last_challenge, void* out_final_
     if (sc->global_round != total) return fail(DPB_ESTATE, "only %u of %u rounds ran", sc->global_round, total);
     int rc;
     if (sc->log2_ranks > 0) rc = dpb_sumcheck_finish(sc->tail, last_challenge, out_final_evals);
-    else if (sc->lt_active) rc = sc->gl ? lt_finish<GlFam>(sc, last_challenge, out_final_evals)
-                                        : lt_finish<FrFam>(sc, last_challenge, out_final_evals);
     else if (sc->tail_active) rc = sc->gl ? tail_finish<GlFam>(sc, last_challenge, out_final_evals)
                                           : tail_finish<FrFam>(sc, last_challenge, out_final_evals);
     else rc = sc->gl ? run_finish<GlFam>(sc, last_challenge, out_final_evals)
@@ -2210,7 +1764,6 @@ void dpb_sumcheck_free(dpb_sc* sc) {
     if (sc->tail) dpb_sumcheck_free(sc->tail);
     for (auto* m : sc->tail_mles) dpb_mle_free(m);
     device_free(sc->ctx, sc->tail_dev);
-    device_free(sc->ctx, sc->d_logup);
     // the fold buffers and every descriptor array live in this one block
     if (sc->slab && sc->slab == sc->ctx->slab_cache) sc->ctx->slab_cache_busy = false;
     else device_free(sc->ctx, sc->slab);

@@ -57,6 +57,7 @@ inline uint32_t log2u(uint64_t x) {
     return l;
 }
 
+constexpr size_t kSlabCacheMax = (size_t)4 << 30;  // larger blocks (claim batching over a whole model) are not kept
 constexpr int kMaxAcc = 8;  // round-polynomial evaluations per launch (degree <= 7)
 
 // Opt-in host-side phase timers (dpb_trace_enable): wall time per named phase of the whole-protocol entry points,
@@ -230,17 +231,12 @@ struct LogupSpec {
 // outputs (dpb_logup_outputs, 4 elements each), and the call then waits for them.  out: n handles, all or none.
 int logup_build_batch(dpb_ctx* ctx, const LogupSpec* specs, uint32_t n, dpb_logup** out, void* host_outputs);
 
-// What the batched logup prover knows about a layer sumcheck it is about to run (host/logup.hpp): the instances in the
-// order of the sumcheck's tables, and the layer's constants.  sumcheck_hint_logup hands it to a sumcheck right after
-// dpb_sumcheck_begin; when the sumcheck runs in split-eq form with that single eq table, its large rounds then use
-// the layer's own formula (sc_round_logup) instead of the term list.  The hint must describe the polynomial the term
-// list describes; a hint the sumcheck cannot use is ignored.
+// What the batched logup prover knows about an instance in the layer it is about to prove (logup_layer.hpp).
 struct LogupHintInst {
     int kind;        // 0 inner layer (4 tables), 1 lookup input layer (2 * ncol tables), 2 table input layer (2 + 2 * ncol)
     uint32_t first;  // index of its first table
     uint32_t ncol;
     alignas(16) uint8_t alpha[32], constant[32], sep[32];  // challenge elements: alpha_j, and for input layers c and s
 };
-void sumcheck_hint_logup(dpb_sc* sc, const LogupHintInst* inst, uint32_t n_inst, const void* lambda, uint32_t eq_table);
 
 }  // namespace dpb

@@ -390,8 +390,6 @@ LogUpBatchProof<F> new_batch_multiple_sizes_prove(dpb_ctx* ctx, const std::vecto
         dpb::TracePhase t_expr("logup.layer_expressions");
         std::vector<dpb_mle*> mles;
         std::vector<dpb_mle*> eq_mles;
-        std::vector<X> group_exprs;
-        X claim_expr = X::ZERO();
         size_t layer_count = 0;
         uint16_t wit_off = 0;
         struct EqGuard {
@@ -399,74 +397,52 @@ LogUpBatchProof<F> new_batch_multiple_sizes_prove(dpb_ctx* ctx, const std::vecto
             ~EqGuard() { for (auto* m : v) dpb_mle_free(m); }
         } eq_guard{eq_mles};
         // Every layer but the last is an inner layer of every instance it touches (an instance reaches its input
-        // layer when one variable remains, all of them together).  Its expression is known in closed form,
-        //   alpha_j * (n_lo d_hi + n_hi d_lo + lambda d_lo d_hi) * eq        (circuit.rs:231-296),
-        // so the three product terms per instance and the claim are written down directly; only the last layer,
-        // whose expression depends on the instances' columns, goes through the expression builder.
+        // layer when one variable remains, all of them together).  An instance's share of the claim is
+        // alpha_j * (num + lambda den) at the folded evaluations of the layer above (circuit.rs:231-412).
         const bool inner = remaining != 1;
-        dp_crypto::VirtualPolynomials<F> vp;
         E current_claim = F::zero();
-        std::vector<uint32_t> term_group;  // per direct term: the size group whose eq table closes it
-        std::vector<dpb::LogupHintInst> hint;  // this rank's instances as the round kernel of a logup layer wants them
-        E alpha_pow = F::one();            // alpha^layer_count
+        std::vector<dpb::LogupHintInst> hint;  // this rank's instances as the layer's sumcheck takes them
+        struct Place {  // .. and where they stand, for the general sumcheck
+            LogUpCircuit<F>* circuit;
+            size_t layer_vars, layer_count;
+            uint16_t wit;
+            uint32_t group;
+            E alpha;
+        };
+        std::vector<Place> places;
+        E alpha_pow = F::one();  // alpha^layer_count
         for (size_t size : sizes) {
             if (size < remaining) continue;
             const E mult_e = F::from_u64(1ull << (total_layers - size));
-            const X mult = X::Constant(mult_e);
             const size_t layer_vars = size - remaining + 1;
-            X group = X::ZERO();
             for (auto& c : circuits) {
                 if (c->num_vars() != size) continue;
                 // the whole batch holds this instance once per rank, next to each other; only this rank's takes
                 // part in its sumcheck, all of them in the claim
                 for (size_t q = 0; q < G; q++) {
-                    if (inner) {
-                        const size_t b = layer_count * 4;
-                        if (b + 3 >= wit_evals.size()) throw Error(DPB_EINVAL, "Proving failed: evaluations of the layer above are short");
-                        const E &w0 = wit_evals[b], &w1 = wit_evals[b + 1], &w2 = wit_evals[b + 2], &w3 = wit_evals[b + 3];
-                        const E num = F::add(F::mul(rho, F::sub(w1, w0)), w0), den = F::add(F::mul(rho, F::sub(w3, w2)), w2);
-                        current_claim = F::add(current_claim, F::mul(mult_e, F::mul(alpha_pow, F::add(num, F::mul(lambda, den)))));
-                        if (q == g_rank) {
-                            auto lm = c->layer_mles(layer_vars);
-                            mles.insert(mles.end(), lm.begin(), lm.end());
-                            const E al = F::mul(alpha_pow, lambda);
-                            const uint16_t w = wit_off;
-                            auto term = [&](const E& coef, uint16_t x, uint16_t y) {
-                                if (F::is_zero(coef)) return;
-                                dpb_term t;
-                                memset(&t, 0, sizeof t);
-                                memcpy(t.coeff, &coef, sizeof(E));
-                                t.n_factors = 3;
-                                t.idx[0] = x;
-                                t.idx[1] = y;
-                                vp.terms.push_back(t);
-                                term_group.push_back((uint32_t)group_exprs.size());
-                            };
+                    const size_t b = layer_count * 4;
+                    if (b + 3 >= wit_evals.size()) throw Error(DPB_EINVAL, "Proving failed: evaluations of the layer above are short");
+                    const E &w0 = wit_evals[b], &w1 = wit_evals[b + 1], &w2 = wit_evals[b + 2], &w3 = wit_evals[b + 3];
+                    const E num = F::add(F::mul(rho, F::sub(w1, w0)), w0), den = F::add(F::mul(rho, F::sub(w3, w2)), w2);
+                    current_claim = F::add(current_claim, F::mul(mult_e, F::mul(alpha_pow, F::add(num, F::mul(lambda, den)))));
+                    if (q == g_rank) {
+                        auto lm = c->layer_mles(layer_vars);
+                        mles.insert(mles.end(), lm.begin(), lm.end());
+                        places.push_back({c.get(), layer_vars, layer_count, wit_off, (uint32_t)eq_mles.size(), alpha_pow});
+                        if (inner) {
                             dpb::LogupHintInst h;
                             memset(&h, 0, sizeof h);
                             h.kind = 0;
-                            h.first = w;
+                            h.first = wit_off;
                             memcpy(h.alpha, &alpha_pow, sizeof(E));
                             hint.push_back(h);
-                            term(alpha_pow, w, (uint16_t)(w + 3));       // n_lo d_hi
-                            term(alpha_pow, (uint16_t)(w + 1), (uint16_t)(w + 2));  // n_hi d_lo
-                            term(al, (uint16_t)(w + 2), (uint16_t)(w + 3));         // lambda d_lo d_hi
-                            wit_off = (uint16_t)(wit_off + 4);
+                        } else {
+                            hint.push_back(c->input_layer_hint(wit_off, alpha_pow));
                         }
-                        layer_count++;
-                        alpha_pow = F::mul(alpha_pow, alpha);
-                        continue;
+                        wit_off = (uint16_t)(wit_off + lm.size());
                     }
-                    auto le = c->layer_exprs(layer_vars, layer_count, wit_off);
-                    if (q == g_rank) hint.push_back(c->input_layer_hint(wit_off, alpha_pow));
-                    alpha_pow = F::mul(alpha_pow, alpha);
                     layer_count++;
-                    claim_expr = claim_expr + mult * le.claim;
-                    if (q != g_rank) continue;
-                    auto lm = c->layer_mles(layer_vars);
-                    mles.insert(mles.end(), lm.begin(), lm.end());
-                    wit_off = (uint16_t)(wit_off + le.num_witnesses);
-                    group = group + le.sumcheck;
+                    alpha_pow = F::mul(alpha_pow, alpha);
                 }
             }
             dpb_mle* eq = nullptr;
@@ -475,31 +451,51 @@ LogUpBatchProof<F> new_batch_multiple_sizes_prove(dpb_ctx* ctx, const std::vecto
                 check(dpb_eq_table(ctx, F::kChalDtype, point.data() + (point.size() - layer_vars), (uint32_t)layer_vars, &eq));
             }
             eq_mles.push_back(eq);
-            group_exprs.push_back(group);
         }
-        if (!inner) current_claim = claim_expr.evaluate(wit_evals, {alpha, lambda, rho});
         transcript.append_scalars(&current_claim, 1);
 
         std::vector<dpb_mle*> all(mles);
         all.insert(all.end(), eq_mles.begin(), eq_mles.end());
-        if (inner) {
-            if (vp.terms.empty()) throw Error(DPB_EINVAL, "virtual polynomial has no terms");
-            for (size_t t = 0; t < vp.terms.size(); t++) vp.terms[t].idx[2] = (uint16_t)(wit_off + term_group[t]);
-            vp.num_vars = (uint32_t)v;
-            vp.mles = all;
-            vp.max_degree = 3;
-        } else {
-            X full = X::ZERO();
-            for (size_t i = 0; i < group_exprs.size(); i++) full = full + group_exprs[i] * X::WitIn((uint16_t)(wit_off + i));
-            auto builder = dp_crypto::VirtualPolynomialsBuilder<F>::new_with_mles(1, (uint32_t)v, all);
-            dpb::TracePhase t_expand("logup.expand_terms");
-            vp = builder.to_virtual_polys({full}, {alpha, lambda});
-        }
         t_expr.stop();
+        std::pair<dp_crypto::IOPProof<F>, dp_crypto::IOPProverState<F>> res;
         // one size group: one eq table, right after the instances' tables
-        const bool hinted = group_exprs.size() == 1;
-        auto res = dp_crypto::IOPProverState<F>::prove(ctx, vp, transcript, partial ? 2 : 0, hinted ? &hint : nullptr, &lambda,
-                                                       (uint32_t)wit_off);
+        if (eq_mles.size() != 1 || !dp_crypto::IOPProverState<F>::prove_logup_layer(ctx, (uint32_t)v, all, hint, lambda, transcript, partial, &res)) {
+            dpb::TracePhase t_expand("logup.expand_terms");
+            dp_crypto::VirtualPolynomials<F> vp;
+            if (inner) {
+                // alpha_j * (n_lo d_hi + n_hi d_lo + lambda d_lo d_hi) * eq, written down directly (circuit.rs:231-296)
+                auto term = [&](const E& coef, uint16_t x, uint16_t y, uint32_t group) {
+                    if (F::is_zero(coef)) return;
+                    dpb_term t;
+                    memset(&t, 0, sizeof t);
+                    memcpy(t.coeff, &coef, sizeof(E));
+                    t.n_factors = 3;
+                    t.idx[0] = x;
+                    t.idx[1] = y;
+                    t.idx[2] = (uint16_t)(wit_off + group);
+                    vp.terms.push_back(t);
+                };
+                for (const auto& p : places) {
+                    term(p.alpha, p.wit, (uint16_t)(p.wit + 3), p.group);                        // n_lo d_hi
+                    term(p.alpha, (uint16_t)(p.wit + 1), (uint16_t)(p.wit + 2), p.group);        // n_hi d_lo
+                    term(F::mul(p.alpha, lambda), (uint16_t)(p.wit + 2), (uint16_t)(p.wit + 3), p.group);
+                }
+                if (vp.terms.empty()) throw Error(DPB_EINVAL, "virtual polynomial has no terms");
+                vp.num_vars = (uint32_t)v;
+                vp.mles = all;
+                vp.max_degree = 3;
+            } else {
+                std::vector<X> group_exprs(eq_mles.size(), X::ZERO());
+                for (const auto& p : places)
+                    group_exprs[p.group] = group_exprs[p.group] + p.circuit->layer_exprs(p.layer_vars, p.layer_count, p.wit).sumcheck;
+                X full = X::ZERO();
+                for (size_t i = 0; i < group_exprs.size(); i++) full = full + group_exprs[i] * X::WitIn((uint16_t)(wit_off + i));
+                auto builder = dp_crypto::VirtualPolynomialsBuilder<F>::new_with_mles(1, (uint32_t)v, all);
+                vp = builder.to_virtual_polys({full}, {alpha, lambda});
+            }
+            t_expand.stop();
+            res = dp_crypto::IOPProverState<F>::prove(ctx, vp, transcript, partial ? 2 : 0);
+        }
         point = res.second.collect_raw_challenges();
         const auto& finals = res.second.get_mle_flatten_final_evaluations();
         std::vector<E> evals(finals.begin(), finals.begin() + wit_off);

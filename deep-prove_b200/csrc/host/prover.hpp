@@ -20,6 +20,7 @@
 
 #include "../../../include/dpb.h"
 #include "../family.cuh"
+#include "../logup_layer.hpp"
 #include "transcript.hpp"
 
 namespace dp_crypto {
@@ -299,9 +300,7 @@ class IOPProverState {
     // Runs every round on the GPU behind `ctx`; the transcript is only touched here, on the host.
     template <class T>
     static std::pair<IOPProof<F>, IOPProverState> prove(dpb_ctx* ctx, const VirtualPolynomials<F>& vp,
-                                                        T& transcript, int sharded = 0,
-                                                        const std::vector<dpb::LogupHintInst>* logup_hint = nullptr,
-                                                        const E* logup_lambda = nullptr, uint32_t logup_eq = 0) {
+                                                        T& transcript, int sharded = 0) {
         if (vp.terms.empty()) throw Error(DPB_EINVAL, "virtual polynomial has no terms");
         IOPProverState st;
         IOPProof<F> proof;
@@ -311,9 +310,6 @@ class IOPProverState {
         // rank runs this same loop
         check((sharded == 2 ? dpb_sumcheck_begin_partial : sharded ? dpb_sumcheck_begin_sharded : dpb_sumcheck_begin)(
             ctx, vp.num_vars, vp.mles.data(), (uint32_t)vp.mles.size(), vp.terms.data(), (uint32_t)vp.terms.size(), &sc));
-        // the logup prover says what its layer looks like: the large rounds then run from the layer's formula
-        if (logup_hint && logup_lambda && !logup_hint->empty())
-            dpb::sumcheck_hint_logup(sc, logup_hint->data(), (uint32_t)logup_hint->size(), logup_lambda, logup_eq);
         t_begin.stop();
         dpb::TracePhase t_rounds("sumcheck.rounds");
         struct Guard {
@@ -339,6 +335,45 @@ class IOPProverState {
         st.final_evals_.resize(vp.mles.size());
         check(dpb_sumcheck_finish(sc, &r, st.final_evals_.data()));
         return {std::move(proof), std::move(st)};
+    }
+    // The same loop for a layer of the batched logup prover, from the layer's own formula (logup_layer.hpp) instead of a
+    // term list: the same messages and transcript.  false: the layer is not of that form, nothing has happened.
+    template <class T>
+    static bool prove_logup_layer(dpb_ctx* ctx, uint32_t num_vars, const std::vector<dpb_mle*>& mles,
+                                  const std::vector<dpb::LogupHintInst>& inst, const E& lambda, T& transcript, bool partial,
+                                  std::pair<IOPProof<F>, IOPProverState>* out) {
+        constexpr uint32_t d = 3;
+        dpb::TracePhase t_begin("sumcheck.begin");
+        dpb::LogupLayerSc* sc = nullptr;
+        check(dpb::logup_layer_begin(ctx, num_vars, mles.data(), (uint32_t)mles.size(), inst.data(), (uint32_t)inst.size(), &lambda,
+                                     partial, &sc));
+        if (!sc) return false;
+        struct Guard {
+            dpb::LogupLayerSc* s;
+            ~Guard() { dpb::logup_layer_free(s); }
+        } guard{sc};
+        t_begin.stop();
+        dpb::TracePhase t_rounds("sumcheck.rounds");
+        IOPProverState st;
+        IOPProof<F> proof;
+        const E header[2] = {F::from_u64(num_vars), F::from_u64(d)};
+        transcript.append_scalars(header, 2);
+        E r = F::zero();
+        for (uint32_t i = 0; i < num_vars; i++) {
+            IOPProverMessage<F> msg;
+            msg.evaluations.resize(d + 1);
+            check(dpb::logup_layer_round(sc, i == 0 ? nullptr : &r, msg.evaluations.data()));
+            transcript.append_scalars(msg.evaluations);
+            r = transcript.append_and_sample(kRoundLabel);
+            st.challenges_.push_back(r);
+            proof.proofs.push_back(std::move(msg));
+        }
+        t_rounds.stop();
+        dpb::TracePhase t_finish("sumcheck.finish");
+        st.final_evals_.resize(mles.size());
+        check(dpb::logup_layer_finish(sc, &r, st.final_evals_.data()));
+        *out = {std::move(proof), std::move(st)};
+        return true;
     }
     // challenge j is the value of variable j
     const std::vector<E>& collect_raw_challenges() const { return challenges_; }
