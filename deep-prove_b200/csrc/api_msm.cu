@@ -8,14 +8,14 @@
 //                     a histogram of the (window, bucket) keys
 //   2. msm_scan_*     exclusive prefix sums of the histogram: where every bucket's list starts
 //   3. msm_scatter    the point indices, grouped by bucket
-//   4. msm_buckets    one thread per bucket adds its points up (mixed Jacobian + affine additions); a bucket with
-//                     more than 96 points (small integers crowd a wide window's low buckets) goes to a list that
-//                     msm_heavy_plan / msm_heavy_chunks / msm_heavy_combine work off in chunks of 2048 points, one
-//                     block per chunk
-//   5. msm_reduce     per window sum_b b * B_b: a thread takes a run of 16 buckets (running sums from the top, plus
-//                     the run's offset times its total), a block adds its 256 runs up in shared memory
-//   6. host           the blocks' partial sums per window (a handful of points), the windows combined by c
-//                     doublings each, one inversion for the affine result.
+//   4. msm_segments   the index list is cut into equal runs, one per thread, whatever buckets they belong to; a bucket
+//                     that ends where it began in the same run is written at once, the pieces of one that spans runs
+//                     are added up inside the block; msm_join adds what spans blocks
+//   5. msm_reduce     per window sum_b b * B_b, as plain sums over the buckets whose number has a given bit set: four
+//                     buckets per thread, then a tree in shared memory (msm_reduce over 512 buckets, msm_reduce_blocks
+//                     over a window's blocks)
+//   6. host           the sixteen sums per window and the windows put together in one chain of doublings, one
+//                     inversion for the affine result.
 // Integer tables (DPB_FR_I32 / DPB_FR_I64) enter as magnitudes: a negative scalar adds the negated point, and only
 // the one to four windows their bits reach are ever touched: committing to quantised tensors and 16-bit lookup
 // columns costs a fraction of a commit to full-width scalars.
@@ -32,9 +32,6 @@ struct dpb_g1_bases {
 };
 
 namespace dpb {
-
-constexpr int kMsmRun = 16;         // buckets a reduction thread walks
-constexpr int kMsmReduceThreads = 256;
 
 struct MsmScalars {
     const void* ptr;
@@ -201,163 +198,260 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
-constexpr uint32_t kMsmHeavy = 96;  // a bucket with more points than this is summed by a whole block
+// Bucket sums.  The scatter leaves the point indices grouped by bucket, in the order of the buckets, so the list is cut
+// into equal runs, one per thread of a grid that fills the GPU once: every lane of a warp makes the same number of
+// additions whether the digits are uniform (16 points a bucket at 2^20 points), crowd a few buckets or are almost all
+// one value.  (With a thread per bucket a warp waits for its fullest bucket, 27 points where the mean is 16, and
+// buckets of more than 96 points need kernels of their own: six integer columns of
+// 2^20 committed together took 3944 us that way and take 2099 us with equal runs and the bit sums below.)  A run begins inside a bucket as a rule and ends inside
+// another: those two pieces meet their neighbours' in shared memory.
+//
+// Pieces of a span of runs (a thread's, later a part of the block's, at last the block's):
+//   L  the sum of the span's first points, of a bucket that began before the span and ends inside it
+//   R  the sum of its last points, of a bucket that begins inside the span and goes on after it
+//   W  (kept in L's place) the whole span belongs to one bucket that began before and goes on after
+// Two neighbouring spans meet in at most one addition: R or W of the left one with L or W of the right one.  R + L
+// completes a bucket; all those pairs are added at once, so that only buckets that span three runs or more go through
+// the levels of the tree.
+constexpr int kSegThreads = 128;
+constexpr int kSegBlocks = 4;            // resident blocks per SM at 128 registers
+constexpr uint32_t kSegMinRun = 2;       // an addition of the run and a level of the tree take about as long
+constexpr uint32_t kHasL = 1, kHasR = 2, kWhole = 4;
 
-__global__ void __launch_bounds__(kThreads)
-    msm_buckets(const G1Affine* __restrict__ bases, const uint32_t* __restrict__ offsets,
-                const uint32_t* __restrict__ counts, const uint32_t* __restrict__ items, uint64_t n_keys,
-                G1Jac* __restrict__ buckets, uint32_t* __restrict__ heavy_list, uint32_t* __restrict__ heavy_count) {
-    const uint64_t key = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (key >= n_keys) return;
-    const uint32_t lo = offsets[key], cnt = counts[key];
-    if (cnt > kMsmHeavy) {  // skewed digits (small integers in a wide window): left to msm_heavy_buckets
-        heavy_list[atomicAdd(heavy_count, 1u)] = (uint32_t)key;
-        return;
+struct MsmEdge {
+    G1Sum L, R;
+    uint32_t flags, key_r, pad[2];
+};
+
+// last key whose list starts at or before item j, at or after `from` (offsets[from] <= j)
+__device__ __forceinline__ uint32_t msm_key_of(const uint32_t* __restrict__ offsets, uint32_t n_keys, uint32_t from, uint32_t j) {
+    uint32_t lo = from, hi = n_keys;
+    for (uint32_t step = 1; lo + step < hi; step <<= 1) {  // the next key as a rule: look near first
+        if (offsets[lo + step] > j) {
+            hi = lo + step;
+            break;
+        }
+        lo += step;
     }
-    G1Jac acc = g1_infinity();
-    for (uint32_t j = 0; j < cnt; j++) {
-        const uint32_t it = items[lo + j];
-        G1Affine p = bases[it & 0x7fffffffu];
-        if (it & 0x80000000u) p = g1_affine_neg(p);
-        acc = g1_add_mixed(acc, p);
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (offsets[mid] <= j) lo = mid;
+        else hi = mid;
     }
-    buckets[key] = acc;
+    return lo;
 }
 
-// Heavy buckets are cut into chunks of kHeavyChunk points so that a bucket of a million points (16-bit values in a
-// 13-bit window leave seven such buckets in the second window) is work for the whole GPU instead of one block.
-// msm_heavy_plan: chunk_first[h] = number of chunks before heavy bucket h (one block; the list has at most
-// n * windows / kMsmHeavy entries).
-constexpr uint32_t kHeavyChunk = 2048;
-__global__ void __launch_bounds__(1024)
-    msm_heavy_plan(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ heavy_list,
-                   const uint32_t* __restrict__ heavy_count, uint32_t* __restrict__ chunk_first) {
-    __shared__ uint32_t part[1024];
-    const uint32_t n_heavy = *heavy_count;
-    const uint32_t per = (n_heavy + blockDim.x - 1) / blockDim.x;
-    const uint32_t lo = threadIdx.x * per < n_heavy ? threadIdx.x * per : n_heavy;
-    const uint32_t hi = lo + per < n_heavy ? lo + per : n_heavy;
-    uint32_t sum = 0;
-    for (uint32_t h = lo; h < hi; h++) sum += (counts[heavy_list[h]] + kHeavyChunk - 1) / kHeavyChunk;
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (uint32_t t = 0; t < blockDim.x; t++) {
-            const uint32_t v = part[t];
-            part[t] = run;
-            run += v;
-        }
-        chunk_first[n_heavy] = run;  // total
+// *to = *x + *y: one copy of the addition for every step of a tree, its operands in memory
+__device__ __noinline__ void msm_add(G1Sum* to, const G1Sum* x, const G1Sum* y) { *to = g1_add(*x, *y); }
+
+// Joins span `a` with the span `b` to its right; the result is span a.  The whole of a span lies in its L; r[a] is
+// where its R lies, key_r[a] the bucket R belongs to.
+struct MsmSpans {
+    uint32_t* flags;
+    uint32_t* key_r;
+    uint32_t* r;
+};
+template <class Left, class Right>
+__device__ __forceinline__ void msm_meet(const MsmSpans& sp, uint32_t a, uint32_t b, const Left& left, const Right& right,
+                                         G1Sum* __restrict__ buckets) {
+    const uint32_t fa = sp.flags[a], fb = sp.flags[b];
+    uint32_t f = (fa & kHasL) | (fb & kHasR);
+    if ((fa & (kHasR | kWhole)) && (fb & (kHasL | kWhole))) {
+        G1Sum* x = fa & kWhole ? left(a) : right(sp.r[a]);
+        G1Sum* to = (fa | fb) & kWhole ? x : &buckets[sp.key_r[a]];
+        msm_add(to, x, left(b));
+        if (fa & fb & kWhole) f = kWhole;
+        else if (fa & kWhole) f |= kHasL;
+        else if (fb & kWhole) f |= kHasR;
     }
-    __syncthreads();
-    uint32_t run = part[threadIdx.x];
-    for (uint32_t h = lo; h < hi; h++) {
-        chunk_first[h] = run;
-        run += (counts[heavy_list[h]] + kHeavyChunk - 1) / kHeavyChunk;
+    if (!(fb & kWhole)) {
+        sp.key_r[a] = sp.key_r[b];
+        sp.r[a] = sp.r[b];
     }
+    sp.flags[a] = f;
 }
 
-// one block per chunk (grid-stride): every thread adds a strided share of the chunk's points, then a tree in shared
-// memory; chunk_sums[g] = the chunk's sum
-__global__ void __launch_bounds__(kMsmReduceThreads)
-    msm_heavy_chunks(const G1Affine* __restrict__ bases, const uint32_t* __restrict__ offsets,
-                     const uint32_t* __restrict__ counts, const uint32_t* __restrict__ items,
-                     const uint32_t* __restrict__ heavy_list, const uint32_t* __restrict__ heavy_count,
-                     const uint32_t* __restrict__ chunk_first, G1Jac* __restrict__ chunk_sums) {
-    __shared__ G1Jac sh[kMsmReduceThreads];
-    const uint32_t n_heavy = *heavy_count;
-    const uint32_t total = chunk_first[n_heavy];
-    for (uint32_t g = blockIdx.x; g < total; g += gridDim.x) {
-        // the heavy bucket this chunk belongs to: last h with chunk_first[h] <= g
-        uint32_t lo_h = 0, hi_h = n_heavy;
-        while (hi_h - lo_h > 1) {
-            const uint32_t mid = (lo_h + hi_h) >> 1;
-            if (chunk_first[mid] <= g) lo_h = mid;
-            else hi_h = mid;
-        }
-        const uint32_t key = heavy_list[lo_h];
-        const uint32_t first = offsets[key] + (g - chunk_first[lo_h]) * kHeavyChunk;
-        const uint32_t end_all = offsets[key] + counts[key];
-        const uint32_t end = first + kHeavyChunk < end_all ? first + kHeavyChunk : end_all;
-        G1Jac acc = g1_infinity();
-        for (uint32_t j = first + threadIdx.x; j < end; j += blockDim.x) {
+// Bound by the multiplier: ten products per point (1216 multiply-adds), the points gathered from L2.
+__global__ void __launch_bounds__(kSegThreads, kSegBlocks)
+    msm_segments(const G1Affine* __restrict__ bases, const uint32_t* __restrict__ offsets,
+                 const uint32_t* __restrict__ counts, const uint32_t* __restrict__ items, uint32_t n_keys,
+                 G1Sum* __restrict__ buckets, MsmEdge* __restrict__ edges) {
+    __shared__ G1Sum L[kSegThreads], R[kSegThreads];
+    __shared__ uint32_t flags[kSegThreads], key_r[kSegThreads], r_at[kSegThreads];
+    const uint32_t total = offsets[n_keys - 1] + counts[n_keys - 1], t = threadIdx.x;
+    const uint32_t threads = gridDim.x * kSegThreads;
+    uint32_t run = (uint32_t)(((uint64_t)total + threads - 1) / threads);
+    if (run < kSegMinRun) run = kSegMinRun;
+    const uint64_t start64 = (uint64_t)(blockIdx.x * kSegThreads + t) * run;
+    const uint32_t start = start64 < total ? (uint32_t)start64 : total;
+    const uint32_t end = total - start < run ? total : start + run;
+    uint32_t f = 0, key = 0;
+    if (start < end) {
+        key = msm_key_of(offsets, n_keys, 0, start);
+        uint32_t key_end = offsets[key] + counts[key];
+        bool before = offsets[key] < start;  // the bucket at hand began before this run
+        G1Sum acc = g1_infinity();
+        for (uint32_t j = start; j < end; j++) {
+            if (j == key_end) {
+                if (before) {
+                    L[t] = acc;
+                    f |= kHasL;
+                } else {
+                    buckets[key] = acc;
+                }
+                key = msm_key_of(offsets, n_keys, key, j);
+                key_end = offsets[key] + counts[key];
+                before = false;
+                acc = g1_infinity();
+            }
             const uint32_t it = items[j];
             G1Affine p = bases[it & 0x7fffffffu];
             if (it & 0x80000000u) p = g1_affine_neg(p);
             acc = g1_add_mixed(acc, p);
         }
-        sh[threadIdx.x] = acc;
-        __syncthreads();
-        for (uint32_t s = kMsmReduceThreads / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) sh[threadIdx.x] = g1_add(sh[threadIdx.x], sh[threadIdx.x + s]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) chunk_sums[g] = sh[0];
-        __syncthreads();
-    }
-}
-
-// one block per heavy bucket (grid-stride): the sum of its chunks' sums
-__global__ void __launch_bounds__(kMsmReduceThreads)
-    msm_heavy_combine(const uint32_t* __restrict__ heavy_list, const uint32_t* __restrict__ heavy_count,
-                      const uint32_t* __restrict__ chunk_first, const G1Jac* __restrict__ chunk_sums,
-                      G1Jac* __restrict__ buckets) {
-    __shared__ G1Jac sh[kMsmReduceThreads];
-    const uint32_t n_heavy = *heavy_count;
-    for (uint32_t h = blockIdx.x; h < n_heavy; h += gridDim.x) {
-        const uint32_t first = chunk_first[h], end = chunk_first[h + 1];
-        if (end - first == 1) {  // the usual case: a bucket of a few hundred points
-            if (threadIdx.x == 0) buckets[heavy_list[h]] = chunk_sums[first];
-            continue;
-        }
-        G1Jac acc = g1_infinity();
-        for (uint32_t g = first + threadIdx.x; g < end; g += blockDim.x) acc = g1_add(acc, chunk_sums[g]);
-        sh[threadIdx.x] = acc;
-        __syncthreads();
-        for (uint32_t s = kMsmReduceThreads / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s) sh[threadIdx.x] = g1_add(sh[threadIdx.x], sh[threadIdx.x + s]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) buckets[heavy_list[h]] = sh[0];
-        __syncthreads();
-    }
-}
-
-// out[w * blocks_per_window + blk] = sum over the block's buckets b of b * B_b
-__global__ void __launch_bounds__(kMsmReduceThreads)
-    msm_reduce(const G1Jac* __restrict__ buckets, uint32_t c, uint32_t blocks_per_window, G1Jac* __restrict__ out) {
-    __shared__ G1Jac sh[kMsmReduceThreads];
-    const uint32_t w = blockIdx.x / blocks_per_window, blk = blockIdx.x % blocks_per_window;
-    const uint64_t n_b = 1ull << c;
-    const uint64_t run_id = (uint64_t)blk * kMsmReduceThreads + threadIdx.x;
-    const uint64_t b_lo = run_id * kMsmRun;  // first bucket of this thread's run
-    G1Jac total = g1_infinity();
-    if (b_lo < n_b) {
-        const uint64_t b_hi = b_lo + kMsmRun < n_b ? b_lo + kMsmRun : n_b;
-        const G1Jac* B = buckets + ((size_t)w << c);
-        G1Jac running = g1_infinity(), sum = g1_infinity();
-        for (uint64_t b = b_hi; b-- > b_lo;) {  // sum = sum_b (b - b_lo + 1) B_b
-            running = g1_add(running, B[b]);
-            sum = g1_add(sum, running);
-        }
-        // sum_b b B_b = sum + (b_lo - 1) * running; bucket 0 is empty, so for b_lo = 0 the term (-1) * running
-        // is cancelled by counting one copy less: walk it as sum - running
-        if (b_lo == 0) {
-            G1Jac neg = running;
-            neg.Y = fq_neg(neg.Y);
-            total = g1_add(sum, neg);
+        if (before) {
+            L[t] = acc;
+            f |= key_end > end ? kWhole : kHasL;
+        } else if (key_end > end) {
+            R[t] = acc;
+            f |= kHasR;
         } else {
-            total = g1_add(sum, g1_mul_small(running, (uint32_t)(b_lo - 1)));
+            buckets[key] = acc;
         }
     }
-    sh[threadIdx.x] = total;
+    flags[t] = f;
+    key_r[t] = key;
+    r_at[t] = t;
     __syncthreads();
-    for (uint32_t s = kMsmReduceThreads / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] = g1_add(sh[threadIdx.x], sh[threadIdx.x + s]);
+    // buckets of two runs, all at once
+    const bool pair = t + 1 < kSegThreads && (f & kHasR) && (flags[t + 1] & kHasL);
+    if (pair) msm_add(&buckets[key_r[t]], &R[t], &L[t + 1]);
+    __syncthreads();
+    if (pair) {
+        atomicAnd(&flags[t], ~kHasR);
+        atomicAnd(&flags[t + 1], ~kHasL);
+    }
+    __syncthreads();
+    const MsmSpans sp = {flags, key_r, r_at};
+    for (uint32_t s = 1; s < kSegThreads; s <<= 1) {
+        const uint32_t a = 2 * s * t;
+        if (a < kSegThreads)
+            msm_meet(sp, a, a + s, [&](uint32_t i) { return &L[i]; }, [&](uint32_t i) { return &R[i]; }, buckets);
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
+    MsmEdge& e = edges[blockIdx.x];
+    if (t == 0) {
+        e.flags = flags[0];
+        e.key_r = key_r[0];
+        if (flags[0] & (kHasL | kWhole)) e.L = L[0];
+    }
+    if (t == 32 && (flags[0] & kHasR)) e.R = R[r_at[0]];
+}
+
+// The pieces that span blocks of msm_segments (at most a few hundred blocks).  Block 0 takes the buckets that span
+// three blocks or more through the levels of the tree, the others the pairs, 128 each: the two sets are disjoint.
+constexpr int kJoinThreads = 512, kJoinStep = 128, kJoinMax = 2048;
+__global__ void __launch_bounds__(kJoinThreads)
+    msm_join(MsmEdge* __restrict__ edges, uint32_t n, G1Sum* __restrict__ buckets) {
+    __shared__ uint32_t flags[kJoinMax], key_r[kJoinMax], r_at[kJoinMax];
+    const uint32_t t = threadIdx.x;
+    if (blockIdx.x > 0) {
+        const uint32_t i = (blockIdx.x - 1) * kJoinStep + t;
+        if (t < kJoinStep && i + 1 < n && (edges[i].flags & kHasR) && (edges[i + 1].flags & kHasL))
+            msm_add(&buckets[edges[i].key_r], &edges[i].R, &edges[i + 1].L);
+        return;
+    }
+    bool left = false;
+    for (uint32_t i = t; i < n; i += kJoinThreads) {
+        uint32_t f = edges[i].flags;
+        if ((f & kHasR) && i + 1 < n && (edges[i + 1].flags & kHasL)) f &= ~kHasR;
+        if ((f & kHasL) && i > 0 && (edges[i - 1].flags & kHasR)) f &= ~kHasL;
+        flags[i] = f;
+        key_r[i] = edges[i].key_r;
+        r_at[i] = i;
+        left = left || f != 0;
+    }
+    if (!__syncthreads_or(left)) return;
+    const MsmSpans sp = {flags, key_r, r_at};
+    for (uint32_t s = 1; s < n; s <<= 1) {
+        for (uint32_t a = 2 * s * t; a + s < n; a += 2 * s * kJoinThreads)
+            msm_meet(sp, a, a + s, [&](uint32_t i) { return &edges[i].L; }, [&](uint32_t i) { return &edges[i].R; }, buckets);
+        __syncthreads();
+    }
+}
+
+// sum_b b B_b of a window as plain sums: over the buckets whose number has bit k set, for every k.  Pairs of spans of
+// 2^l elements join by adding their sums bit by bit; the right one's total is the new bit l.  In place: element 0 of
+// a span holds its total, element 2^k the sum over the elements with bit k set.  l + 1 additions per pair, two per
+// element over all levels (as many as a running sum takes), none waiting for another of its level.
+// sums of a block: 0: sum of (b mod 4) B_b; 1..7: of the B_b with bit 2..8 of b set; 8: of all
+constexpr int kReduceThreads = 128, kReduceLevels = 7, kReducePer = 4;
+constexpr uint32_t kReduceSpan = kReduceThreads * kReducePer, kBlockSums = kReduceLevels + 2;
+// sums of a window: 0..7 the blocks' added up; 8..14: of all B_b with bit 9..15 of b set
+constexpr uint32_t kWindowSums = 16;
+// which of them enters with weight 2^bit, or -1
+static int msm_sum_of_bit(uint32_t bit) { return bit == 0 ? 0 : bit == 1 ? -1 : (int)bit - 1; }
+
+__global__ void __launch_bounds__(kReduceThreads, 4)
+    msm_reduce(const G1Sum* __restrict__ buckets, const uint32_t* __restrict__ counts, uint32_t c, uint32_t blocks_per_window,
+               G1Sum* __restrict__ part) {
+    __shared__ G1Sum S[kReduceThreads], T[kReduceThreads];
+    const uint32_t w = blockIdx.x / blocks_per_window, blk = blockIdx.x % blocks_per_window, t = threadIdx.x;
+    const uint32_t first = blk * kReduceSpan + t * kReducePer;
+    S[t] = T[t] = g1_infinity();
+    bool any = false;
+#pragma unroll 1
+    for (int b = kReducePer - 1; b >= 0; b--) {  // S = sum of b B_b, T = sum of B_b
+        const size_t key = ((size_t)w << c) + first + b;
+        if (first + b < (1u << c) && counts[key]) {  // the bucket of digit 0 has no points
+            msm_add(&T[t], &T[t], &buckets[key]);
+            any = true;
+        }
+        if (b) msm_add(&S[t], &S[t], &T[t]);
+    }
+    if (__syncthreads_or(any)) {
+#pragma unroll 1
+        for (uint32_t l = 0; l < kReduceLevels; l++) {
+            const uint32_t s = 1u << l, pairs = kReduceThreads >> (l + 1);
+            if (t < pairs * (l + 2)) {
+                // the last `pairs` tasks are the plain sums S
+                const uint32_t pair = t < pairs * (l + 1) ? t / (l + 1) : t - pairs * (l + 1);
+                const uint32_t k = t < pairs * (l + 1) ? t % (l + 1) : 0;
+                G1Sum* x = (t < pairs * (l + 1) ? T : S) + (pair << (l + 1)) + (k ? 1u << (k - 1) : 0u);
+                msm_add(x, x, x + s);
+            }
+            __syncthreads();
+        }
+    }
+    if (t < kBlockSums) part[(size_t)blockIdx.x * kBlockSums + t] = t == 0 ? S[0] : t == kBlockSums - 1 ? T[0] : T[1u << (t - 1)];
+}
+
+// one block per window and sum: the sums 0..7 over the window's blocks, the blocks' totals by the bits of the block
+__global__ void __launch_bounds__(kReduceThreads, 4)
+    msm_reduce_blocks(const G1Sum* __restrict__ part, uint32_t blocks_per_window, G1Sum* __restrict__ sums) {
+    __shared__ G1Sum T[kReduceThreads];
+    const uint32_t w = blockIdx.x / kBlockSums, v = blockIdx.x % kBlockSums, t = threadIdx.x;
+    T[t] = t < blocks_per_window ? part[((size_t)w * blocks_per_window + t) * kBlockSums + v] : g1_infinity();
+    const bool bits = v == kBlockSums - 1;
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t l = 0; l < kReduceLevels && (1u << l) < blocks_per_window; l++) {
+        const uint32_t sums_per = bits ? l + 1 : 1;
+        if (t < (kReduceThreads >> (l + 1)) * sums_per) {
+            const uint32_t k = t % sums_per;
+            G1Sum* x = T + ((t / sums_per) << (l + 1)) + (k ? 1u << (k - 1) : 0u);
+            msm_add(x, x, x + (1u << l));
+        }
+        __syncthreads();
+    }
+    G1Sum* out = sums + (size_t)w * kWindowSums;
+    if (!bits) {
+        if (t == 0) out[v] = T[0];
+    } else if (t < kReduceLevels) {
+        out[kBlockSums - 1 + t] = (1u << t) < blocks_per_window ? T[1u << t] : g1_infinity();
+    } else if (t == kReduceLevels) {
+        out[kWindowSums - 1] = g1_infinity();
+    }
 }
 
 __global__ void __launch_bounds__(kThreads) msm_bases_to_mont(G1Affine* p, uint64_t n, unsigned int* bad) {
@@ -402,15 +496,14 @@ static uint32_t msm_window_bits(uint64_t n) {
 constexpr uint32_t kMsmGroup = 16;               // commitments of a batch in flight together
 constexpr size_t kMsmHostBytes = 1 << 20;         // pinned staging for their window sums
 
-// One commitment: its layout in one block of device memory [counts | offsets | cursor | heavy count | items |
-// heavy list | scan tiles | buckets | window sums | heavy chunk table | heavy chunk sums].
+// One commitment: its layout in one block of device memory [counts | offsets | cursor | items | scan tiles | buckets |
+// block edges | block sums | window sums].
 struct MsmJob {
     uint64_t n = 0;
-    uint32_t c = 0, windows = 0, blocks_per_window = 0, n_tiles = 0;
-    size_t n_keys = 0, n_partials = 0, host_off = 0;
-    uint64_t max_heavy = 0, max_chunks = 0;
-    size_t o_counts = 0, o_offsets = 0, o_cursor = 0, o_heavy_count = 0, o_items = 0, o_heavy = 0, o_tiles = 0, o_buckets = 0,
-           o_part = 0, o_chunk_first = 0, o_chunk_sums = 0;
+    uint32_t c = 0, windows = 0, blocks_per_window = 0, n_tiles = 0, segment_blocks = 0;
+    size_t n_keys = 0, n_sums = 0, host_off = 0;
+    size_t o_counts = 0, o_offsets = 0, o_cursor = 0, o_items = 0, o_tiles = 0, o_buckets = 0, o_edges = 0, o_part = 0,
+           o_sums = 0;
     void* slab = nullptr;
 };
 
@@ -425,9 +518,11 @@ static int msm_plan(dpb_ctx* ctx, const dpb_g1_bases* bases, const dpb_mle* scal
     const uint32_t scalar_bits = scalars->dtype == DPB_FR ? 254 : scalars->dtype == DPB_FR_I32 ? 32 : 64;
     job.windows = (scalar_bits + job.c - 1) / job.c;
     job.n_keys = (size_t)job.windows << job.c;
-    const uint32_t runs = (uint32_t)(((1ull << job.c) + kMsmRun - 1) / kMsmRun);
-    job.blocks_per_window = (runs + kMsmReduceThreads - 1) / kMsmReduceThreads;
-    job.n_partials = (size_t)job.windows * job.blocks_per_window;
+    job.blocks_per_window = (uint32_t)(((1ull << job.c) + kReduceSpan - 1) / kReduceSpan);
+    job.n_sums = (size_t)job.windows * kWindowSums;
+    job.segment_blocks = (uint32_t)ctx->sm_count * kSegBlocks;
+    const uint64_t most = ((uint64_t)n * job.windows + kSegThreads * kSegMinRun - 1) / (kSegThreads * kSegMinRun);
+    if (most < job.segment_blocks) job.segment_blocks = (uint32_t)most;
     job.n_tiles = (uint32_t)((job.n_keys + kScanTile - 1) / kScanTile);
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -438,70 +533,61 @@ static int msm_plan(dpb_ctx* ctx, const dpb_g1_bases* bases, const dpb_mle* scal
     job.o_counts = take(job.n_keys * 4);
     job.o_offsets = take(job.n_keys * 4);
     job.o_cursor = take(job.n_keys * 4);
-    job.o_heavy_count = take(256);
     job.o_items = take((size_t)n * job.windows * 4);
-    job.o_heavy = take(job.n_keys * 4);
     job.o_tiles = take((size_t)job.n_tiles * 4);
-    job.o_buckets = take(job.n_keys * sizeof(G1Jac));
-    job.o_part = take(job.n_partials * sizeof(G1Jac));
-    // heavy buckets: at most n * windows / kMsmHeavy of them, cut into at most that many + n * windows / kHeavyChunk chunks
-    job.max_heavy = (uint64_t)n * job.windows / kMsmHeavy + 1;
-    if (job.max_heavy > job.n_keys) job.max_heavy = job.n_keys;
-    job.max_chunks = job.max_heavy + (uint64_t)n * job.windows / kHeavyChunk + 1;
-    job.o_chunk_first = take((job.max_heavy + 1) * 4);
-    job.o_chunk_sums = take(job.max_chunks * sizeof(G1Jac));
+    job.o_buckets = take(job.n_keys * sizeof(G1Sum));
+    job.o_edges = take((size_t)job.segment_blocks * sizeof(MsmEdge));
+    job.o_part = take((size_t)job.windows * job.blocks_per_window * kBlockSums * sizeof(G1Sum));
+    job.o_sums = take(job.n_sums * sizeof(G1Sum));
     return device_alloc(ctx, off, &job.slab);
 }
 
 // every kernel of one commitment and the copy of its window sums to `h_part` (pinned), on stream `st`
 static cudaError_t msm_launch(dpb_ctx* ctx, const dpb_g1_bases* bases, const dpb_mle* scalars, const MsmJob& job,
-                              cudaStream_t st, G1Jac* h_part) {
+                              cudaStream_t st, G1Sum* h_sums) {
     char* base = (char*)job.slab;
     uint32_t* counts = (uint32_t*)(base + job.o_counts);
     uint32_t* offsets = (uint32_t*)(base + job.o_offsets);
     uint32_t* cursor = (uint32_t*)(base + job.o_cursor);
     uint32_t* items = (uint32_t*)(base + job.o_items);
-    uint32_t* heavy_list = (uint32_t*)(base + job.o_heavy);
-    uint32_t* heavy_count = (uint32_t*)(base + job.o_heavy_count);
     uint32_t* tile_sums = (uint32_t*)(base + job.o_tiles);
-    uint32_t* chunk_first = (uint32_t*)(base + job.o_chunk_first);
-    G1Jac* chunk_sums = (G1Jac*)(base + job.o_chunk_sums);
-    G1Jac* buckets = (G1Jac*)(base + job.o_buckets);
-    G1Jac* partials = (G1Jac*)(base + job.o_part);
+    G1Sum* buckets = (G1Sum*)(base + job.o_buckets);
+    MsmEdge* edges = (MsmEdge*)(base + job.o_edges);
+    G1Sum* part = (G1Sum*)(base + job.o_part);
+    G1Sum* sums = (G1Sum*)(base + job.o_sums);
     MsmScalars s;
     s.ptr = scalars->ptr;
     s.dtype = scalars->dtype;
     const uint64_t n = job.n;
     const uint32_t c = job.c, windows = job.windows;
     const size_t n_keys = job.n_keys;
-    cudaError_t e = cudaMemsetAsync(counts, 0, job.o_items - job.o_counts, st);  // counts, offsets, cursor, heavy count
+    cudaError_t e = cudaMemsetAsync(counts, 0, job.o_items - job.o_counts, st);  // counts, offsets, cursor
     if (e != cudaSuccess) return e;
     msm_count<<<grid_for(ctx, n), kThreads, 0, st>>>(s, n, c, windows, counts);
     msm_scan_tile_sums<<<job.n_tiles, kScanThreads, 0, st>>>(counts, n_keys, tile_sums);
     msm_scan_tiles<<<1, 1024, 0, st>>>(tile_sums, job.n_tiles);
     msm_scan_in_tiles<<<job.n_tiles, kScanThreads, 0, st>>>(counts, tile_sums, n_keys, offsets);
     msm_scatter<<<grid_for(ctx, n), kThreads, 0, st>>>(s, n, c, windows, offsets, cursor, items);
-    msm_buckets<<<(uint32_t)((n_keys + kThreads - 1) / kThreads), kThreads, 0, st>>>(
-        bases->dev, offsets, counts, items, n_keys, buckets, heavy_list, heavy_count);
-    const uint32_t cap = (uint32_t)ctx->sm_count * 16;  // idle blocks leave at once
-    msm_heavy_plan<<<1, 1024, 0, st>>>(counts, heavy_list, heavy_count, chunk_first);
-    msm_heavy_chunks<<<(uint32_t)(job.max_chunks < cap ? job.max_chunks : cap), kMsmReduceThreads, 0, st>>>(
-        bases->dev, offsets, counts, items, heavy_list, heavy_count, chunk_first, chunk_sums);
-    msm_heavy_combine<<<(uint32_t)(job.max_heavy < cap ? job.max_heavy : cap), kMsmReduceThreads, 0, st>>>(
-        heavy_list, heavy_count, chunk_first, chunk_sums, buckets);
-    msm_reduce<<<(uint32_t)job.n_partials, kMsmReduceThreads, 0, st>>>(buckets, c, job.blocks_per_window, partials);
+    msm_segments<<<job.segment_blocks, kSegThreads, 0, st>>>(bases->dev, offsets, counts, items, (uint32_t)n_keys, buckets,
+                                                             edges);
+    msm_join<<<1 + (job.segment_blocks + kJoinStep - 1) / kJoinStep, kJoinThreads, 0, st>>>(edges, job.segment_blocks, buckets);
+    msm_reduce<<<windows * job.blocks_per_window, kReduceThreads, 0, st>>>(buckets, counts, c, job.blocks_per_window, part);
+    msm_reduce_blocks<<<windows * kBlockSums, kReduceThreads, 0, st>>>(part, job.blocks_per_window, sums);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(h_part, partials, job.n_partials * sizeof(G1Jac), cudaMemcpyDeviceToHost, st);
+    return cudaMemcpyAsync(h_sums, sums, job.n_sums * sizeof(G1Sum), cudaMemcpyDeviceToHost, st);
 }
 
-// host: windows from the top, total = 2^c * total + window sum; one inversion for the affine result
-static void msm_finish(const MsmJob& job, const G1Jac* h_part, void* out_affine_xy) {
-    G1Jac total = g1_infinity();
+// host: bit by bit from the top, total = 2 total + the sums that enter at this bit of this window; one inversion for
+// the affine result
+static void msm_finish(const MsmJob& job, const G1Sum* h_sums, void* out_affine_xy) {
+    G1Sum total = g1_infinity();
     for (uint32_t w = job.windows; w-- > 0;) {
-        for (uint32_t d = 0; d < job.c; d++) total = g1_double(total);
-        for (uint32_t k = 0; k < job.blocks_per_window; k++)
-            total = g1_add(total, h_part[(size_t)w * job.blocks_per_window + k]);
+        for (uint32_t bit = job.c; bit-- > 0;) {
+            total = g1_double(total);
+            const int at = msm_sum_of_bit(bit);
+            if (at >= 0) total = g1_add(total, h_sums[(size_t)w * kWindowSums + at]);
+        }
     }
     const G1Affine a = g1_to_affine(total);
     Fq xy[2];
@@ -627,7 +713,7 @@ int dpb_pcs_batch_commit(dpb_ctx* ctx, const dpb_g1_bases* bases, dpb_mle* const
         for (uint32_t j = 0; j < cnt && rc == DPB_OK; j++) {
             rc = msm_plan(ctx, bases, polys[first + j], jobs[j]);
             jobs[j].host_off = host_off;
-            host_off += jobs[j].n_partials * sizeof(G1Jac);
+            host_off += jobs[j].n_sums * sizeof(G1Sum);
         }
         if (rc == DPB_OK && host_off > kMsmHostBytes) rc = fail(DPB_EINVAL, "commitment staging of %zu bytes", host_off);
         cudaError_t e = cudaSuccess;
@@ -642,7 +728,7 @@ int dpb_pcs_batch_commit(dpb_ctx* ctx, const dpb_g1_bases* bases, dpb_mle* const
             }
             for (uint32_t j = 0; j < cnt && e == cudaSuccess; j++) {
                 cudaStream_t st = side ? ctx->msm_stream[j % dpb_ctx::kMsmStreams] : ctx->stream;
-                e = msm_launch(ctx, bases, polys[first + j], jobs[j], st, (G1Jac*)((char*)ctx->msm_host + jobs[j].host_off));
+                e = msm_launch(ctx, bases, polys[first + j], jobs[j], st, (G1Sum*)((char*)ctx->msm_host + jobs[j].host_off));
             }
             if (side) {
                 // ... and this context's stream goes on after them (even when a launch failed: the slabs are freed below)
@@ -658,7 +744,7 @@ int dpb_pcs_batch_commit(dpb_ctx* ctx, const dpb_g1_bases* bases, dpb_mle* const
         if (rc != DPB_OK) return rc;
         if (e != cudaSuccess) return fail(DPB_ECUDA, "msm: %s", cudaGetErrorString(e));
         for (uint32_t j = 0; j < cnt; j++)
-            msm_finish(jobs[j], (const G1Jac*)((const char*)ctx->msm_host + jobs[j].host_off),
+            msm_finish(jobs[j], (const G1Sum*)((const char*)ctx->msm_host + jobs[j].host_off),
                        (char*)out_affine_xy + (size_t)(first + j) * 64);
     }
     return DPB_OK;

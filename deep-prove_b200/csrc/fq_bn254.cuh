@@ -181,6 +181,13 @@ DPB_HD Fq fq_mul(const Fq& a, const Fq& b) {
     return (t[4] || fq_geq_q(r)) ? fq_sub_q(r) : r;
 }
 DPB_HD Fq fq_sqr(const Fq& a) { return fq_mul(a, a); }
+// a b - c d
+DPB_HD Fq fq_mul_sub_mul(const Fq& a, const Fq& b, const Fq& c, const Fq& d) {
+#if defined(__CUDA_ARCH__)
+    return fq_from_words(fqw::mul_add_mul(fq_words(a), fq_words(b), fq_words(fq_neg(c)), fq_words(d)));
+#endif
+    return fq_sub(fq_mul(a, b), fq_mul(c, d));
+}
 DPB_HD Fq fq_to_mont(const Fq& a) { return fq_mul(a, fq_rr()); }
 DPB_HD Fq fq_from_mont(const Fq& a) {
     Fq one;

@@ -116,5 +116,45 @@ __device__ __forceinline__ F8 sub(const F8& a, const F8& b) {
     return d;
 }
 
+// the reduction half of mont_step
+template <int I>
+__device__ __forceinline__ void redc_step(uint32_t* P, uint32_t* Q) {
+    const uint32_t m = (I ? P[I] + Q[I] : P[I]) * DPB_FQW_INV;
+    frw::chain_mul(P + I, P[I + 8], DPB_FQW_Q0, DPB_FQW_Q2, DPB_FQW_Q4, DPB_FQW_Q6, m);
+    if (I) chain_q_odd_lead(Q + I + 1, Q[I + 9], m, Q[I]);
+    else frw::chain_mul(Q + I + 1, Q[I + 9], DPB_FQW_Q1, DPB_FQW_Q3, DPB_FQW_Q5, DPB_FQW_Q7, m);
+}
+
+// a b + c d over 2^256 mod q with one reduction: 192 multiply-adds instead of 256.  The sum of the two products is
+// below 2 q^2 < 2^509; the low eight words' reduction is at most q and the high eight words are below 0.38 q, so one
+// conditional subtraction of q finishes.
+__device__ __forceinline__ F8 mul_add_mul(const F8& a, const F8& b, const F8& c, const F8& d) {
+    frw::Wide s = frw::wide_zero();
+    frw::wide_mac(s, a, b);
+    frw::wide_mac(s, c, d);
+    uint32_t E[18], O[18];
+#pragma unroll
+    for (int i = 0; i < 18; i++) {
+        E[i] = i < 16 ? s.w[i] : 0;
+        O[i] = 0;
+    }
+    redc_step<0>(E, O);
+    redc_step<1>(O, E);
+    redc_step<2>(E, O);
+    redc_step<3>(O, E);
+    redc_step<4>(E, O);
+    redc_step<5>(O, E);
+    redc_step<6>(E, O);
+    redc_step<7>(O, E);
+    F8 v;
+    asm("add.cc.u32 %0, %8, %16; addc.cc.u32 %1, %9, %17; addc.cc.u32 %2, %10, %18; addc.cc.u32 %3, %11, %19;\n\t"
+        "addc.cc.u32 %4, %12, %20; addc.cc.u32 %5, %13, %21; addc.cc.u32 %6, %14, %22; addc.u32 %7, %15, %23;"
+        : "=&r"(v.w[0]), "=&r"(v.w[1]), "=&r"(v.w[2]), "=&r"(v.w[3]), "=&r"(v.w[4]), "=&r"(v.w[5]), "=&r"(v.w[6]),
+          "=&r"(v.w[7])
+        : "r"(E[8]), "r"(E[9]), "r"(E[10]), "r"(E[11]), "r"(E[12]), "r"(E[13]), "r"(E[14]), "r"(E[15]), "r"(O[8]),
+          "r"(O[9]), "r"(O[10]), "r"(O[11]), "r"(O[12]), "r"(O[13]), "r"(O[14]), "r"(O[15]));
+    return fqw::reduce_once(v);
+}
+
 }  // namespace fqw
 }  // namespace dpb
