@@ -536,6 +536,8 @@ void dpb_shutdown(dpb_ctx* ctx) {
         }
     for (int i = 0; i <= dpb_ctx::kMsmStreams; i++)
         if (ctx->msm_ev[i]) cudaEventDestroy(ctx->msm_ev[i]);
+    for (cudaEvent_t ev : ctx->msm_done)
+        if (ev) cudaEventDestroy(ev);
     if (ctx->msm_host) cudaFreeHost(ctx->msm_host);
     cudaStreamDestroy(ctx->tail_stream);
     cudaEventDestroy(ctx->tail_ev[0]);

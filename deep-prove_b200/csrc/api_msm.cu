@@ -202,9 +202,10 @@ __global__ void __launch_bounds__(kThreads)
 // into equal runs, one per thread of a grid that fills the GPU once: every lane of a warp makes the same number of
 // additions whether the digits are uniform (16 points a bucket at 2^20 points), crowd a few buckets or are almost all
 // one value.  (With a thread per bucket a warp waits for its fullest bucket, 27 points where the mean is 16, and
-// buckets of more than 96 points need kernels of their own: six integer columns of
-// 2^20 committed together took 3944 us that way and take 2099 us with equal runs and the bit sums below.)  A run begins inside a bucket as a rule and ends inside
-// another: those two pieces meet their neighbours' in shared memory.
+// buckets of more than 96 points need kernels of their own: six integer columns of 2^20 committed together took 3944 us
+// that way; equal runs and the bit sums below took 2099 us, four lanes per addition in the trees and the host's share
+// next to the kernels 1784 us.)  A run begins inside a bucket as a rule and ends inside another: those two pieces meet
+// their neighbours' in shared memory.
 //
 // Pieces of a span of runs (a thread's, later a part of the block's, at last the block's):
 //   L  the sum of the span's first points, of a bucket that began before the span and ends inside it
@@ -244,7 +245,57 @@ __device__ __forceinline__ uint32_t msm_key_of(const uint32_t* __restrict__ offs
 // *to = *x + *y: one copy of the addition for every step of a tree, its operands in memory
 __device__ __noinline__ void msm_add(G1Sum* to, const G1Sum* x, const G1Sum* y) { *to = g1_add(*x, *y); }
 
-// Joins span `a` with the span `b` to its right; the result is span a.  The whole of a span lies in its L; r[a] is
+// The same by four neighbouring lanes, for the levels of a tree that leave lanes idle: the fourteen products of the
+// addition in four steps of one product per lane (a warp alone on its scheduler issues a product in about 0.3 us
+// whatever the number of its lanes that take part).  All four lanes are called with the same pointers.
+__device__ __noinline__ void msm_add4(G1Sum* to, const G1Sum* x, const G1Sum* y) {
+    const uint32_t lane = threadIdx.x & 31, q = lane & 3;
+    const uint32_t quad = 0xfu << (lane & ~3u);
+    auto from = [&](const Fq& v, int src) {
+        Fq r;
+#pragma unroll
+        for (int i = 0; i < 4; i++) r.l[i] = __shfl_sync(quad, v.l[i], src, 4);
+        return r;
+    };
+    const bool x_inf = g1_is_infinity(*x), y_inf = g1_is_infinity(*y);
+    __syncwarp(quad);
+    if (x_inf || y_inf) {
+        const Fq* src = (const Fq*)(x_inf ? y : x);
+        ((Fq*)to)[q] = src[q];
+        return;
+    }
+    // 1: U1, U2, S1, S2 of lanes 0..3
+    const Fq* mine = (const Fq*)(q & 1 ? y : x);    // its X or Y
+    const Fq* other = (const Fq*)(q & 1 ? x : y);   // with this one's ZZ or ZZZ
+    const uint32_t h = q >> 1;
+    const Fq v1 = fq_mul(mine[h], other[2 + h]);
+    Fq d = from(v1, (int)(q ^ 1));
+    d = q & 1 ? fq_sub(v1, d) : fq_sub(d, v1);  // P in lanes 0 and 1, R in lanes 2 and 3
+    const unsigned zero = __ballot_sync(quad, fq_is_zero(d)) >> (lane & ~3u);
+    if (zero & 1) {  // the same point or opposite points
+        if (q == 0) *to = zero & 4 ? g1_double(*x) : g1_infinity();
+        __syncwarp(quad);
+        return;
+    }
+    // 2: PP, ZZ1 ZZ2, RR, ZZZ1 ZZZ2
+    const Fq v2 = fq_mul(q & 1 ? mine[2 + h] : d, q & 1 ? other[2 + h] : d);
+    // 3: P PP, ZZ1 ZZ2 PP, U1 PP
+    const Fq pp = from(v2, 0), u1 = from(v1, 0);
+    const Fq v3 = fq_mul(q == 0 ? d : q == 1 ? v2 : u1, pp);
+    // 4: S1 PPP, -, R (Q - X), ZZZ1 ZZZ2 PPP
+    const Fq ppp = from(v3, 0), s1 = from(v1, 2);
+    const Fq X = fq_sub(fq_sub(v2, ppp), fq_dbl(v3));  // lane 2: RR - PPP - 2 Q
+    const Fq v4 = fq_mul(q == 0 ? s1 : q == 2 ? d : v2, q == 2 ? fq_sub(v3, X) : ppp);
+    const Fq s1ppp = from(v4, 0);
+    if (q == 1) to->ZZ = v3;
+    if (q == 2) {
+        to->X = X;
+        to->Y = fq_sub(v4, s1ppp);
+    }
+    if (q == 3) to->ZZZ = v4;
+}
+
+// Joins span `a` with the span `b` to its right, by four lanes; the result is span a.  The whole of a span lies in its L; r[a] is
 // where its R lies, key_r[a] the bucket R belongs to.
 struct MsmSpans {
     uint32_t* flags;
@@ -259,11 +310,13 @@ __device__ __forceinline__ void msm_meet(const MsmSpans& sp, uint32_t a, uint32_
     if ((fa & (kHasR | kWhole)) && (fb & (kHasL | kWhole))) {
         G1Sum* x = fa & kWhole ? left(a) : right(sp.r[a]);
         G1Sum* to = (fa | fb) & kWhole ? x : &buckets[sp.key_r[a]];
-        msm_add(to, x, left(b));
+        msm_add4(to, x, left(b));
         if (fa & fb & kWhole) f = kWhole;
         else if (fa & kWhole) f |= kHasL;
         else if (fb & kWhole) f |= kHasR;
     }
+    __syncwarp(0xfu << (threadIdx.x & 28));  // all four have read
+    if (threadIdx.x & 3) return;
     if (!(fb & kWhole)) {
         sp.key_r[a] = sp.key_r[b];
         sp.r[a] = sp.r[b];
@@ -271,7 +324,8 @@ __device__ __forceinline__ void msm_meet(const MsmSpans& sp, uint32_t a, uint32_
     sp.flags[a] = f;
 }
 
-// Bound by the multiplier: ten products per point (1216 multiply-adds), the points gathered from L2.
+// Bound by the multiplier: ten products per point (1216 multiply-adds), the points gathered from L2.  2^20 points: 284 us
+// for 16-bit values and 266 us for 12-bit ones, where the multiply-adds alone take 147.
 __global__ void __launch_bounds__(kSegThreads, kSegBlocks)
     msm_segments(const G1Affine* __restrict__ bases, const uint32_t* __restrict__ offsets,
                  const uint32_t* __restrict__ counts, const uint32_t* __restrict__ items, uint32_t n_keys,
@@ -334,8 +388,7 @@ __global__ void __launch_bounds__(kSegThreads, kSegBlocks)
     __syncthreads();
     const MsmSpans sp = {flags, key_r, r_at};
     for (uint32_t s = 1; s < kSegThreads; s <<= 1) {
-        const uint32_t a = 2 * s * t;
-        if (a < kSegThreads)
+        for (uint32_t a = 2 * s * (t / 4); a < kSegThreads; a += 2 * s * (kSegThreads / 4))
             msm_meet(sp, a, a + s, [&](uint32_t i) { return &L[i]; }, [&](uint32_t i) { return &R[i]; }, buckets);
         __syncthreads();
     }
@@ -374,12 +427,14 @@ __global__ void __launch_bounds__(kJoinThreads)
     if (!__syncthreads_or(left)) return;
     const MsmSpans sp = {flags, key_r, r_at};
     for (uint32_t s = 1; s < n; s <<= 1) {
-        for (uint32_t a = 2 * s * t; a + s < n; a += 2 * s * kJoinThreads)
+        for (uint32_t a = 2 * s * (t / 4); a + s < n; a += 2 * s * (kJoinThreads / 4))
             msm_meet(sp, a, a + s, [&](uint32_t i) { return &edges[i].L; }, [&](uint32_t i) { return &edges[i].R; }, buckets);
         __syncthreads();
     }
 }
 
+// Bound by the latency of its dependent additions (a block of 512 buckets: five, then seven levels): 106 + 38 us for two
+// windows of 2^16 buckets where runs of 16 buckets with running sums took 440.
 // sum_b b B_b of a window as plain sums: over the buckets whose number has bit k set, for every k.  Pairs of spans of
 // 2^l elements join by adding their sums bit by bit; the right one's total is the new bit l.  In place: element 0 of
 // a span holds its total, element 2^k the sum over the elements with bit k set.  l + 1 additions per pair, two per
@@ -413,12 +468,12 @@ __global__ void __launch_bounds__(kReduceThreads, 4)
 #pragma unroll 1
         for (uint32_t l = 0; l < kReduceLevels; l++) {
             const uint32_t s = 1u << l, pairs = kReduceThreads >> (l + 1);
-            if (t < pairs * (l + 2)) {
-                // the last `pairs` tasks are the plain sums S
-                const uint32_t pair = t < pairs * (l + 1) ? t / (l + 1) : t - pairs * (l + 1);
-                const uint32_t k = t < pairs * (l + 1) ? t % (l + 1) : 0;
-                G1Sum* x = (t < pairs * (l + 1) ? T : S) + (pair << (l + 1)) + (k ? 1u << (k - 1) : 0u);
-                msm_add(x, x, x + s);
+            for (uint32_t a = t / 4; a < pairs * (l + 2); a += kReduceThreads / 4) {
+                // the last `pairs` additions are the plain sums S
+                const bool bits = a < pairs * (l + 1);
+                const uint32_t pair = bits ? a / (l + 1) : a - pairs * (l + 1), k = bits ? a % (l + 1) : 0;
+                G1Sum* x = (bits ? T : S) + (pair << (l + 1)) + (k ? 1u << (k - 1) : 0u);
+                msm_add4(x, x, x + s);
             }
             __syncthreads();
         }
@@ -437,10 +492,10 @@ __global__ void __launch_bounds__(kReduceThreads, 4)
 #pragma unroll 1
     for (uint32_t l = 0; l < kReduceLevels && (1u << l) < blocks_per_window; l++) {
         const uint32_t sums_per = bits ? l + 1 : 1;
-        if (t < (kReduceThreads >> (l + 1)) * sums_per) {
-            const uint32_t k = t % sums_per;
-            G1Sum* x = T + ((t / sums_per) << (l + 1)) + (k ? 1u << (k - 1) : 0u);
-            msm_add(x, x, x + (1u << l));
+        for (uint32_t a = t / 4; a < (kReduceThreads >> (l + 1)) * sums_per; a += kReduceThreads / 4) {
+            const uint32_t k = a % sums_per;
+            G1Sum* x = T + ((a / sums_per) << (l + 1)) + (k ? 1u << (k - 1) : 0u);
+            msm_add4(x, x, x + (1u << l));
         }
         __syncthreads();
     }
@@ -493,7 +548,7 @@ static uint32_t msm_window_bits(uint64_t n) {
     return 8;
 }
 
-constexpr uint32_t kMsmGroup = 16;               // commitments of a batch in flight together
+constexpr uint32_t kMsmGroup = dpb_ctx::kMsmGroup;
 constexpr size_t kMsmHostBytes = 1 << 20;         // pinned staging for their window sums
 
 // One commitment: its layout in one block of device memory [counts | offsets | cursor | items | scan tiles | buckets |
@@ -520,7 +575,7 @@ static int msm_plan(dpb_ctx* ctx, const dpb_g1_bases* bases, const dpb_mle* scal
     job.n_keys = (size_t)job.windows << job.c;
     job.blocks_per_window = (uint32_t)(((1ull << job.c) + kReduceSpan - 1) / kReduceSpan);
     job.n_sums = (size_t)job.windows * kWindowSums;
-    job.segment_blocks = (uint32_t)ctx->sm_count * kSegBlocks;
+    job.segment_blocks = std::min<uint32_t>((uint32_t)ctx->sm_count * kSegBlocks, kJoinMax);
     const uint64_t most = ((uint64_t)n * job.windows + kSegThreads * kSegMinRun - 1) / (kSegThreads * kSegMinRun);
     if (most < job.segment_blocks) job.segment_blocks = (uint32_t)most;
     job.n_tiles = (uint32_t)((job.n_keys + kScanTile - 1) / kScanTile);
@@ -580,7 +635,7 @@ static cudaError_t msm_launch(dpb_ctx* ctx, const dpb_g1_bases* bases, const dpb
 
 // host: bit by bit from the top, total = 2 total + the sums that enter at this bit of this window; one inversion for
 // the affine result
-static void msm_finish(const MsmJob& job, const G1Sum* h_sums, void* out_affine_xy) {
+static void msm_finish(const MsmJob& job, const G1Sum* h_sums, Fq* xy) {
     G1Sum total = g1_infinity();
     for (uint32_t w = job.windows; w-- > 0;) {
         for (uint32_t bit = job.c; bit-- > 0;) {
@@ -590,14 +645,18 @@ static void msm_finish(const MsmJob& job, const G1Sum* h_sums, void* out_affine_
         }
     }
     const G1Affine a = g1_to_affine(total);
-    Fq xy[2];
     if (g1_affine_is_infinity(a)) {
         xy[0] = xy[1] = fq_zero();
     } else {
         xy[0] = fq_from_mont(a.x);
         xy[1] = fq_from_mont(a.y);
     }
-    memcpy(out_affine_xy, xy, sizeof xy);
+}
+
+static int msm_done_events(dpb_ctx* ctx, uint32_t n) {
+    for (uint32_t j = 0; j < n; j++)
+        if (!ctx->msm_done[j]) DPB_CUDA(cudaEventCreateWithFlags(&ctx->msm_done[j], cudaEventDisableTiming));
+    return DPB_OK;
 }
 
 static int msm_side_streams(dpb_ctx* ctx) {
@@ -703,11 +762,13 @@ int dpb_pcs_batch_commit(dpb_ctx* ctx, const dpb_g1_bases* bases, dpb_mle* const
         if (polys[i]->ctx != ctx) return fail(DPB_EINVAL, "polynomial %u belongs to another context", i);
     }
     if (n_polys > 1) DPB_TRY(msm_side_streams(ctx));
+    DPB_TRY(msm_done_events(ctx, std::min<uint32_t>(kMsmGroup, n_polys)));
     // groups of commitments in flight together: their kernels are short chains of curve additions that leave most
     // of the GPU idle one at a time
     for (uint32_t first = 0; first < n_polys; first += kMsmGroup) {
         const uint32_t cnt = std::min<uint32_t>(kMsmGroup, n_polys - first);
         std::vector<MsmJob> jobs(cnt);
+        std::vector<Fq> xy(2 * (size_t)cnt);  // handed out when the whole group is done
         int rc = DPB_OK;
         size_t host_off = 0;
         for (uint32_t j = 0; j < cnt && rc == DPB_OK; j++) {
@@ -729,6 +790,7 @@ int dpb_pcs_batch_commit(dpb_ctx* ctx, const dpb_g1_bases* bases, dpb_mle* const
             for (uint32_t j = 0; j < cnt && e == cudaSuccess; j++) {
                 cudaStream_t st = side ? ctx->msm_stream[j % dpb_ctx::kMsmStreams] : ctx->stream;
                 e = msm_launch(ctx, bases, polys[first + j], jobs[j], st, (G1Sum*)((char*)ctx->msm_host + jobs[j].host_off));
+                if (e == cudaSuccess) e = cudaEventRecord(ctx->msm_done[j], st);
             }
             if (side) {
                 // ... and this context's stream goes on after them (even when a launch failed: the slabs are freed below)
@@ -737,15 +799,19 @@ int dpb_pcs_batch_commit(dpb_ctx* ctx, const dpb_g1_bases* bases, dpb_mle* const
                     cudaStreamWaitEvent(ctx->stream, ctx->msm_ev[q], 0);
                 }
             }
+            // the host's share of a commitment while the kernels of the next ones run
+            for (uint32_t j = 0; j < cnt && e == cudaSuccess; j++) {
+                e = cudaEventSynchronize(ctx->msm_done[j]);
+                if (e == cudaSuccess)
+                    msm_finish(jobs[j], (const G1Sum*)((const char*)ctx->msm_host + jobs[j].host_off), &xy[2 * j]);
+            }
             const cudaError_t es = cudaStreamSynchronize(ctx->stream);
             if (e == cudaSuccess) e = es;
         }
         for (auto& job : jobs) device_free(ctx, job.slab);
         if (rc != DPB_OK) return rc;
         if (e != cudaSuccess) return fail(DPB_ECUDA, "msm: %s", cudaGetErrorString(e));
-        for (uint32_t j = 0; j < cnt; j++)
-            msm_finish(jobs[j], (const G1Sum*)((const char*)ctx->msm_host + jobs[j].host_off),
-                       (char*)out_affine_xy + (size_t)(first + j) * 64);
+        memcpy((char*)out_affine_xy + (size_t)first * 64, xy.data(), (size_t)cnt * 64);
     }
     return DPB_OK;
 }

@@ -158,6 +158,8 @@ struct dpb_ctx {
     static constexpr int kMsmStreams = 4;
     cudaStream_t msm_stream[kMsmStreams] = {};
     cudaEvent_t msm_ev[kMsmStreams + 1] = {};
+    static constexpr int kMsmGroup = 16;  // commitments of a batch in flight together
+    cudaEvent_t msm_done[kMsmGroup] = {};
     void* msm_host = nullptr;  // pinned: the window sums of the commitments in flight
     // the block of device memory the last sumcheck used, kept for the next one (dpb_sumcheck_begin)
     void* slab_cache = nullptr;

@@ -187,7 +187,7 @@ class LogUpCircuit {
         return {alpha_j * (-d_hi - d_lo + lam * d_lo * d_hi), claim, (uint16_t)(2 * ncol)};
     }
 
-    // the input layer as sc_round_logup takes it (kinds 1 and 2 of dpb::LogupHintInst)
+    // the input layer as the layer kernels take it (kinds 1 and 2 of dpb::LogupHintInst)
     dpb::LogupHintInst input_layer_hint(uint16_t wit0, const E& alpha_j) const {
         dpb::LogupHintInst h;
         memset(&h, 0, sizeof h);
