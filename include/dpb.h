@@ -165,7 +165,7 @@ int dpb_trace_read(char* out, size_t cap, size_t* needed);
  * chain length per thread (1..2^20).  No reference counterpart. */
 int dpb_issue_rate_probe(dpb_ctx* ctx, int kind, uint32_t iters, double* ops_per_second, double* elapsed_ms);
 
-/* The last rounds of a sumcheck (a few hundred pairs or fewer) run in one
+/* The last rounds of a sumcheck (a few thousand pairs or fewer) run in one
  * resident kernel that exchanges round sums and challenges with the host
  * through mapped memory instead of one launch per round.  enable = 0 turns
  * that off (every round is a launch); wait_ms bounds how long the kernel
