@@ -125,8 +125,10 @@ __device__ __forceinline__ void redc_step(uint32_t* P, uint32_t* Q) {
     else frw::chain_mul(Q + I + 1, Q[I + 9], DPB_FQW_Q1, DPB_FQW_Q3, DPB_FQW_Q5, DPB_FQW_Q7, m);
 }
 
-// a b + c d over 2^256 mod q with one reduction: 192 multiply-adds instead of 256.  The sum of the two products is
-// below 2 q^2 < 2^509; the low eight words' reduction is at most q and the high eight words are below 0.38 q, so one
+// a b + c d over 2^256 mod q with one reduction: 192 multiply-adds instead of 256.  The low eight words alone take the
+// reduction: its steps end their carries in the word above the one they work on, which has room only while that word
+// counts carries; with the sum's own words there, one of 0xffffffff lost the carry.  The sum of the two products is
+// below 2 q^2, so its high eight words are below 0.38 q; the low eight words' reduction is at most q, and one
 // conditional subtraction of q finishes.
 __device__ __forceinline__ F8 mul_add_mul(const F8& a, const F8& b, const F8& c, const F8& d) {
     frw::Wide s = frw::wide_zero();
@@ -135,7 +137,7 @@ __device__ __forceinline__ F8 mul_add_mul(const F8& a, const F8& b, const F8& c,
     uint32_t E[18], O[18];
 #pragma unroll
     for (int i = 0; i < 18; i++) {
-        E[i] = i < 16 ? s.w[i] : 0;
+        E[i] = i < 8 ? s.w[i] : 0;
         O[i] = 0;
     }
     redc_step<0>(E, O);
@@ -148,11 +150,14 @@ __device__ __forceinline__ F8 mul_add_mul(const F8& a, const F8& b, const F8& c,
     redc_step<7>(O, E);
     F8 v;
     asm("add.cc.u32 %0, %8, %16; addc.cc.u32 %1, %9, %17; addc.cc.u32 %2, %10, %18; addc.cc.u32 %3, %11, %19;\n\t"
-        "addc.cc.u32 %4, %12, %20; addc.cc.u32 %5, %13, %21; addc.cc.u32 %6, %14, %22; addc.u32 %7, %15, %23;"
+        "addc.cc.u32 %4, %12, %20; addc.cc.u32 %5, %13, %21; addc.cc.u32 %6, %14, %22; addc.u32 %7, %15, %23;\n\t"
+        "add.cc.u32 %0, %0, %24; addc.cc.u32 %1, %1, %25; addc.cc.u32 %2, %2, %26; addc.cc.u32 %3, %3, %27;\n\t"
+        "addc.cc.u32 %4, %4, %28; addc.cc.u32 %5, %5, %29; addc.cc.u32 %6, %6, %30; addc.u32 %7, %7, %31;"
         : "=&r"(v.w[0]), "=&r"(v.w[1]), "=&r"(v.w[2]), "=&r"(v.w[3]), "=&r"(v.w[4]), "=&r"(v.w[5]), "=&r"(v.w[6]),
           "=&r"(v.w[7])
         : "r"(E[8]), "r"(E[9]), "r"(E[10]), "r"(E[11]), "r"(E[12]), "r"(E[13]), "r"(E[14]), "r"(E[15]), "r"(O[8]),
-          "r"(O[9]), "r"(O[10]), "r"(O[11]), "r"(O[12]), "r"(O[13]), "r"(O[14]), "r"(O[15]));
+          "r"(O[9]), "r"(O[10]), "r"(O[11]), "r"(O[12]), "r"(O[13]), "r"(O[14]), "r"(O[15]), "r"(s.w[8]), "r"(s.w[9]),
+          "r"(s.w[10]), "r"(s.w[11]), "r"(s.w[12]), "r"(s.w[13]), "r"(s.w[14]), "r"(s.w[15]));
     return fqw::reduce_once(v);
 }
 
