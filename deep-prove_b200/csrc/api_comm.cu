@@ -100,6 +100,21 @@ int xch_collect(dpb_ctx* ctx, unsigned int seq, size_t msg_bytes, void* out, dou
     return DPB_OK;
 }
 
+int comm_allgather_message(dpb_ctx* ctx, const void* msg, size_t msg_bytes) {
+    if (!ctx->xch_host) {
+        char* slot = (char*)ctx->gather_dev + (size_t)ctx->rank * msg_bytes;
+        DPB_CUDA(cudaMemcpyAsync(slot, msg, msg_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        return allgather_to_host(ctx, slot, msg_bytes);
+    }
+    ctx->xseq++;
+    volatile TailChunk* c = (volatile TailChunk*)((char*)ctx->xch_host + xch_slot_offset(ctx->rank, ctx->xseq));
+    const size_t words = msg_bytes / 8;
+    for (size_t w = 0; w < words; w++) c[w].data = ((const uint64_t*)msg)[w];
+    std::atomic_thread_fence(std::memory_order_release);
+    for (size_t w = 0; w < words; w++) c[w].seq = ctx->xseq;
+    return xch_collect(ctx, ctx->xseq, msg_bytes, ctx->gather_host, 60.0);
+}
+
 // FNV-1a over the host name and the boot id: equal on two ranks exactly when they share a host
 static uint64_t host_fingerprint() {
     char buf[512];

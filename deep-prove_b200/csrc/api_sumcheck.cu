@@ -99,7 +99,7 @@ struct dpb_sc {
     alignas(16) uint8_t prev_coeffs[5 * 32] = {0};  // previous round polynomial, low to high (fused rounds)
     // sharded sumchecks: the local part has n variables, the whole sumcheck n + log2_ranks
     uint32_t log2_ranks = 0;
-    bool partial = false;  // this rank holds some of the TERMS (whole tables): every round's sums are added over the ranks
+    bool partial = false;  // this rank holds some of the TERMS (whole tables): every round's messages are added over the ranks
     uint32_t global_round = 0;
     std::vector<dpb_term> terms_copy;
     dpb_sc* tail = nullptr;             // the last log2_ranks rounds, identical on every rank
@@ -941,9 +941,11 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
     E r = F::zero();
     if (i > 0) memcpy(&r, prev_challenge, sizeof(E));
 
-    // A sharded sumcheck publishes into this rank's slot of the exchange area (in-place all-gather).
+    // A sharded sumcheck publishes into this rank's slot of the exchange area (in-place all-gather).  A partial one runs
+    // its own terms' round here as a sumcheck of its own and exchanges the finished message below: which kernel a rank's
+    // terms take, and what that kernel samples, is that rank's affair.
     const size_t msg_bytes = (sc->d + 1) * sizeof(E);
-    const bool sharded = sc->log2_ranks > 0 || sc->partial;
+    const bool sharded = sc->log2_ranks > 0;
     const bool shared_xch = sharded && ctx->xch_host != nullptr;
     if (shared_xch) {
         // this rank's slot of the shared host segment: the kernel's last block writes the sums, then the sequence number
@@ -960,7 +962,7 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
     }
     if (sc->spliteq && i > 0) spliteq_advance<F>(sc, i, r);
     // the last rounds go to the resident kernel (one per context at a time; not while profiling per launch)
-    bool use_tail = sc->tail_active || (sc->has_prog && ctx->tail_enabled && !sharded && !ctx->profile && !sc->heavy &&
+    bool use_tail = sc->tail_active || (sc->has_prog && ctx->tail_enabled && !sharded && !sc->partial && !ctx->profile && !sc->heavy &&
                                         i >= sc->tail_start && ctx->tail_owner == nullptr);
     // Rounds too small to fill the GPU with one thread per pair run as a fold launch plus an evaluation spread over
     // (pair, slice of the term list) items: a thread's chain of dependent field products is what such a round
@@ -1085,6 +1087,16 @@ static int run_round(dpb_sc* sc, const void* prev_challenge, void* out_evals) {
         }
         memcpy(out_evals, raw, msg_bytes);
         memcpy(sc->prev_evals, raw, msg_bytes);
+    }
+    if (sc->partial) {
+        // evaluations at 0..=d of every rank's part: they add up whatever made them
+        DPB_TRY(comm_allgather_message(ctx, out_evals, msg_bytes));
+        E* total = (E*)out_evals;
+        const E* g = (const E*)ctx->gather_host;
+        for (uint32_t x = 0; x <= sc->d; x++) {
+            total[x] = g[x];
+            for (int q = 1; q < ctx->nranks; q++) total[x] = F::add(total[x], g[(size_t)q * (sc->d + 1) + x]);
+        }
     }
     if (profiled) {
         float ms = 0.f;

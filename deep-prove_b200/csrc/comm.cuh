@@ -27,6 +27,10 @@ inline size_t xch_bytes_for(int nranks) { return kXchHeader + (size_t)nranks * 2
 // Waits until every rank's slot of exchange `seq` is published, then copies the messages to out[rank][msg_bytes].
 int xch_collect(dpb_ctx* ctx, unsigned int seq, size_t msg_bytes, void* out, double seconds);
 
+// Every rank's message of `msg_bytes` (up to kMaxAcc elements, from host memory) into ctx->gather_host, rank after rank:
+// through the shared segment when there is one, else through NCCL.  Bounded wait.
+int comm_allgather_message(dpb_ctx* ctx, const void* msg, size_t msg_bytes);
+
 NcclApi& nccl_api();
 int nccl_load();
 int sync_bounded(dpb_ctx* ctx, double seconds);

@@ -293,9 +293,10 @@ int dpb_sumcheck_begin_sharded(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* 
                                const dpb_term* terms, uint32_t n_terms, dpb_sc** out);
 /* A sumcheck whose TERMS are spread over the ranks of the context's communicator (the instances of a batch, the
  * heads of a stacked product): every rank passes whole tables and its own part of the term list, of the same
- * degree on every rank; each round's sums are added over the ranks (same exchange as the sharded form), all ranks
- * feed the same transcript, and dpb_sumcheck_finish returns the final evaluations of THIS rank's tables.  The
- * messages equal those of one sumcheck over the union of the term lists.  With one rank: dpb_sumcheck_begin. */
+ * degree on every rank but otherwise of any form; each rank makes the message of its own part, the messages are added
+ * over the ranks (same exchange as the sharded form), all ranks feed the same transcript, and dpb_sumcheck_finish
+ * returns the final evaluations of THIS rank's tables.  The messages equal those of one sumcheck over the union of
+ * the term lists.  With one rank: dpb_sumcheck_begin. */
 int dpb_sumcheck_begin_partial(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, uint32_t k,
                                const dpb_term* terms, uint32_t n_terms, dpb_sc** out);
 /* Degree of the round polynomial (max factors per term). */
