@@ -1353,6 +1353,13 @@ static int begin_merged(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, u
     return DPB_OK;
 }
 
+// the fold buffers and every descriptor array live in this one block
+static void release_slab(dpb_sc* sc) {
+    if (sc->slab && sc->slab == sc->ctx->slab_cache) sc->ctx->slab_cache_busy = false;
+    else device_free(sc->ctx, sc->slab);
+    sc->slab = nullptr;
+}
+
 // The last challenge of a merged sumcheck: the inner one's evaluations, and the merged tables' at the point (eq tables
 // from their coordinates, the others in one pass over all of them).
 template <class F>
@@ -1360,6 +1367,10 @@ static int merged_finish(dpb_sc* sc, const void* last_challenge, void* out) {
     typedef typename F::E E;
     std::vector<E> inner(sc->merged->k);
     DPB_TRY(dpb_sumcheck_finish(sc->merged, last_challenge, inner.data()));
+    // the rounds' memory makes room for the eq table of the evaluation below
+    release_slab(sc->merged);
+    for (auto* m : sc->merged_owned) dpb_mle_free(m);
+    sc->merged_owned.clear();
     sc->merged_point.insert(sc->merged_point.end(), (const uint8_t*)last_challenge, (const uint8_t*)last_challenge + sizeof(E));
     const E* point = (const E*)sc->merged_point.data();
     std::vector<E> values(sc->merged_members.size());
@@ -1382,7 +1393,10 @@ static int merged_finish(dpb_sc* sc, const void* last_challenge, void* out) {
     }
     if (!list.empty()) {
         std::vector<E> got(list.size());
-        DPB_TRY(dpb_mle_evaluate_many(sc->ctx, list.data(), (uint32_t)list.size(), point, sc->n, got.data()));
+        int rc = dpb_mle_evaluate_many(sc->ctx, list.data(), (uint32_t)list.size(), point, sc->n, got.data());
+        if (rc == DPB_ENOMEM && dpb_trim(sc->ctx) == DPB_OK)  // the slab above may be kept for the next sumcheck
+            rc = dpb_mle_evaluate_many(sc->ctx, list.data(), (uint32_t)list.size(), point, sc->n, got.data());
+        DPB_TRY(rc);
         for (size_t q = 0; q < list.size(); q++) values[place[q]] = got[q];
     }
     size_t next = 0;
@@ -1672,7 +1686,11 @@ int dpb_sumcheck_begin(dpb_ctx* ctx, uint32_t num_vars, dpb_mle* const* mles, ui
     if (ctx && mles && terms && out) {
         std::vector<int> position;
         const auto groups = plan_merge(num_vars, ctx, mles, k, terms, n_terms, position);
-        if (!groups.empty()) return begin_merged(ctx, num_vars, mles, k, terms, n_terms, groups, position, out);
+        if (!groups.empty()) {
+            const int rc = begin_merged(ctx, num_vars, mles, k, terms, n_terms, groups, position, out);
+            if (rc != DPB_ENOMEM || dpb_trim(ctx) != DPB_OK) return rc;
+            // two tables: their combination takes more than the fold buffers it saves, and those may still fit
+        }
     }
     return begin_general(ctx, num_vars, mles, k, terms, n_terms, out);
 }
@@ -1776,9 +1794,7 @@ void dpb_sumcheck_free(dpb_sc* sc) {
     if (sc->tail) dpb_sumcheck_free(sc->tail);
     for (auto* m : sc->tail_mles) dpb_mle_free(m);
     device_free(sc->ctx, sc->tail_dev);
-    // the fold buffers and every descriptor array live in this one block
-    if (sc->slab && sc->slab == sc->ctx->slab_cache) sc->ctx->slab_cache_busy = false;
-    else device_free(sc->ctx, sc->slab);
+    release_slab(sc);
     delete sc;
 }
 
