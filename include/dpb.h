@@ -274,7 +274,10 @@ int dpb_einsum_fix_axes(dpb_ctx* ctx, int family_dtype, const int64_t* tensor, i
 
 /* ---- sumcheck (dp_crypto::structs::IOPProverState) --------------------- */
 /* Starts a sumcheck over `num_vars` variables of  sum_t coeff_t * prod_j mle[idx_tj].
- * Tables are borrowed and never modified.  A table with fewer than num_vars
+ * Tables are borrowed and never modified.  Their memory must stay as it is until
+ * dpb_sumcheck_finish has returned (or, for a sumcheck that is dropped, until
+ * dpb_sumcheck_free has): a round, and the final evaluations, may read any of
+ * them again.  A table with fewer than num_vars
  * variables is a function of the LAST variables only (constant in the early
  * rounds), the convention the batched logup prover relies on
  * (zkml/src/lookup/logup_gkr/prover.rs:217-249).
