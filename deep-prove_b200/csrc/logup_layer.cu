@@ -411,7 +411,9 @@ static int round_impl(LogupLayerSc* sc, const void* prev_challenge, void* out_ev
         S = F::mul(S, F::add(F::mul(q, r), F::mul(F::sub(one, q), F::sub(one, r))));
         memcpy(sc->S, &S, sizeof(E));
     }
-    bool tail = sc->tail_active || (ctx->tail_enabled && !sc->partial && !ctx->profile && i >= sc->tail_start && ctx->tail_owner == nullptr);
+    // with `extra` the kernel binds the second columns too, from the originals: rounds 0 and 1 only
+    const bool can_start = i >= sc->tail_start && !(sc->extra && i > 1);
+    bool tail = sc->tail_active || (ctx->tail_enabled && !sc->partial && !ctx->profile && can_start && ctx->tail_owner == nullptr);
     const bool first = tail && !sc->tail_active;
     // the samples go to the host's chunk area, this rank's slot of the shared segment, or a collective
     const size_t msg_bytes = 3 * sizeof(E);
