@@ -591,6 +591,16 @@ int dpb_resident_rounds(dpb_ctx* ctx, int enable, uint32_t wait_ms) {
     return DPB_OK;
 }
 
+// Tests: the host sleeps for hold_ms before it posts the challenge of that number (the first one from now on is 0; ~0: none)
+// to a resident kernel.  Returns how many were posted since the call before.
+uint64_t dpb_resident_hold(dpb_ctx* ctx, uint64_t post, uint32_t hold_ms) {
+    const uint64_t posted = ctx->tail_posts;
+    ctx->tail_posts = 0;
+    ctx->tail_hold_post = post;
+    ctx->tail_hold_ms = hold_ms;
+    return posted;
+}
+
 int dpb_profile_enable(dpb_ctx* ctx, int on) {
     if (!ctx) return fail(DPB_EINVAL, "null context");
     if (on) ctx->prof_log.clear();

@@ -739,7 +739,7 @@ static int tail_round(dpb_sc* sc, uint32_t i, const typename F::E& r, typename F
         sc->tail_active = true;
         ctx->tail_owner = sc;
     } else {
-        tail_post<E>(box, &r, i);
+        tail_post<E>(ctx, &r, i);
     }
     const uint32_t want = i + 1;
     for (int attempt = 0;; attempt++) {
@@ -784,7 +784,7 @@ static int tail_finish(dpb_sc* sc, const void* last_challenge, void* out) {
     typedef typename F::E E;
     dpb_ctx* ctx = sc->ctx;
     TailBox* box = (TailBox*)ctx->tail_box_host;
-    tail_post<E>(box, last_challenge, sc->n);
+    tail_post<E>(ctx, last_challenge, sc->n);
     uint32_t j = 0;
     int rc = tail_wait_host(ctx, box, [&] {
         while (j < sc->k) {

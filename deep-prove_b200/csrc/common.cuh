@@ -168,6 +168,9 @@ struct dpb_ctx {
     bool tail_enabled = true;
     uint64_t sumcheck_launches = 0;  // kernels launched by the sumcheck entry points
     unsigned long long tail_wait_ns = 1ull * 1000 * 1000 * 1000;
+    // tests: challenges posted to a resident kernel so far, and the one that is held back (dpb_resident_hold)
+    uint64_t tail_posts = 0, tail_hold_post = ~0ull;
+    uint32_t tail_hold_ms = 0;
     // optional per-kernel timing log (dpb_profile_enable)
     bool profile = false;
     cudaEvent_t prof_ev[2] = {nullptr, nullptr};

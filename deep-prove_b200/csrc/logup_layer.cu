@@ -353,7 +353,7 @@ static int replay(LogupLayerSc* sc, uint32_t upto) {
         const int rc = take_samples<F>(sc, j, raw);
         if (rc != DPB_OK) return rc < 0 ? rc : fail(DPB_ETIMEOUT, "the resident round kernel gave up waiting for a challenge");
         const E ch = get<F>(sc->point.data(), j);
-        tail_post<E>((TailBox*)ctx->tail_box_host, &ch, j + 1);
+        tail_post<E>(ctx, &ch, j + 1);
     }
     return DPB_OK;
 }
@@ -444,7 +444,7 @@ static int round_impl(LogupLayerSc* sc, const void* prev_challenge, void* out_ev
         sc->tail_active = true;
         ctx->tail_owner = sc;
     } else if (tail) {
-        tail_post<E>((TailBox*)ctx->tail_box_host, &r, i);
+        tail_post<E>(ctx, &r, i);
     } else {
         DPB_TRY(launch());
     }
@@ -521,7 +521,7 @@ static int finish_impl(LogupLayerSc* sc, const void* last_challenge, void* out_r
     bool columns = false;  // the input columns' values are still missing
     if (sc->tail_active) {
         TailBox* box = (TailBox*)ctx->tail_box_host;
-        tail_post<E>(box, &r, sc->n);
+        tail_post<E>(ctx, &r, sc->n);
         std::vector<uint32_t> want;  // the tables the kernel reports
         for (const auto& h : sc->inst) {
             const uint32_t n = h.kind == kLogupInner ? 4 : (h.kind == kLogupTable ? 2 : 0) + (sc->extra ? 2 * h.ncol : 0);

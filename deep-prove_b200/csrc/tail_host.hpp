@@ -2,6 +2,7 @@
 #pragma once
 #include <atomic>
 #include <chrono>
+#include <thread>
 
 #include "common.cuh"
 #include "generic_round.cuh"
@@ -43,7 +44,10 @@ static int tail_wait_host(dpb_ctx* ctx, TailBox* box, Ready ready) {
 
 // the challenge as chunks: data first, then the sequence numbers
 template <class E>
-static void tail_post(TailBox* box, const void* chal, uint32_t seq) {
+static void tail_post(dpb_ctx* ctx, const void* chal, uint32_t seq) {
+    TailBox* box = (TailBox*)ctx->tail_box_host;
+    if (ctx->tail_posts++ == ctx->tail_hold_post)
+        std::this_thread::sleep_for(std::chrono::milliseconds(ctx->tail_hold_ms));  // dpb_resident_hold
     const uint64_t* w = (const uint64_t*)chal;
     constexpr int W8 = sizeof(E) / 8;
     for (int i = 0; i < W8; i++) ((volatile TailChunk*)box->chal)[i].data = w[i];

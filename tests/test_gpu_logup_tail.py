@@ -1,9 +1,8 @@
 """The last rounds of a logup layer in their own resident kernel (one block, or a cluster of blocks that hands over to
 one): proof bytes equal the oracle's at sizes around every switch, for all kinds of input layer, and stay the same
-when the host is held up past the kernel's wait, so that the kernel is started again and its rounds played once more."""
-import os
-import subprocess
-import sys
+when the host is held up past the kernel's wait at any of its challenges, so that the kernel is started again and its
+rounds played once more."""
+import ctypes
 
 import numpy as np
 import pytest
@@ -72,38 +71,32 @@ def test_proofs_around_the_switches(dpb, ctx, F, name, m):
         h.free()
 
 
-STOPPER = """
-import os, signal, sys, time
-pid, end = int(sys.argv[1]), time.time() + 3
-while time.time() < end:
-    time.sleep(0.013)
-    os.kill(pid, signal.SIGSTOP)
-    time.sleep(0.02)
-    os.kill(pid, signal.SIGCONT)
-"""
-
-
 @pytest.mark.parametrize("F", FIELDS)
-def test_host_held_up(dpb, F):
-    """A neighbour stops this process for 20 ms every now and then; the kernel waits 3 ms for a challenge."""
+@pytest.mark.parametrize("name,m,ints", [("three", 12, True), ("nine", 9, False), ("tables", 10, True)])
+def test_host_held_up(dpb, F, name, m, ints):
+    """The kernel waits 5 ms for a challenge; the host holds one back for 20 ms: every challenge of the proof in turn, so
+    that kernels are started again at each of their rounds (one block, a cluster, the hand-over) and at their end."""
+    hold = dpb.lib.dpb_resident_hold  # not part of the interface
+    hold.restype, hold.argtypes = ctypes.c_uint64, [ctypes.c_void_p, ctypes.c_uint64, ctypes.c_uint32]
+    none = 2**64 - 1
     ctx = dpb.Context(0)
-    rng = np.random.default_rng(9790)
-    lib_in, orc_in, handles = build(dpb, ctx, F, rng, LOOKUPS["three"], 12, ints=True)
+    rng = np.random.default_rng(9790 + m)
+    lib_in, orc_in, handles = build(dpb, ctx, F, rng, {**LOOKUPS, **TABLES}[name], m, ints=ints)
     fam = family_dtype(dpb, F)
     want = orc.serialize_logup_proof(F, orc.logup_batch_prove(F, orc_in, orc.Transcript(F)))
-    prove(ctx, F, fam, lib_in)
-    ctx.resident_rounds(True, 3)
+    hold(ctx.h, none, 0)
     before = ctx.sumcheck_launches()
     assert prove(ctx, F, fam, lib_in) == want
     undisturbed = ctx.sumcheck_launches() - before
-    stopper = subprocess.Popen([sys.executable, "-c", STOPPER, str(os.getpid())])
-    restarted = 0
-    while stopper.poll() is None:  # it ends by itself: never killed between a stop and its continue
+    ctx.resident_rounds(True, 5)
+    posts = hold(ctx.h, none, 0)
+    assert posts > m
+    for post in range(posts):
+        hold(ctx.h, post, 20)
         before = ctx.sumcheck_launches()
-        assert prove(ctx, F, fam, lib_in) == want
-        restarted += ctx.sumcheck_launches() - before > undisturbed
-    stopper.wait()
-    assert restarted > 0  # some stop fell into a resident round
+        assert prove(ctx, F, fam, lib_in) == want, f"challenge {post} of {posts}"
+        # the last one ends the input layer, whose kernel may have nothing left to report
+        assert ctx.sumcheck_launches() - before > undisturbed or post == posts - 1, f"challenge {post} of {posts}"
     for h in handles:
         h.free()
     ctx.close()
