@@ -111,12 +111,6 @@ class LogUpCircuit {
     size_t num_vars() const { return m_ - 1; }
     size_t denominator_column_count() const { return cols_.size(); }
     size_t final_eval_count() const { return 2 * cols_.size() + (kind_ == ProofType::Table ? 2 : 0); }
-    std::vector<E> outputs() const {
-        std::vector<E> o(4);
-        check(dpb_logup_outputs(tree_, o.data()));
-        return o;
-    }
-    const dpb_logup* tree() const { return tree_; }
 
     // Tables of the layer whose halves have `layer_vars` variables, in the
     // order layer_proving_info registers them.  Views stay alive with *this.

@@ -139,7 +139,7 @@ struct LgColumns<FrFam, MODE> {
 
 // Entry e of a slot in the round's tables.  `prev`: which of the slots' buffers holds the round before (kLgSlots).
 template <class F, int MODE>
-__device__ __forceinline__ typename F::E lg_slot(const LgInst& in, const LgConst<F>& k, const LgRows* rows, uint32_t slot, uint64_t e,
+__device__ __forceinline__ typename F::E lg_slot(const LgInst& in, const LgConst<F>& k, uint32_t slot, uint64_t e,
                                                  const typename F::FoldKey& rk, const typename F::FoldKey& lamk, uint32_t prev) {
     typedef typename F::E E;
     if (MODE == kLgSlots) {
@@ -148,9 +148,9 @@ __device__ __forceinline__ typename F::E lg_slot(const LgInst& in, const LgConst
         return F::add(a, F::mul_key(rk, F::sub(b, a)));
     }
     const bool inner = in.kind == kLogupInner;
-    if (slot == 0) return inner ? lg_entry<F, MODE>(in, 2, e, rk) : LgColumns<F, MODE>::get(in, k, rows, 0, e, rk);
+    if (slot == 0) return inner ? lg_entry<F, MODE>(in, 2, e, rk) : LgColumns<F, MODE>::get(in, k, nullptr, 0, e, rk);
     if (slot == 3) return lg_entry<F, MODE>(in, 0, e, rk);
-    const E d = inner ? lg_entry<F, MODE>(in, 3, e, rk) : LgColumns<F, MODE>::get(in, k, rows, 1, e, rk);
+    const E d = inner ? lg_entry<F, MODE>(in, 3, e, rk) : LgColumns<F, MODE>::get(in, k, nullptr, 1, e, rk);
     if (slot == 1) return d;
     return F::add(lg_entry<F, MODE>(in, 1, e, rk), F::mul_key(lamk, d));
 }
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(128, sizeof(typename F::E) == 16 ? 4 : MODE ==
             const LgConst<F>& k = consts_g[i];
             const LgRows* rows = rows_g ? rows_g + i : nullptr;
             auto value = [&](uint32_t slot, uint64_t e) -> E {
-                if (MODE == kLgSlots) return lg_slot<F, kLgSlots>(in, k, rows, slot, e, rk, lamk, prev);
+                if (MODE == kLgSlots) return lg_slot<F, kLgSlots>(in, k, slot, e, rk, lamk, prev);
                 constexpr int M = MODE == kLgSlots ? kLgOriginal : MODE;
                 if (slot == 3) return lg_entry<F, M>(in, 0, e, rk);
                 if (KIND == kLogupInner) return lg_entry<F, M>(in, slot == 0 ? 2 : 3, e, rk);
@@ -293,8 +293,8 @@ __global__ void __launch_bounds__(128)
     if (i >= n_inst) return;
     const LgInst& in = inst[i];
     for (uint32_t s = 0; s < lg_slots(in); s++)
-        out[4 * i + s] = last_round == 0 ? lg_slot<F, kLgBind>(in, consts[i], nullptr, s, 0, rk, lamk, 0)
-                                         : lg_slot<F, kLgSlots>(in, consts[i], nullptr, s, 0, rk, lamk, (last_round - 1) & 1);
+        out[4 * i + s] = last_round == 0 ? lg_slot<F, kLgBind>(in, consts[i], s, 0, rk, lamk, 0)
+                                         : lg_slot<F, kLgSlots>(in, consts[i], s, 0, rk, lamk, (last_round - 1) & 1);
 }
 
 // ---- the resident kernel ----------------------------------------------------------
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kTailThreads)
             const uint32_t slot = t - in.tab0, slots = lg_slots(in);
             E v;
             if (slot < slots) {
-                v = lg_slot<F, MODE>(in, consts[i], nullptr, slot, e0 + e, sh_key, sh_lam, prev);
+                v = lg_slot<F, MODE>(in, consts[i], slot, e0 + e, sh_key, sh_lam, prev);
             } else {  // the second column's halves, for the end (only from the originals: MODE is not kLgSlots then)
                 const uint32_t q = (in.kind == kLogupTable ? 2u : 0u) + (slot - slots) * 2 + 1;
                 v = lg_entry<F, MODE == kLgSlots ? kLgOriginal : MODE>(in, q, e0 + e, sh_key);
