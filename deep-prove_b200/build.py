@@ -18,7 +18,7 @@ FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC,-Wall,-Wno-unused-function",
-    "--expt-relaxed-constexpr", "--split-compile=0",
+    "--expt-relaxed-constexpr",
     "-I", os.path.join(HERE, "..", "include"),
 ]
 
