@@ -45,19 +45,59 @@ static void int_rows(LogupTree<FrFam>& t, uint32_t j) {
 }
 static void int_rows(LogupTree<GlFam>&, uint32_t) {}
 
+// From this many rows, or fractions of a level, of all trees together a BN254 level is a launch of its own (level 1: of
+// trees over field columns).  Two levels at a time and so, four columns: 2^19 rows 134 and 133 us, 2^20 196 and 181.
+constexpr uint64_t kLogupSingle = 1ull << 20;
+
+// The levels of `cnt` of the call's n trees.
+template <class F, bool ONE>
+static void launch_trees(dpb_ctx* ctx, const LogupTree<F>* dt, const LogupTree<F>* trees, uint32_t cnt, uint32_t n, typename F::E* outputs) {
+    uint32_t max_m = 0;
+    bool any_rows = false, all_rows = true;
+    for (uint32_t i = 0; i < cnt; i++) {
+        max_m = std::max(max_m, trees[i].m);
+        any_rows |= trees[i].int_rows != 0;
+        all_rows &= trees[i].int_rows != 0;
+    }
+    auto grid = [&](uint32_t items_log2) {  // per tree; all trees together fill the GPU
+        const uint64_t want = ((1ull << items_log2) + kThreads - 1) / kThreads, cap = ((uint64_t)ctx->sm_count * 8 + n - 1) / n;
+        return dim3((uint32_t)std::max<uint64_t>(1, std::min(want, cap)), cnt);
+    };
+    const LogupTree<F>& one = trees[0];
+    constexpr bool kFr = sizeof(typename F::E) == 32;
+    auto single = [&](uint32_t l) { return ((uint64_t)n << (max_m - l)) >= kLogupSingle; };
+    const bool split = kFr && !all_rows && single(0);
+    if (!split || any_rows) logup_leaf_levels<F, ONE><<<grid(max_m - 2), kThreads, 0, ctx->stream>>>(dt, one, split);
+    if constexpr (kFr) {
+        if (split) {
+            logup_leaf_level<F, ONE><<<grid(max_m - 1), kThreads, 0, ctx->stream>>>(dt, one);
+            logup_one_level<F, ONE><<<grid(max_m - 2), kThreads, 0, ctx->stream>>>(dt, one, 1);
+        }
+    }
+    for (uint32_t l = 2; l + 2 <= max_m && (1ull << (max_m - l)) > kLogupSmall; l += 2) {
+        if constexpr (kFr) {
+            if (single(l)) {
+                logup_one_level<F, ONE><<<grid(max_m - l - 1), kThreads, 0, ctx->stream>>>(dt, one, l);
+                logup_one_level<F, ONE><<<grid(max_m - l - 2), kThreads, 0, ctx->stream>>>(dt, one, l + 1);
+                continue;
+            }
+        }
+        logup_two_levels<F, ONE><<<grid(max_m - l - 2), kThreads, 0, ctx->stream>>>(dt, one, l);
+    }
+    logup_small_levels<F, ONE><<<cnt, kThreads, 0, ctx->stream>>>(dt, one, outputs);
+}
+
 // The trees' levels, and their outputs (4 elements each) to the host when asked for.
 template <class F>
 static int build_trees(dpb_ctx* ctx, const LogupSpec* specs, uint32_t n, dpb_logup** out, void* host_outputs) {
     typedef typename F::E E;
     std::vector<LogupTree<F>> trees(n);
-    uint32_t max_m = 0;
     for (uint32_t i = 0; i < n; i++) {
         const LogupSpec& p = specs[i];
         dpb_logup* lu = out[i];
         LogupTree<F>& t = trees[i];
         memset((void*)&t, 0, sizeof t);
         const uint32_t m = lu->m;
-        max_m = std::max(max_m, m);
         DPB_TRY(device_alloc(ctx, logup_level_offset(m, m) * sizeof(E), &lu->slab));
         for (uint32_t l = 1; l < m; l++) {
             lu->num.push_back((E*)lu->slab + logup_level_offset(m, l));
@@ -74,40 +114,35 @@ static int build_trees(dpb_ctx* ctx, const LogupSpec* specs, uint32_t n, dpb_log
         memcpy(&t.constant, p.constant, sizeof(E));
         E sep, pw = F::one();
         memcpy(&sep, p.sep, sizeof(E));
-        t.int_cols = 1;
+        t.int_rows = sizeof(E) == 32;
         E sum = F::zero();
         for (uint32_t j = 0; j < p.n_cols; j++) {
             t.col[j] = p.columns[j]->ptr;
             t.dtype[j] = p.columns[j]->dtype;
-            if (!is_int_dtype(t.dtype[j])) t.int_cols = 0;
+            if (!is_int_dtype(t.dtype[j])) t.int_rows = 0;
             t.sep_pow[j] = pw;
             sum = F::add(sum, pw);
             pw = F::mul(pw, sep);
         }
         t.int_constant = F::sub(t.constant, F::mul(F::from_u64(0x80000000ull), sum));
-        for (uint32_t j = 0; t.int_cols && j < p.n_cols; j++) int_rows(t, j);
+        for (uint32_t j = 0; t.int_rows && j < p.n_cols; j++) int_rows(t, j);
     }
-    char* d = nullptr;  // [trees | outputs]
-    const size_t o_out = (n * sizeof(LogupTree<F>) + 31) & ~(size_t)31;
-    DPB_TRY(device_alloc(ctx, o_out + (size_t)n * 4 * sizeof(E), (void**)&d));
-    const LogupTree<F>* dt = (const LogupTree<F>*)d;
-    int rc = upload_small(ctx, d, trees.data(), n * sizeof(LogupTree<F>));
+    // one tree goes to the kernels as a parameter, several through memory: [trees | outputs]
+    char* d = nullptr;
+    const size_t o_out = n > 1 ? (n * sizeof(LogupTree<F>) + 31) & ~(size_t)31 : 0;
+    if (n > 1 || host_outputs) DPB_TRY(device_alloc(ctx, o_out + (size_t)n * 4 * sizeof(E), (void**)&d));
+    E* outputs = d ? (E*)(d + o_out) : nullptr;
+    int rc = n > 1 ? upload_small(ctx, d, trees.data(), n * sizeof(LogupTree<F>)) : DPB_OK;
     if (rc == DPB_OK) {
-        auto blocks = [&](uint64_t items) {  // per tree; all trees together fill the GPU
-            const uint64_t want = (items + kThreads - 1) / kThreads, cap = ((uint64_t)ctx->sm_count * 8 + n - 1) / n;
-            return (uint32_t)std::max<uint64_t>(1, std::min(want, cap));
-        };
         for (uint32_t first = 0; first < n; first += 65535) {  // the grid's second dimension
             const uint32_t cnt = std::min<uint32_t>(65535, n - first);
-            logup_leaf_levels<F><<<dim3(blocks(1ull << (max_m - 2)), cnt), kThreads, 0, ctx->stream>>>(dt + first);
-            for (uint32_t l = 2; l + 2 <= max_m && (1ull << (max_m - l)) > kLogupSmall; l += 2)
-                logup_two_levels<F><<<dim3(blocks(1ull << (max_m - l - 2)), cnt), kThreads, 0, ctx->stream>>>(dt + first, l);
-            logup_small_levels<F><<<cnt, kThreads, 0, ctx->stream>>>(dt + first, (E*)(d + o_out) + 4 * (size_t)first);
+            if (n > 1) launch_trees<F, false>(ctx, (const LogupTree<F>*)d + first, trees.data() + first, cnt, n, outputs ? outputs + 4 * (size_t)first : nullptr);
+            else launch_trees<F, true>(ctx, nullptr, trees.data(), 1, 1, outputs);
         }
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess && host_outputs) {
             TracePhase t_out("logup.outputs");
-            e = cudaMemcpyAsync(host_outputs, d + o_out, (size_t)n * 4 * sizeof(E), cudaMemcpyDeviceToHost, ctx->stream);
+            e = cudaMemcpyAsync(host_outputs, outputs, (size_t)n * 4 * sizeof(E), cudaMemcpyDeviceToHost, ctx->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         }
         if (e != cudaSuccess) rc = fail(DPB_ECUDA, "logup trees: %s", cudaGetErrorString(e));

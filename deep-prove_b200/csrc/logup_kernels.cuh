@@ -35,7 +35,7 @@ struct LogupTree {
     int32_t dtype[kMaxLogupCols];
     int32_t mult_dtype;
     uint32_t n_cols, m;
-    uint32_t is_table, int_cols;           // int_cols: every column holds integers
+    uint32_t is_table, int_rows;           // int_rows: BN254, every column holds integers (rows above)
 };
 
 // entries before level l of a tree over 2^m rows (level l has 2^(m-l) fractions)
@@ -104,50 +104,113 @@ __device__ __forceinline__ LogupFrac<F> logup_load(const LogupTree<F>& t, uint32
     return f;
 }
 
-template <class F>
-__device__ __forceinline__ typename F::E logup_denominator(const LogupTree<F>& t, uint64_t i) {
-    if (sizeof(typename F::E) == 32 && t.int_cols) return logup_int_denominator(t, i);
-    typename F::E d = t.constant;
-    for (uint32_t j = 0; j < t.n_cols; j++) {
-        const typename F::E v = F::load(t.col[j], t.dtype[j], i);
-        // sep^0 = 1: the first column is added as is (circuit.rs:162-171)
-        d = F::add(d, j == 0 ? v : F::mul(t.sep_pow[j], v));
+// Denominators of K rows, column by column, so that K loads and products are under way at once (Goldilocks, 2^24 rows, two
+// columns: 411 us one row at a time, 348 by four).
+// A launch of logup_leaf_level never meets integer columns' rows: ROWS = false keeps their registers out of it.
+template <class F, bool ROWS, int K>
+__device__ __forceinline__ void logup_denominators(const LogupTree<F>& t, const uint64_t (&row)[K], typename F::E (&d)[K]) {
+    if (ROWS && sizeof(typename F::E) == 32 && t.int_rows) {
+#pragma unroll
+        for (int k = 0; k < K; k++) d[k] = logup_int_denominator(t, row[k]);
+        return;
     }
-    return d;
+#pragma unroll
+    for (int k = 0; k < K; k++) d[k] = t.constant;
+    for (uint32_t j = 0; j < t.n_cols; j++) {
+        typename F::E v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = F::load(t.col[j], t.dtype[j], row[k]);
+        // sep^0 = 1: the first column is added as is (circuit.rs:162-171)
+#pragma unroll
+        for (int k = 0; k < K; k++) d[k] = F::add(d[k], j == 0 ? v[k] : F::mul(t.sep_pow[j], v[k]));
+    }
 }
-// entry i of level 1: the rows i and i + 2^(m-1).  A lookup's numerators are -1 (circuit.rs:151-182), a table's its
-// multiplicities (circuit.rs:117-150).
-template <class F>
-__device__ __forceinline__ LogupFrac<F> logup_leaf(const LogupTree<F>& t, uint64_t i) {
+// entry i of level 1: the rows i and i + 2^(m-1) with denominators d1 and d2.  A lookup's numerators are -1
+// (circuit.rs:151-182), a table's its multiplicities (circuit.rs:117-150).
+template <class F, bool ROWS>
+__device__ __forceinline__ LogupFrac<F> logup_leaf(const LogupTree<F>& t, uint64_t i, const typename F::E& d1, const typename F::E& d2) {
     const uint64_t half = 1ull << (t.m - 1);
-    const typename F::E d1 = logup_denominator<F>(t, i), d2 = logup_denominator<F>(t, i + half);
     LogupFrac<F> r;
-    r.n = t.is_table ? TwoProducts<F>::sum(F::load(t.mult, t.mult_dtype, i), d2, d1, F::load(t.mult, t.mult_dtype, i + half))
-                     : F::neg(F::add(d1, d2));
+    if (!t.is_table) r.n = F::neg(F::add(d1, d2));
+    else if (ROWS) r.n = TwoProducts<F>::sum(F::load(t.mult, t.mult_dtype, i), d2, d1, F::load(t.mult, t.mult_dtype, i + half));
+    else r.n = F::add(F::mul(F::load(t.mult, t.mult_dtype, i), d2), F::mul(d1, F::load(t.mult, t.mult_dtype, i + half)));
     r.d = F::mul(d1, d2);
     return r;
 }
 
-// Levels 1 and 2 from the columns.
-template <class F>
+// ONE: a launch over one tree takes it as a parameter.  That saves the upload (10 us of a tree of 2^10 rows) and a trip
+// to memory for every column's address.
+template <class F, bool ONE>
+__device__ __forceinline__ const LogupTree<F>& logup_tree(const LogupTree<F>* trees, const LogupTree<F>& one, uint32_t i) {
+    return ONE ? one : trees[i];
+}
+
+// Levels 1 and 2 from the columns; with rows_only the trees over integer columns alone (BN254, rows).
+template <class F, bool ONE>
 __global__ void __launch_bounds__(kThreads, 2)
-    logup_leaf_levels(const LogupTree<F>* __restrict__ trees) {
-    const LogupTree<F>& t = trees[blockIdx.y];
+    logup_leaf_levels(const LogupTree<F>* __restrict__ trees, const __grid_constant__ LogupTree<F> one, bool rows_only) {
+    const LogupTree<F>& t = logup_tree<F, ONE>(trees, one, blockIdx.y);
+    if (rows_only && !t.int_rows) return;
     const uint64_t q = 1ull << (t.m - 2), stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < q; i += stride) {
-        const LogupFrac<F> a = logup_leaf<F>(t, i);
-        logup_store<F>(t, 1, i, a);
-        const LogupFrac<F> b = logup_leaf<F>(t, i + q);
+        LogupFrac<F> a, b;
+        if (sizeof(typename F::E) == 32) {  // 128 registers hold two rows of BN254 columns
+            typename F::E d[2];
+            logup_denominators<F, true>(t, {i, i + 2 * q}, d);
+            a = logup_leaf<F, true>(t, i, d[0], d[1]);
+            logup_store<F>(t, 1, i, a);
+            logup_denominators<F, true>(t, {i + q, i + 3 * q}, d);
+            b = logup_leaf<F, true>(t, i + q, d[0], d[1]);
+        } else {
+            typename F::E d[4];
+            logup_denominators<F, true>(t, {i, i + 2 * q, i + q, i + 3 * q}, d);
+            a = logup_leaf<F, true>(t, i, d[0], d[1]);
+            logup_store<F>(t, 1, i, a);
+            b = logup_leaf<F, true>(t, i + q, d[2], d[3]);
+        }
         logup_store<F>(t, 1, i + q, b);
         if (t.m > 2) logup_store<F>(t, 2, i, logup_add<F>(a, b));
     }
 }
 
+// Level 1 alone, for the trees logup_leaf_levels leaves out with rows_only, and one later level: large BN254 levels are
+// bound by loads and products that want four blocks per SM (64 registers, a reduction per product), where two levels
+// together take 104 or 128 registers and a sum of two products 76.  Trees of 2^24 rows, 1 / 2 / 4 field columns: 898 /
+// 1305 / 2108 us in launches of two levels, 745 / 1036 / 1620 here.
+template <class F, bool ONE>
+__global__ void __launch_bounds__(kThreads, 4)
+    logup_leaf_level(const LogupTree<F>* __restrict__ trees, const __grid_constant__ LogupTree<F> one) {
+    const LogupTree<F>& t = logup_tree<F, ONE>(trees, one, blockIdx.y);
+    if (t.int_rows) return;
+    const uint64_t half = 1ull << (t.m - 1), stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < half; i += stride) {
+        typename F::E d[2];
+        logup_denominators<F, false>(t, {i, i + half}, d);
+        logup_store<F>(t, 1, i, logup_leaf<F, false>(t, i, d[0], d[1]));
+    }
+}
+// Level l + 1 from level l.  l = 1: for the trees of logup_leaf_level; later: in pairs with an even l first, for the
+// trees whose level at that even l is still too large for one block.
+template <class F, bool ONE>
+__global__ void __launch_bounds__(kThreads, 4)
+    logup_one_level(const LogupTree<F>* __restrict__ trees, const __grid_constant__ LogupTree<F> one, uint32_t l) {
+    const LogupTree<F>& t = logup_tree<F, ONE>(trees, one, blockIdx.y);
+    if (l == 1 ? t.int_rows || t.m <= 2 : t.m < (l & ~1u) + 2 || (1ull << (t.m - (l & ~1u))) <= kLogupSmall) return;
+    const uint64_t half = 1ull << (t.m - l - 1), stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < half; i += stride) {
+        const LogupFrac<F> a = logup_load<F>(t, l, i), b = logup_load<F>(t, l, i + half);
+        LogupFrac<F> r;
+        r.n = F::add(F::mul(a.n, b.d), F::mul(b.n, a.d));
+        r.d = F::mul(a.d, b.d);
+        logup_store<F>(t, l + 1, i, r);
+    }
+}
+
 // Levels l + 1 and l + 2 from level l, for the trees whose level l is still too large for one block.
-template <class F>
+template <class F, bool ONE>
 __global__ void __launch_bounds__(kThreads, 2)
-    logup_two_levels(const LogupTree<F>* __restrict__ trees, uint32_t l) {
-    const LogupTree<F>& t = trees[blockIdx.y];
+    logup_two_levels(const LogupTree<F>* __restrict__ trees, const __grid_constant__ LogupTree<F> one, uint32_t l) {
+    const LogupTree<F>& t = logup_tree<F, ONE>(trees, one, blockIdx.y);
     if (t.m < l + 2 || (1ull << (t.m - l)) <= kLogupSmall) return;
     const uint64_t q = 1ull << (t.m - l - 2), stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < q; i += stride) {
@@ -159,11 +222,13 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
-// The rest of every tree, one block each, and the top level's four values per tree side by side in `outputs`.
-template <class F>
+// The rest of every tree, one block each, and the top level's four values per tree side by side in `outputs` (when
+// given).
+template <class F, bool ONE>
 __global__ void __launch_bounds__(kThreads)
-    logup_small_levels(const LogupTree<F>* __restrict__ trees, typename F::E* __restrict__ outputs) {
-    const LogupTree<F>& t = trees[blockIdx.x];
+    logup_small_levels(const LogupTree<F>* __restrict__ trees, const __grid_constant__ LogupTree<F> one,
+                       typename F::E* __restrict__ outputs) {
+    const LogupTree<F>& t = logup_tree<F, ONE>(trees, one, blockIdx.x);
     uint32_t l = t.m > 2 ? 2 : 1;  // the last level there is
     while ((1ull << (t.m - l)) > kLogupSmall) l += 2;
     for (; l + 1 < t.m; l++) {
@@ -172,7 +237,7 @@ __global__ void __launch_bounds__(kThreads)
             logup_store<F>(t, l + 1, i, logup_add<F>(logup_load<F>(t, l, i), logup_load<F>(t, l, i + half)));
         __syncthreads();  // this level is complete (and visible to the block) before the next one reads it
     }
-    if (threadIdx.x < 4) {
+    if (outputs && threadIdx.x < 4) {
         const typename F::E* top = t.slab + logup_level_offset(t.m, t.m - 1);
         outputs[4 * blockIdx.x + threadIdx.x] = top[threadIdx.x];
     }
