@@ -337,12 +337,13 @@ def bn254_record(dpb, prover, ctx, torch, stream, device, steps, n):
     for e in sorted(prof, key=lambda e: e["round"])[:6]:
         per_ms = e["total_ms"] / e["launches"]
         pairs = 1 << (n - e["round"] - 1)
-        # round 0: samples at 0, 1, inf, -1 of a product of three = 8 products per pair;
-        # later rounds: 6 folds by the challenge (precomputed rows) + 3 samples x 2 products
-        floor_s = pairs * (8 / mul_rate if e["round"] == 0 else 6 / fixed_rate + 6 / mul_rate)
+        # A product that stays unreduced is half of one (64 of its 128 multiply-adds).  Round 0: two tables at 0, 1 and
+        # infinity (-1 is derived), the third unreduced at all four samples = 3 + 4/2 products per pair; later rounds:
+        # 6 folds by the challenge (precomputed rows) + two tables at three samples + 3/2
+        floor_s = pairs * (5 / mul_rate if e["round"] == 0 else 6 / fixed_rate + 4.5 / mul_rate)
         kernels.append({"kernel": e["kernel"], "round": e["round"], "ms_per_launch": per_ms,
                         "GBps": e["alg_bytes_per_launch"] / (per_ms * 1e-3) / 1e9,
-                        "products_per_pair": 8 if e["round"] == 0 else 12,
+                        "products_per_pair": 5 if e["round"] == 0 else 10.5,
                         "frac_of_multiplier_floor": floor_s / (per_ms * 1e-3)})
     top = max(kernels, key=lambda k: k["ms_per_launch"]) if kernels else None
     peak, _ = load_peak()
@@ -355,7 +356,7 @@ def bn254_record(dpb, prover, ctx, torch, stream, device, steps, n):
         ach = (1 << (n - top["round"] - 1)) * top["products_per_pair"] / (top["ms_per_launch"] * 1e-3)
         rec["roofline"] = {"bound": "imad", "kernel": top["kernel"], "round": top["round"],
                            "achieved": ach, "unit": "field products/s",
-                           "peak": mul_rate if top["round"] == 0 else 12 / (6 / fixed_rate + 6 / mul_rate),
+                           "peak": mul_rate if top["round"] == 0 else 10.5 / (6 / fixed_rate + 4.5 / mul_rate),
                            "frac": top["frac_of_multiplier_floor"],
                            "peak_source": "dpb_issue_rate_probe on this GPU (chains of the kernels' own product "
                                           "routines on register operands)"}
