@@ -9,10 +9,12 @@
 // The large levels are bound by their products and by HBM, the many small ones by launches.  So blockIdx.y is the
 // instance, a thread makes two entries of one level and, from registers, the entry of the next that they add up to
 // (the first of the two levels is written, never read back), and one block per instance finishes once a level has at
-// most kLogupSmall entries.  A BN254 denominator  c + col_0 + s col_1 + ..  over integer columns is one sum of rows
-// (8 multiply-adds per column) with one reduction, where every column was widened and multiplied mod r.
-// Three instances of 2^21 rows, 5 integer columns, BN254: 560 us in 33 launches before, 416 us in 7; 36 instances of
-// 2^16 rows, Goldilocks: 780 us in 216 launches and 64 us in 5.
+// most kLogupSmall entries.  Where registers for two levels cost more than reading a level back, a launch makes one
+// (logup_leaf_level, logup_one_level).  A BN254 denominator  c + col_0 + s col_1 + ..  over integer columns is one sum of
+// rows (8 multiply-adds per column) with one reduction, where every column was widened and multiplied mod r.
+// 36 instances of 2^16 rows, Goldilocks: 780 us in 216 launches of one instance's level each, 64 us in 5; three
+// instances of 2^21 rows, 5 integer columns, BN254: 560 us in 33 launches, 416 us two levels at a time, about 20 us less
+// since large levels are made alone.
 #pragma once
 #include "family.cuh"
 #include "lazy_sum.cuh"
