@@ -276,7 +276,7 @@ __device__ __forceinline__ void lincomb_row_mac(frw::RowAcc& acc, const uint32_t
     const uint32_t r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     frw::rowacc_mac(acc, r, x);
 }
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)  // four blocks per SM: 64 registers
     linear_combination_fr(const LinCombSrc* __restrict__ src, const uint32_t* __restrict__ rows, uint32_t n, uint64_t len,
                           Fr* __restrict__ out) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
